@@ -727,8 +727,7 @@ int b200sv_apply_ops_fused(b200sv_handle h, const b200sv_op *ops, uint32_t nops)
         descs.reserve(rec.size());
         for (auto &o : rec) descs.push_back(compile_op(o, o.inverse, h->nq));  // validate all first
         void *s[1] = {h->d_state};
-        if (!fused_worthwhile(h->dtype, h->nq)) {
-            // too few tiles to fill the GPU: one launch per gate
+        if (!fused_worthwhile(h->dtype, h->nq, descs.size(), h->stream())) {
             for (auto &g : descs) apply_desc(h, s, 1, g);
             return;
         }
@@ -1197,7 +1196,7 @@ int b200sv_adjoint_jacobian(b200sv_handle psi, const b200sv_op *ops, uint32_t no
             std::vector<GateDesc> fwd;
             for (auto &o : rec) fwd.push_back(compile_op(o, o.inverse, h->nq));
             void *s1[1] = {lambda};
-            if (fused_worthwhile(h->dtype, h->nq))
+            if (fused_worthwhile(h->dtype, h->nq, fwd.size(), st))
                 apply_fused(lambda, h->nq, h->dtype, fwd, [&](const GateDesc &g) { apply_desc(h, s1, 1, g); }, st);
             else
                 for (auto &g : fwd) apply_desc(h, s1, 1, g);
@@ -1239,6 +1238,17 @@ int b200sv_adjoint_jacobian(b200sv_handle psi, const b200sv_op *ops, uint32_t no
         }
         std::vector<void *> lambda_and_bras{lambda};
         lambda_and_bras.insert(lambda_and_bras.end(), bras.begin(), bras.end());
+        // several bras: a second lambda for the fused passes (the observables' work state where
+        // there was one); without the memory for it the steps run one by one
+        void *lambda2 = tmp;
+        if (nobs > 1 && !lambda2) {
+            if (cudaMallocAsync(&lambda2, h->state_bytes(), st) == cudaSuccess) {
+                bufs.push_back(lambda2);
+            } else {
+                cudaGetLastError();
+                lambda2 = nullptr;
+            }
+        }
         // one step: the products (one-wire gates: products and inverse in one pass over the pairs)
         auto exec_single = [&](size_t i) {
             const AdjItem &it = items[i];
@@ -1266,11 +1276,11 @@ int b200sv_adjoint_jacobian(b200sv_handle psi, const b200sv_op *ops, uint32_t no
                                                        h->d_partials, dst, 1, st, h->arrival());
                 }
             }
+            lambda_and_bras[0] = lambda;
             apply_desc_multi(h, lambda_and_bras, it.adj);  // lambda and every bra in one launch
         };
-        if (nobs == 1 && fused_adjoint_worthwhile(h->dtype, h->nq)) {
-            // one bra (the VJP form): fused passes over lambda and the bra
-            apply_fused_adjoint(lambda, bras[0], h->nq, h->dtype, items, exec_single, d_jac, st);
+        if (nobs == 1 || (nobs > 1 && nobs <= 65535 && lambda2)) {
+            apply_fused_adjoint(lambda, lambda2, bras, h->nq, h->dtype, items, exec_single, d_jac, st);
         } else {
             for (size_t i = 0; i < items.size(); ++i) exec_single(i);
         }

@@ -46,6 +46,11 @@ template <typename R> struct Geo;
 template <> struct Geo<double> { static constexpr int kt = 12, a = 3, A = 8, reserve = 3; };
 template <> struct Geo<float> { static constexpr int kt = 13, a = 4, A = 16, reserve = 4; };
 
+// Tile bits of a state of nq qubits.  A state narrower than the full tile is one tile of its own
+// size, run by one CTA of 2^(bits - a) threads; below one warp of threads the tile is padded to
+// a warp's worth of amplitudes whose upper part lies outside the state (never loaded or stored).
+template <typename G> int tile_width(uint32_t nq) { return std::max(std::min<int>(G::kt, (int)nq), G::a + 5); }
+
 // Shared-memory position of tile amplitude l.  complex128: the three low bits are XORed
 // with bits 3..5, so eight threads whose amplitudes differ in any three of bits 0..5
 // (bits s and s+3 not both) hit eight different 16-byte bank groups.  complex64: bits
@@ -410,12 +415,18 @@ template <typename T> __device__ __forceinline__ void stage(T *dst, const T *src
 // phases, register ops, shared-memory ops and coefficients.  A tile is moved in 16-byte
 // chunks (V amplitudes each, V = 16 / the amplitude size); chunk c of a thread is
 // c = threadIdx.x + j * blockDim.x, j < A / V.
-template <typename R>
-__global__ void __launch_bounds__(kFThreads, 1) k_fused(C<R> *__restrict__ state, SegArgs a, uint64_t ntiles) {
-    constexpr int KT = Geo<R>::kt, A = Geo<R>::A;
-    constexpr uint32_t TN = 1u << KT;
+// NARROW: the state is one tile of `kt` < Geo<R>::kt bits (run-time tile and block sizes).  One CTA
+// then runs a chain of phases, where a launch per gate was bound by about 3 us of launch each: a
+// 10-qubit complex128 evaluation (117 gates and a 20-word Hamiltonian) went from 747 to 447 us.
+template <typename R, bool NARROW>
+__global__ void __launch_bounds__(kFThreads, 1) k_fused(C<R> *__restrict__ state, SegArgs a, uint64_t ntiles, int kt,
+                                                        uint64_t namp) {
+    constexpr int A = Geo<R>::A;
+    const int KT = NARROW ? kt : Geo<R>::kt;
+    const uint32_t NT = NARROW ? blockDim.x : (uint32_t)kFThreads;
+    const uint32_t TN = 1u << KT;
     constexpr int V = 16 / (int)sizeof(C<R>);
-    constexpr int PER = (int)(TN / V) / kFThreads;  // 16-byte chunks per thread
+    constexpr int PER = A / V;  // 16-byte chunks per thread
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t s_lbits[16], s_gbits[48];
     __shared__ uint64_t s_hi[PER];  // state offset of chunk row j (the same for every thread)
@@ -435,12 +446,14 @@ __global__ void __launch_bounds__(kFThreads, 1) k_fused(C<R> *__restrict__ state
     stage(sfop, a.fops, a.nfop);
     stage(scf, static_cast<const C<R> *>(a.coefs), a.ncoef);
     __syncthreads();
-    // address parts of the tile moves: chunk c = threadIdx.x + j * 512 -> tile amplitude c * V
-    if (threadIdx.x < PER) s_hi[threadIdx.x] = deposit((uint64_t)threadIdx.x * kFThreads * V, s_lbits, KT);
+    // address parts of the tile moves: chunk c = threadIdx.x + j * blockDim.x -> tile amplitude c * V
+    if (threadIdx.x < PER) s_hi[threadIdx.x] = deposit((uint64_t)threadIdx.x * NT * V, s_lbits, KT);
     __syncthreads();
     const uint64_t lo = deposit((uint64_t)threadIdx.x * V, s_lbits, KT);
     // swizzled shared-memory position of chunk j of this thread
-    auto sw = [&](int j) { return swz<R>((threadIdx.x + (uint32_t)j * kFThreads) * V); };
+    auto sw = [&](int j) { return swz<R>((threadIdx.x + (uint32_t)j * NT) * V); };
+    // a padded tile's amplitudes outside the state are zeros that never leave the CTA
+    auto inside = [&](uint64_t x) { return !NARROW || x < namp; };
 
     uint64_t t = blockIdx.x;
     uint32_t cur = 0;
@@ -448,7 +461,11 @@ __global__ void __launch_bounds__(kFThreads, 1) k_fused(C<R> *__restrict__ state
     if (t < ntiles) {
         tb_cur = deposit(t, s_gbits, a.ng);
 #pragma unroll
-        for (int j = 0; j < PER; ++j) cp_async16(buf0 + sw(j), state + (tb_cur | lo | s_hi[j]));
+        for (int j = 0; j < PER; ++j) {
+            const uint64_t x = tb_cur | lo | s_hi[j];
+            if (inside(x)) cp_async16(buf0 + sw(j), state + x);
+            else *reinterpret_cast<float4 *>(buf0 + sw(j)) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     }
     cp_async_commit();
     for (; t < ntiles; t += gridDim.x) {
@@ -458,7 +475,7 @@ __global__ void __launch_bounds__(kFThreads, 1) k_fused(C<R> *__restrict__ state
             tb_next = deposit(tnext, s_gbits, a.ng);
             C<R> *dst = buf0 + (cur ^ 1u) * TN;
 #pragma unroll
-            for (int j = 0; j < PER; ++j) cp_async16(dst + sw(j), state + (tb_next | lo | s_hi[j]));
+            for (int j = 0; j < PER; ++j) cp_async16(dst + sw(j), state + (tb_next | lo | s_hi[j]));  // never NARROW
         }
         cp_async_commit();
         cp_async_wait1();
@@ -496,7 +513,8 @@ __global__ void __launch_bounds__(kFThreads, 1) k_fused(C<R> *__restrict__ state
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
             const float4 x = *reinterpret_cast<const float4 *>(s + sw(j));
-            *reinterpret_cast<float4 *>(state + (tbase | lo | s_hi[j])) = x;
+            const uint64_t at = tbase | lo | s_hi[j];
+            if (inside(at)) *reinterpret_cast<float4 *>(state + at) = x;
         }
         __syncthreads();  // the buffer is refilled next iteration
         cur ^= 1u;
@@ -716,8 +734,8 @@ using RopHook = std::function<void(size_t, ROp &, const int *)>;
 
 template <typename R, typename G = Geo<R>>
 void lower_phase(SegCode<R> &sc, uint32_t rmask, const std::vector<const GateDesc *> &ops,
-                 const std::vector<int> &loc, const RopHook &hook = nullptr) {
-    constexpr int KT = G::kt, a = G::a, A = G::A;
+                 const std::vector<int> &loc, int KT, const RopHook &hook = nullptr) {
+    constexpr int a = G::a, A = G::A;
     // pad the register bits to a bits with the highest free tile bits
     for (int b = KT - 1; b >= 0 && __builtin_popcount(rmask) < a; --b)
         if (!((rmask >> b) & 1)) rmask |= 1u << b;
@@ -861,7 +879,7 @@ void lower_phase(SegCode<R> &sc, uint32_t rmask, const std::vector<const GateDes
 // earliest gate left.  A gate of the shared-memory form runs as a phase of its own once it
 // is ready and no register gate can move.
 template <typename R>
-void lower_segment(SegCode<R> &sc, const std::vector<GateDesc> &ops, const std::vector<int> &loc) {
+void lower_segment(SegCode<R> &sc, const std::vector<GateDesc> &ops, const std::vector<int> &loc, int kt) {
     constexpr int a = Geo<R>::a;
     const size_t n = ops.size();
     std::vector<int64_t> tgt(n);
@@ -873,10 +891,12 @@ void lower_segment(SegCode<R> &sc, const std::vector<GateDesc> &ops, const std::
         diag[i] = is_diagonal(ops[i]);
         if (ops[i].kind == Kind::Noop) done[i] = 1;
     }
-    auto ready = [&](size_t i) {
-        for (size_t j = 0; j < i; ++j)
-            if (!done[j] && (bits[j] & bits[i]) && !(diag[j] && diag[i])) return false;
-        return true;
+    // bits of the gates left behind so far in a scan (any of them, and the non-diagonal ones)
+    uint64_t left_any = 0, left_nondiag = 0;
+    auto ready = [&](size_t i) { return !(bits[i] & (diag[i] ? left_nondiag : left_any)); };
+    auto leave = [&](size_t i) {
+        left_any |= bits[i];
+        if (!diag[i]) left_nondiag |= bits[i];
     };
     size_t left = 0;
     for (size_t i = 0; i < n; ++i) left += done[i] ? 0 : 1;
@@ -885,10 +905,14 @@ void lower_segment(SegCode<R> &sc, const std::vector<GateDesc> &ops, const std::
         uint32_t rmask = 0;
         for (bool progress = true; progress;) {
             progress = false;
+            left_any = left_nondiag = 0;
             for (size_t i = 0; i < n; ++i) {
-                if (done[i] || tgt[i] < 0 || !ready(i)) continue;
+                if (done[i]) continue;
                 const uint32_t need = (uint32_t)tgt[i];
-                if (__builtin_popcount(rmask | need) > a) continue;
+                if (tgt[i] < 0 || !ready(i) || __builtin_popcount(rmask | need) > a) {
+                    leave(i);
+                    continue;
+                }
                 rmask |= need;
                 cur.push_back(&ops[i]);
                 done[i] = 1;
@@ -897,12 +921,16 @@ void lower_segment(SegCode<R> &sc, const std::vector<GateDesc> &ops, const std::
             }
         }
         if (!cur.empty()) {
-            lower_phase<R>(sc, rmask, cur, loc);
+            lower_phase<R>(sc, rmask, cur, loc, kt);
             continue;
         }
         // no register gate can move: the earliest ready shared-memory gate goes next
         size_t i = 0;
-        while (i < n && (done[i] || tgt[i] >= 0 || !ready(i))) ++i;
+        left_any = left_nondiag = 0;
+        while (i < n && (done[i] || tgt[i] >= 0 || !ready(i))) {
+            if (!done[i]) leave(i);
+            ++i;
+        }
         if (i == n) throw Unsupported("fused phase planning made no progress");
         RPhase ph{};
         ph.fop = (int32_t)sc.fops.size();
@@ -921,8 +949,8 @@ struct Segment {
 template <typename R>
 void run_fused(void *state, uint32_t nq, const std::vector<GateDesc> &descs,
                const std::function<void(const GateDesc &)> &apply_single, cudaStream_t st) {
-    constexpr int kt = Geo<R>::kt;
-    if ((int)nq < kt) throw Unsupported("state narrower than the fused tile");
+    const int kt = tile_width<Geo<R>>(nq);
+    const bool narrow = (int)nq < Geo<R>::kt;
     const uint64_t low = (uint64_t(1) << Geo<R>::reserve) - 1;  // 128 contiguous bytes in every tile
     struct Piece {
         bool seg;
@@ -980,6 +1008,7 @@ void run_fused(void *state, uint32_t nq, const std::vector<GateDesc> &descs,
                 sg.gbits.push_back((uint8_t)x);
             }
         }
+        for (int x = (int)nq; x < kt; ++x) sg.lbits.push_back((uint8_t)x);  // a padded tile's upper bits
         std::vector<const GateDesc *> seg;
         for (size_t j : take) {
             seg.push_back(&descs[j]);
@@ -991,7 +1020,7 @@ void run_fused(void *state, uint32_t nq, const std::vector<GateDesc> &descs,
         sg.fop_begin = (uint32_t)sc.fops.size();
         sg.coef_begin = (uint32_t)sc.coefs.size();
         SegCode<R> local;
-        lower_segment<R>(local, fused, loc);
+        lower_segment<R>(local, fused, loc, kt);
         sc.phases.insert(sc.phases.end(), local.phases.begin(), local.phases.end());
         sc.rops.insert(sc.rops.end(), local.rops.begin(), local.rops.end());
         sc.fops.insert(sc.fops.end(), local.fops.begin(), local.fops.end());
@@ -1037,8 +1066,11 @@ void run_fused(void *state, uint32_t nq, const std::vector<GateDesc> &descs,
     // at most 192 ops per segment: 128 KiB of tiles + 192 x (160 + 48) B + 32 KiB of coefficients
     // (+ 160 B per double excitation)
     if (smem_max > 227 * 1024) throw Unsupported("fused segment records exceed shared memory");
-    B200SV_CUDA(cudaFuncSetAttribute(k_fused<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
-    const uint64_t ntiles = uint64_t(1) << (nq - kt);
+    auto *kern = narrow ? k_fused<R, true> : k_fused<R, false>;
+    if (smem_max > 48 * 1024)
+        B200SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
+    const uint64_t namp = uint64_t(1) << nq, ntiles = narrow ? 1 : namp >> kt;
+    const unsigned threads = 1u << (kt - Geo<R>::a);
     const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)sm_count());
     for (const Piece &p : pieces) {
         if (!p.seg) {
@@ -1057,7 +1089,7 @@ void run_fused(void *state, uint32_t nq, const std::vector<GateDesc> &descs,
         a.ng = (int)p.s.gbits.size();
         std::memcpy(a.lbits, p.s.lbits.data(), p.s.lbits.size());
         std::memcpy(a.gbits, p.s.gbits.data(), p.s.gbits.size());
-        k_fused<R><<<grid, kFThreads, seg_smem(p.s), st>>>(static_cast<C<R> *>(state), a, ntiles);
+        kern<<<grid, threads, seg_smem(p.s), st>>>(static_cast<C<R> *>(state), a, ntiles, kt, namp);
         B200SV_CUDA(cudaGetLastError());
     }
 }
@@ -1162,13 +1194,22 @@ __device__ __forceinline__ double r_product(const C<R> (&v)[A], const C<R> (&w)[
     return p;
 }
 
-template <typename R>
-__global__ void __launch_bounds__(kFThreads, 1) k_fused_adj(C<R> *__restrict__ lam, C<R> *__restrict__ bra,
-                                                            AdjSegArgs a, uint64_t ntiles, double *partials) {
-    constexpr int KT = GeoA<R>::kt, A = GeoA<R>::A;
-    constexpr uint32_t TN = 1u << KT;
+// Several bras: blockIdx.y is the bra.  Every bra's CTAs take lambda's tiles through the segment
+// again beside their own bra's (twice the arithmetic of sharing lambda, but independent CTAs and
+// no launch per step: 11 qubits, 132 parameters, 3 observables went from 4.2 to 2.1 ms, of which
+// most is host work); lambda is read from lam_in and the first bra's CTAs write it to lam_out, a
+// second buffer (the same one when there is one bra).
+template <typename R, bool NARROW>
+__global__ void __launch_bounds__(kFThreads, 1) k_fused_adj(const C<R> *lam_in, C<R> *lam_out,
+                                                            C<R> *const *__restrict__ bras, AdjSegArgs a,
+                                                            uint64_t ntiles, double *partials, int kt, uint64_t namp) {
+    constexpr int A = GeoA<R>::A;
+    const int KT = NARROW ? kt : GeoA<R>::kt;
+    const uint32_t NT = NARROW ? blockDim.x : (uint32_t)kFThreads;
+    const uint32_t TN = 1u << KT;
     constexpr int V = 16 / (int)sizeof(C<R>);
-    constexpr int PER = (int)(TN / V) / kFThreads;
+    constexpr int PER = A / V;
+    C<R> *const bra = bras[blockIdx.y];
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t s_lbits[16], s_gbits[48];
     __shared__ uint64_t s_hi[PER];
@@ -1193,10 +1234,11 @@ __global__ void __launch_bounds__(kFThreads, 1) k_fused_adj(C<R> *__restrict__ l
     stage(scf, static_cast<const C<R> *>(a.coefs), a.ncoef);
     for (int i = threadIdx.x; i < a.nitems * kWarps; i += blockDim.x) sacc[i] = 0.0;
     __syncthreads();
-    if (threadIdx.x < PER) s_hi[threadIdx.x] = deposit((uint64_t)threadIdx.x * kFThreads * V, s_lbits, KT);
+    if (threadIdx.x < PER) s_hi[threadIdx.x] = deposit((uint64_t)threadIdx.x * NT * V, s_lbits, KT);
     __syncthreads();
     const uint64_t lo = deposit((uint64_t)threadIdx.x * V, s_lbits, KT);
-    auto sw = [&](int j) { return swz<R>((threadIdx.x + (uint32_t)j * kFThreads) * V); };
+    auto sw = [&](int j) { return swz<R>((threadIdx.x + (uint32_t)j * NT) * V); };
+    auto inside = [&](uint64_t x) { return !NARROW || x < namp; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     uint64_t t = blockIdx.x;
@@ -1206,8 +1248,14 @@ __global__ void __launch_bounds__(kFThreads, 1) k_fused_adj(C<R> *__restrict__ l
         C<R> *dl = buf + (2 * b) * TN, *db = buf + (2 * b + 1) * TN;
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            cp_async16(dl + sw(j), lam + (tb | lo | s_hi[j]));
-            cp_async16(db + sw(j), bra + (tb | lo | s_hi[j]));
+            const uint64_t x = tb | lo | s_hi[j];
+            if (inside(x)) {
+                cp_async16(dl + sw(j), lam_in + x);
+                cp_async16(db + sw(j), bra + x);
+            } else {
+                *reinterpret_cast<float4 *>(dl + sw(j)) = make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4 *>(db + sw(j)) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
     };
     if (t < ntiles) load(t, 0);
@@ -1267,8 +1315,10 @@ __global__ void __launch_bounds__(kFThreads, 1) k_fused_adj(C<R> *__restrict__ l
         }
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            *reinterpret_cast<float4 *>(lam + (tbase | lo | s_hi[j])) = *reinterpret_cast<const float4 *>(sl + sw(j));
-            *reinterpret_cast<float4 *>(bra + (tbase | lo | s_hi[j])) = *reinterpret_cast<const float4 *>(sb + sw(j));
+            const uint64_t x = tbase | lo | s_hi[j];
+            if (!inside(x)) continue;
+            if (blockIdx.y == 0) *reinterpret_cast<float4 *>(lam_out + x) = *reinterpret_cast<const float4 *>(sl + sw(j));
+            *reinterpret_cast<float4 *>(bra + x) = *reinterpret_cast<const float4 *>(sb + sw(j));
         }
         __syncthreads();
         cur ^= 1u;
@@ -1277,19 +1327,21 @@ __global__ void __launch_bounds__(kFThreads, 1) k_fused_adj(C<R> *__restrict__ l
     __syncthreads();
     for (int i = threadIdx.x; i < a.nitems; i += blockDim.x) {
         double sum = 0.0;
-        for (int wv = 0; wv < kWarps; ++wv) sum += sacc[i * kWarps + wv];
-        partials[(size_t)i * gridDim.x + blockIdx.x] = sum;
+        for (int wv = 0; wv < (int)(NT >> 5); ++wv) sum += sacc[i * kWarps + wv];
+        partials[((size_t)blockIdx.y * a.nitems + i) * gridDim.x + blockIdx.x] = sum;
     }
 }
 
-// jac[col[i]] = alpha[i] * sum_b partials[i * nb + b]   (one block per item, fixed order)
+// jac[col[i] * nobs + o] = alpha[i] * sum_b partials[(o * nitems + i) * nb + b]   (one block per item
+// and bra o, fixed order)
 __global__ void k_adj_fused_final(const double *__restrict__ partials, int nb, const double *__restrict__ alpha,
                                   const int64_t *__restrict__ col, double *__restrict__ jac) {
     __shared__ double sm[32];
     double s[1] = {0.0};
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) s[0] += partials[(size_t)blockIdx.x * nb + b];
+    const size_t at = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * nb;
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) s[0] += partials[at + b];
     block_reduce<1>(s, sm);
-    if (threadIdx.x == 0) jac[col[blockIdx.x]] = alpha[blockIdx.x] * s[0];
+    if (threadIdx.x == 0) jac[col[blockIdx.x] * gridDim.y + blockIdx.y] = alpha[blockIdx.x] * s[0];
 }
 
 // generator -> product record (false when the product has no register form)
@@ -1345,13 +1397,20 @@ int64_t prod_targets(const GateDesc &G, const std::vector<int> &loc) {
 }
 
 template <typename R>
-void run_fused_adjoint(void *lam, void *bra, uint32_t nq, const std::vector<AdjItem> &items,
-                       const std::function<void(size_t)> &exec_single, double *d_jac, cudaStream_t st) {
+void run_fused_adjoint(void *&lam, void *&lam2, const std::vector<void *> &bras, uint32_t nq,
+                       const std::vector<AdjItem> &items, const std::function<void(size_t)> &exec_single, double *d_jac,
+                       cudaStream_t st) {
     using G = GeoA<R>;
-    constexpr int kt = G::kt, a = G::a;
-    if ((int)nq < kt) throw Unsupported("state narrower than the adjoint tile");
+    constexpr int a = G::a;
+    const int kt = tile_width<G>(nq);
+    const bool narrow = (int)nq < G::kt;
+    const unsigned nobs = (unsigned)bras.size();
     const uint64_t low = (uint64_t(1) << G::reserve) - 1;
     const size_t n = items.size();
+    // bits of an item's generator that the tile must hold (a parity's bits may lie outside it)
+    auto gen_bits = [](const AdjItem &it) {
+        return it.diff && it.G.kind != Kind::Parity ? dep_bits(it.G) : uint64_t(0);
+    };
     // which items have a register form (checked with the tile-local map of a full tile)
     std::vector<int> ident(nq);
     for (uint32_t x = 0; x < nq; ++x) ident[x] = (int)x;
@@ -1394,7 +1453,7 @@ void run_fused_adjoint(void *lam, void *bra, uint32_t nq, const std::vector<AdjI
             uint64_t b = 0;
             bool fits = !blocked && fusable(it) && tile_bits(it.adj, b);
             if (fits) {
-                b |= it.diff ? dep_bits(it.G) : 0;
+                b |= gen_bits(it);
                 fits = __builtin_popcountll(used | b | low) <= kt && (int)take.size() + 1 <= kMaxAdjItems &&
                        ncf + coef_count(it.adj) <= kMaxAdjCoefs && nitems + (it.diff ? 1 : 0) <= kMaxAdjItems;
             }
@@ -1428,7 +1487,7 @@ void run_fused_adjoint(void *lam, void *bra, uint32_t nq, const std::vector<AdjI
         for (size_t j : pc.take) {
             uint64_t b = 0;
             tile_bits(items[j].adj, b);
-            used |= b | (items[j].diff ? dep_bits(items[j].G) : 0);
+            used |= b | gen_bits(items[j]);
         }
         std::vector<int> loc(nq, -1);
         uint64_t inl = used | low;
@@ -1441,6 +1500,7 @@ void run_fused_adjoint(void *lam, void *bra, uint32_t nq, const std::vector<AdjI
                 r.gbits.push_back((uint8_t)x);
             }
         }
+        for (int x = (int)nq; x < kt; ++x) r.lbits.push_back((uint8_t)x);  // a padded tile's upper bits
         // phases over the items in sweep order (no reordering inside a segment: products must
         // see exactly the steps before them)
         std::vector<const GateDesc *> cur;
@@ -1459,7 +1519,7 @@ void run_fused_adjoint(void *lam, void *bra, uint32_t nq, const std::vector<AdjI
                 r.alpha.push_back(it.alpha);
                 r.col.push_back(it.col);
             };
-            lower_phase<R, G>(r.sc, rmask, cur, loc, hook);
+            lower_phase<R, G>(r.sc, rmask, cur, loc, kt, hook);
             cur.clear();
             cur_items.clear();
             rmask = 0;
@@ -1478,12 +1538,15 @@ void run_fused_adjoint(void *lam, void *bra, uint32_t nq, const std::vector<AdjI
     }
     // device copies and launches
     const size_t tile_bytes = sizeof(C<R>) << kt;
-    const uint64_t ntiles = uint64_t(1) << (nq - kt);
-    const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)sm_count());
+    const uint64_t namp = uint64_t(1) << nq, ntiles = narrow ? 1 : namp >> kt;
+    const unsigned threads = 1u << (kt - a);
+    // one CTA per SM in all (64 KiB tiles of two states, double-buffered), at least one per bra
+    const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, std::max(1u, ((unsigned)sm_count() + nobs - 1) / nobs));
+    auto *kern = narrow ? k_fused_adj<R, true> : k_fused_adj<R, false>;
     size_t max_items = 1;
     for (auto &r : recs) max_items = std::max(max_items, r.alpha.size());
     double *d_partials = nullptr;
-    B200SV_CUDA(cudaMallocAsync((void **)&d_partials, max_items * grid * sizeof(double), st));
+    B200SV_CUDA(cudaMallocAsync((void **)&d_partials, max_items * grid * nobs * sizeof(double), st));
     std::vector<void *> frees{d_partials};
     struct Free {
         std::vector<void *> &p;
@@ -1502,8 +1565,8 @@ void run_fused_adjoint(void *lam, void *bra, uint32_t nq, const std::vector<AdjI
         const size_t bph = r.sc.phases.size() * sizeof(RPhase), brop = r.sc.rops.size() * sizeof(ROp),
                      bpr = r.prods.size() * sizeof(PProd), bg = r.gcf.size() * sizeof(double2),
                      bcf = r.sc.coefs.size() * sizeof(C<R>), bal = r.alpha.size() * sizeof(double),
-                     bco = r.col.size() * sizeof(int64_t);
-        std::vector<unsigned char> blob(bph + brop + bpr + bg + bcf + bal + bco + 64);
+                     bco = r.col.size() * sizeof(int64_t), bbr = nobs * sizeof(void *);
+        std::vector<unsigned char> blob(bph + brop + bpr + bg + bcf + bal + bco + bbr + 128);
         size_t off = 0;
         auto put = [&](const void *src, size_t bytes) {
             const size_t o = off;
@@ -1513,7 +1576,7 @@ void run_fused_adjoint(void *lam, void *bra, uint32_t nq, const std::vector<AdjI
         };
         const size_t o_ph = put(r.sc.phases.data(), bph), o_rop = put(r.sc.rops.data(), brop),
                      o_pr = put(r.prods.data(), bpr), o_g = put(r.gcf.data(), bg), o_cf = put(r.sc.coefs.data(), bcf),
-                     o_al = put(r.alpha.data(), bal), o_co = put(r.col.data(), bco);
+                     o_al = put(r.alpha.data(), bal), o_co = put(r.col.data(), bco), o_br = put(bras.data(), bbr);
         unsigned char *d_blob = nullptr;
         B200SV_CUDA(cudaMallocAsync((void **)&d_blob, std::max<size_t>(off, 16), st));
         frees.push_back(d_blob);
@@ -1535,12 +1598,16 @@ void run_fused_adjoint(void *lam, void *bra, uint32_t nq, const std::vector<AdjI
         std::memcpy(A.gbits, r.gbits.data(), r.gbits.size());
         const size_t smem = 4 * tile_bytes + bph + brop + bpr + bg + (size_t)A.nitems * kWarps * sizeof(double) + bcf;
         if (smem > 227 * 1024) throw Unsupported("fused adjoint segment exceeds shared memory");
-        B200SV_CUDA(cudaFuncSetAttribute(k_fused_adj<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_fused_adj<R><<<grid, kFThreads, smem, st>>>(static_cast<C<R> *>(lam), static_cast<C<R> *>(bra), A, ntiles,
-                                                      d_partials);
+        if (smem > 48 * 1024)
+            B200SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        C<R> *const out = static_cast<C<R> *>(nobs > 1 ? lam2 : lam);
+        kern<<<dim3(grid, nobs), threads, smem, st>>>(static_cast<const C<R> *>(lam), out,
+                                                      reinterpret_cast<C<R> *const *>(d_blob + o_br), A, ntiles,
+                                                      d_partials, kt, namp);
         B200SV_CUDA(cudaGetLastError());
+        if (nobs > 1) std::swap(lam, lam2);
         if (A.nitems) {
-            k_adj_fused_final<<<A.nitems, 128, 0, st>>>(d_partials, (int)grid,
+            k_adj_fused_final<<<dim3(A.nitems, nobs), 128, 0, st>>>(d_partials, (int)grid,
                                                          reinterpret_cast<const double *>(d_blob + o_al),
                                                          reinterpret_cast<const int64_t *>(d_blob + o_co), d_jac);
             B200SV_CUDA(cudaGetLastError());
@@ -1555,11 +1622,19 @@ int fused_tile_bits(int dtype, uint32_t nq) {
     return (int)std::min<uint32_t>(kt, nq);
 }
 
-// From one tile up: a narrow state leaves SMs idle during a segment, but one launch per
-// segment instead of one per gate is still the shorter path for L2-resident states, where
-// per-gate launches are bound by launch latency.
-bool fused_worthwhile(int dtype, uint32_t nq) {
-    return nq >= (uint32_t)(dtype == B200SV_C64 ? Geo<float>::kt : Geo<double>::kt);
+// A state narrower than a tile is fused from four gates on: the records' upload and the launch
+// cost about as much as three gate launches.  While its stream is being captured it stays on the
+// per-gate launches, whose coefficients are kernel arguments: a replay must not read the records
+// from this call's host memory.  From one tile up every call is fused.
+bool fused_worthwhile(int dtype, uint32_t nq, size_t ngates, cudaStream_t st) {
+    if (nq >= (uint32_t)(dtype == B200SV_C64 ? Geo<float>::kt : Geo<double>::kt)) return true;
+    if (ngates < 4) return false;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return status == cudaStreamCaptureStatusNone;
 }
 
 void apply_fused(void *state, uint32_t nq, int dtype, const std::vector<GateDesc> &descs,
@@ -1569,15 +1644,12 @@ void apply_fused(void *state, uint32_t nq, int dtype, const std::vector<GateDesc
     else run_fused<double>(state, nq, descs, apply_single, st);
 }
 
-bool fused_adjoint_worthwhile(int dtype, uint32_t nq) {
-    return nq >= (uint32_t)(dtype == B200SV_C64 ? GeoA<float>::kt : GeoA<double>::kt);
-}
-
-void apply_fused_adjoint(void *lambda, void *bra, uint32_t nq, int dtype, const std::vector<AdjItem> &items,
-                         const std::function<void(size_t)> &exec_single, double *d_jac, cudaStream_t st) {
+void apply_fused_adjoint(void *&lambda, void *&lambda2, const std::vector<void *> &bras, uint32_t nq, int dtype,
+                         const std::vector<AdjItem> &items, const std::function<void(size_t)> &exec_single,
+                         double *d_jac, cudaStream_t st) {
     if (nq > 48 + 16) throw Unsupported("state too wide for the fused path");
-    if (dtype == B200SV_C64) run_fused_adjoint<float>(lambda, bra, nq, items, exec_single, d_jac, st);
-    else run_fused_adjoint<double>(lambda, bra, nq, items, exec_single, d_jac, st);
+    if (dtype == B200SV_C64) run_fused_adjoint<float>(lambda, lambda2, bras, nq, items, exec_single, d_jac, st);
+    else run_fused_adjoint<double>(lambda, lambda2, bras, nq, items, exec_single, d_jac, st);
 }
 
 }  // namespace b200sv

@@ -260,3 +260,44 @@ def test_adjoint_fused_sweep_every_generator(capi, dtype):
     assert np.abs(got2[0] - got[0]).max() < tol
     want2 = O.adjoint_jacobian(st, ops, [[(1.0, [("PauliZ", [7])])]], tp)
     assert np.abs(got2[1] - want2[0]).max() < tol
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 6, 7, 8, 9, 10, 11, 12, 14])
+def test_fused_narrow_states(capi, n, dtype):
+    """States around and below one shared-memory tile (padded below a warp of threads): every gate
+    kind that fits the width through apply_ops_fused, and the Jacobian of one and of three
+    observables, against the oracle.  Tolerances: as the other fused tests, 1e-12 and 2e-5."""
+    import lq_oracle as O
+    from lightning_b200.workloads import random_unitary
+    rng = np.random.default_rng(100 + n)
+    kinds = {"RX": (1, 1), "RY": (1, 1), "RZ": (1, 1), "PhaseShift": (1, 1), "Hadamard": (1, 0), "PauliX": (1, 0),
+             "CNOT": (2, 0), "CZ": (2, 0), "SWAP": (2, 0), "CRY": (2, 1), "ControlledPhaseShift": (2, 1),
+             "IsingXY": (2, 1), "IsingZZ": (2, 1), "SingleExcitationPlus": (2, 1), "Toffoli": (3, 0), "CSWAP": (3, 0),
+             "DoubleExcitation": (4, 1), "DoubleExcitationMinus": (4, 1)}
+    names = [k for k, (w, _) in kinds.items() if w <= n]
+    ops = []
+    for _ in range(70):
+        name = names[int(rng.integers(len(names)))]
+        w, p = kinds[name]
+        ops.append((name, [int(x) for x in rng.choice(n, w, replace=False)], bool(rng.random() < 0.3),
+                    [float(rng.uniform(0, 2 * np.pi))] if p else []))
+    for k in range(1, min(n, 3) + 1):
+        ops.append(("QubitUnitary", [int(x) for x in rng.choice(n, k, replace=False)], False, [], random_unitary(rng, k)))
+    ops.append(("MultiRZ", list(range(n)), False, [0.4]))
+    tol = 1e-12 if dtype == np.complex128 else 2e-5
+    psi = (rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n))
+    psi = (psi / np.linalg.norm(psi)).astype(dtype)
+    sv = capi.StateVector(n, dtype)
+    sv.upload(psi)
+    sv.apply_ops_fused(ops)
+    assert np.abs(sv.download() - O.run_circuit(n, ops, state=psi.astype(np.complex128))).max() < tol
+    npar = sum(1 for op in ops if op[3])
+    tp = list(range(0, npar, 2))
+    obs = [[(1.0, [("PauliZ", [0])])], [(0.5, [("PauliX", [n - 1])]), (-0.3, [("PauliZ", [n // 2])])],
+           [(1.0, [("PauliY", [n - 1])])]]
+    st = sv.download()
+    for o in (obs[1:2], obs):
+        got = sv.adjoint_jacobian(ops, o, tp)
+        assert np.abs(got - O.adjoint_jacobian(st.astype(np.complex128), ops, o, tp)).max() < tol
+    assert np.array_equal(sv.download(), st)
