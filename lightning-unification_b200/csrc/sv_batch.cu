@@ -175,8 +175,8 @@ __global__ void k_trig(const double *__restrict__ params, uint64_t n, double4 *_
 // Coefficients of a gate (or of its adjoint): MAT1 -> 4, MAT2 -> 16, DIAG -> 2^nt, PARITY -> 2.
 // NM: 16 for two-wire dense steps (F_MAT2), 4 for every other form; an array of exactly
 // that size keeps the coefficients of the common steps in few registers.
-template <typename R, int NM>
-__device__ __forceinline__ void op_coeffs(const DOp &op, const double4 *__restrict__ cs,
+template <typename R, int NM, typename OP>
+__device__ __forceinline__ void op_coeffs(const OP &op, const double4 *__restrict__ cs,
                                           const double2 *__restrict__ consts, bool adj, C<R> (&m)[NM]) {
     if (op.gate == kConstGate) {
         const double2 *c = consts + (size_t)op.cidx * 16;
@@ -248,8 +248,8 @@ __device__ __forceinline__ void op_coeffs(const DOp &op, const double4 *__restri
 }
 
 // 2x2 matrix of a run member (single-wire gate on the run bit), or of its adjoint.
-template <typename R>
-__device__ __forceinline__ void member_mat(const DOp &op, const double4 *__restrict__ cs,
+template <typename R, typename OP>
+__device__ __forceinline__ void member_mat(const OP &op, const double4 *__restrict__ cs,
                                            const double2 *__restrict__ consts, bool adj, C<R> (&m)[4]) {
     const C<R> zero = mk<R>(0, 0), one = mk<R>(1, 0);
     if (op.form == F_SWAP) {
@@ -517,35 +517,7 @@ template <typename R, int CODE>
 __device__ __forceinline__ double pair_gen_im_k(C<R> a0, C<R> a1, C<R> b0, C<R> b1);
 
 // per-thread part of Im<bra|G|ket> on one tile, FP64
-// sum over groups of Im(conj(bra) . G ket) for a 2^K x 2^K generator G (FP64)
-template <typename R, int K>
-__device__ __forceinline__ double gen_inner_k(const C<R> *bra, const C<R> *ket, const Range &rg, const DOp &op,
-                                              const double2 *__restrict__ G) {
-    constexpr int D = 1 << K;
-    double acc = 0.0;
-    for (uint32_t g = rg.g0; g < rg.g1; g += rg.gs) {
-        const uint32_t base = ins_local(g, op.glow, op.gnb);
-        double2 v[D];
-#pragma unroll
-        for (int r = 0; r < D; ++r) v[r] = widen<R>(ket[base + op.goff[r]]);
-#pragma unroll
-        for (int r = 0; r < D; ++r) {
-            double wr = 0, wi = 0;
-#pragma unroll
-            for (int c = 0; c < D; ++c) {
-                const double2 x = G[r * D + c];
-                wr += x.x * v[c].x - x.y * v[c].y;
-                wi += x.x * v[c].y + x.y * v[c].x;
-            }
-            const double2 b = widen<R>(bra[base + op.goff[r]]);
-            acc += b.x * wi - b.y * wr;
-        }
-    }
-    return acc;
-}
-
-// FULL: the batch holds two-wire dense steps or generators (compiled only into the full kernel)
-template <typename R, bool FULL>
+template <typename R>
 __device__ __forceinline__ double gen_inner(const C<R> *bra, const C<R> *ket, int kt, int wl, bool wloc, const DOp &op,
                                             const double2 *__restrict__ consts) {
     double acc = 0.0;
@@ -558,53 +530,48 @@ __device__ __forceinline__ double gen_inner(const C<R> *bra, const C<R> *ket, in
         }
         return acc;
     }
-    if constexpr (FULL) {
-        if (op.gform == G_PAIR4) {
-            // Y on rows (0011, 1100); gamma_g times the identity on the other rows
-            const Range rg = groups(kt, wl, 4, wloc);
-            const uint32_t opa = op.off[2] | op.off[3], opb = op.off[0] | op.off[1];
-            const double gg = op.gk == 1 ? 1.0 : op.gk == 2 ? -1.0 : 0.0;
-            for (uint32_t g = rg.g0; g < rg.g1; g += rg.gs) {
-                const uint32_t base = ins_local(g, op.low, 4) | op.cmask;
-                acc += pair_gen_im_k<R, 2>(ket[base + opa], ket[base + opb], bra[base + opa], bra[base + opb]);
-                if (gg != 0.0) {
-                    double o = 0.0;
-#pragma unroll
-                    for (int r = 0; r < 16; ++r) {
-                        if (r == 3 || r == 12) continue;
-                        const uint32_t i = base + row_offset<4>(op.off, r);
-                        const double2 k = widen<R>(ket[i]), b = widen<R>(bra[i]);
-                        o += b.x * k.y - b.y * k.x;
-                    }
-                    acc += gg * o;
-                }
-            }
-            return acc;
-        }
-    }
-    const double2 *G = consts + (size_t)op.gcidx * 16;
-    const Range rg = groups(kt, wl, op.gnb, wloc);
-    if constexpr (FULL) {
-        // general size (one or two wires), loops over the run-time size
-        const int D = 1 << op.gk;
+    if (op.gform == G_PAIR4) {
+        // Y on rows (0011, 1100); gamma_g times the identity on the other rows
+        const Range rg = groups(kt, wl, 4, wloc);
+        const uint32_t opa = op.off[2] | op.off[3], opb = op.off[0] | op.off[1];
+        const double gg = op.gk == 1 ? 1.0 : op.gk == 2 ? -1.0 : 0.0;
         for (uint32_t g = rg.g0; g < rg.g1; g += rg.gs) {
-            const uint32_t base = ins_local(g, op.glow, op.gnb);
-            double2 v[4];
-            for (int r = 0; r < D; ++r) v[r] = widen<R>(ket[base + op.goff[r]]);
-            for (int r = 0; r < D; ++r) {
-                double wr = 0, wi = 0;
-                for (int c = 0; c < D; ++c) {
-                    const double2 x = G[r * D + c];
-                    wr += x.x * v[c].x - x.y * v[c].y;
-                    wi += x.x * v[c].y + x.y * v[c].x;
+            const uint32_t base = ins_local(g, op.low, 4) | op.cmask;
+            acc += pair_gen_im_k<R, 2>(ket[base + opa], ket[base + opb], bra[base + opa], bra[base + opb]);
+            if (gg != 0.0) {
+                double o = 0.0;
+#pragma unroll
+                for (int r = 0; r < 16; ++r) {
+                    if (r == 3 || r == 12) continue;
+                    const uint32_t i = base + row_offset<4>(op.off, r);
+                    const double2 k = widen<R>(ket[i]), b = widen<R>(bra[i]);
+                    o += b.x * k.y - b.y * k.x;
                 }
-                const double2 b = widen<R>(bra[base + op.goff[r]]);
-                acc += b.x * wi - b.y * wr;
+                acc += gg * o;
             }
         }
         return acc;
     }
-    return gen_inner_k<R, 1>(bra, ket, rg, op, G);
+    const double2 *G = consts + (size_t)op.gcidx * 16;
+    const Range rg = groups(kt, wl, op.gnb, wloc);
+    // general size (one or two wires), loops over the run-time size
+    const int D = 1 << op.gk;
+    for (uint32_t g = rg.g0; g < rg.g1; g += rg.gs) {
+        const uint32_t base = ins_local(g, op.glow, op.gnb);
+        double2 v[4];
+        for (int r = 0; r < D; ++r) v[r] = widen<R>(ket[base + op.goff[r]]);
+        for (int r = 0; r < D; ++r) {
+            double wr = 0, wi = 0;
+            for (int c = 0; c < D; ++c) {
+                const double2 x = G[r * D + c];
+                wr += x.x * v[c].x - x.y * v[c].y;
+                wi += x.x * v[c].y + x.y * v[c].x;
+            }
+            const double2 b = widen<R>(bra[base + op.goff[r]]);
+            acc += b.x * wi - b.y * wr;
+        }
+    }
+    return acc;
 }
 
 __device__ __forceinline__ void add_grad(double *gradw, int32_t gslot, double p, bool first) {
@@ -1163,7 +1130,7 @@ __device__ void store_tile(C<R> *__restrict__ dst, const C<R> *src, const DSeg &
 
 // Apply the gates of one segment to the tile(s): forward (NS = 1) or the adjoint
 // sweep over (lambda, bra) with gradient products (NS = 2, REV).
-template <typename R, int NS, bool REV, bool FULL>
+template <typename R, int NS, bool REV>
 __device__ void exec_segment(const KArgs &A, C<R> *const (&tiles)[NS], int kt, const DSeg &sg, const DOp *ops,
                              const C<R> (*cf)[4], bool first_tile) {
     const int wl = kt - (31 - __clz((int)(blockDim.x >> 5)));  // bits owned by one warp's block
@@ -1205,24 +1172,17 @@ __device__ void exec_segment(const KArgs &A, C<R> *const (&tiles)[NS], int kt, c
         } else {
             const DOp op = *op0;
             if (REV && op.gslot >= 0) {
-                add_grad(A.gradw, op.gslot, gen_inner<R, FULL>(tiles[NS - 1], tiles[0], kt, wl, wloc, op, A.consts),
+                add_grad(A.gradw, op.gslot, gen_inner<R>(tiles[NS - 1], tiles[0], kt, wl, wloc, op, A.consts),
                          first_tile);
                 if (wloc) __syncwarp();
                 else __syncthreads();
             }
-            if constexpr (FULL) {
-                if (op.form == F_MATK) {
-                    apply_matk<R, NS>(tiles, kt, wl, wloc, op, A.consts, REV);
-                } else {
-                    C<R> m[16];
-                    op_coeffs<R, 16>(op, A.cs, A.consts, REV, m);
-                    apply_op_general<R, NS>(tiles, kt, wl, wloc, op, m);
-                }
+            if (op.form == F_MATK) {
+                apply_matk<R, NS>(tiles, kt, wl, wloc, op, A.consts, REV);
             } else {
-                C<R> m[4];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) m[r] = cf[head][r];
-                apply_op<R, NS>(tiles, kt, wl, wloc, op, m);
+                C<R> m[16];
+                op_coeffs<R, 16>(op, A.cs, A.consts, REV, m);
+                apply_op_general<R, NS>(tiles, kt, wl, wloc, op, m);
             }
         }
         prev_wloc = wloc;
@@ -1280,7 +1240,7 @@ __device__ __forceinline__ const DTerm *stage_terms(DTerm *s_terms, const KArgs 
 }
 
 // one circuit, forward: state ends in tile 0 (resident) or pool A (global)
-template <typename R, bool FULL>
+template <typename R>
 __device__ void run_forward(const KArgs &A, const DCirc &c, C<R> *sm, C<R> *pa, DSeg *s_seg, DOp *s_ops,
                             C<R> (*s_cf)[4]) {
     const uint32_t tn = 1u << c.kt;
@@ -1291,7 +1251,7 @@ __device__ void run_forward(const KArgs &A, const DCirc &c, C<R> *sm, C<R> *pa, 
         if (threadIdx.x == 0) sm[0] = mk<R>(1, 0);
         for (uint32_t si = 0; si < c.nseg; ++si) {
             const DSeg &sg = stage_segment<R>(s_seg, s_ops, s_cf, A, c.seg_begin + si, false);
-            exec_segment<R, 1, false, FULL>(A, tiles, c.kt, sg, s_ops, s_cf, true);
+            exec_segment<R, 1, false>(A, tiles, c.kt, sg, s_ops, s_cf, true);
         }
         return;
     }
@@ -1308,7 +1268,7 @@ __device__ void run_forward(const KArgs &A, const DCirc &c, C<R> *sm, C<R> *pa, 
                 load_tile<R>(sm, pa, sg, tbase, tn);
                 tile_wait();
             }
-            exec_segment<R, 1, false, FULL>(A, tiles, c.kt, sg, s_ops, s_cf, true);
+            exec_segment<R, 1, false>(A, tiles, c.kt, sg, s_ops, s_cf, true);
             store_tile<R>(pa, sm, sg, tbase, tn);
             __syncthreads();
         }
@@ -1338,12 +1298,12 @@ __global__ void k_rev_coeffs(const DOp *__restrict__ ops, uint32_t nops, const d
 }
 
 // MODE 0: forward expectation values; MODE 1: forward (unless reused) and the VJP sweep.
-// FULL: compiled with the two-wire dense step and generator paths (only batches that
-// hold such gates launch it; the others get a kernel without them, in fewer registers).
+// Runs the batches that hold two-wire dense gates, double excitations or wider matrices; all others
+// run level by level (sv_batch_tiles.cuh).
 // Compiled for 512 threads (128 registers a thread).  Instantiations for 256 threads with up to
 // 255 registers (no spills in the complex128 steps) were tried: the autotuner kept 512 threads
 // for every workload of the bench (complex128 HEA batch 1027 ms either way).
-template <typename R, int MODE, bool FULL>
+template <typename R, int MODE>
 __global__ void __launch_bounds__(512) k_batch(KArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_next;
@@ -1364,7 +1324,7 @@ __global__ void __launch_bounds__(512) k_batch(KArgs A) {
         C<R> *pb = static_cast<C<R> *>(A.pool_b) + c.off_b;
         const uint64_t namp = uint64_t(1) << c.n;
         const bool reuse = MODE == 1 && !c.resident && A.reuse && *A.reuse != 0;
-        if (!reuse) run_forward<R, FULL>(A, c, sm0, pa, &s_seg, s_ops, s_cf);
+        if (!reuse) run_forward<R>(A, c, sm0, pa, &s_seg, s_ops, s_cf);
         const C<R> *psi = c.resident ? sm0 : pa;
         if (MODE == 0) {
             const DTerm *T = stage_terms(reinterpret_cast<DTerm *>(s_ops), A, c, nullptr);
@@ -1393,7 +1353,7 @@ __global__ void __launch_bounds__(512) k_batch(KArgs A) {
         if (c.resident) {
             for (int32_t si = (int32_t)c.nseg - 1; si >= 0; --si) {
                 const DSeg &sg = stage_segment<R>(&s_seg, s_ops, s_cf, A, c.seg_begin + si, true);
-                exec_segment<R, 2, true, FULL>(A, tiles, c.kt, sg, s_ops, s_cf, true);
+                exec_segment<R, 2, true>(A, tiles, c.kt, sg, s_ops, s_cf, true);
             }
             continue;
         }
@@ -1406,7 +1366,7 @@ __global__ void __launch_bounds__(512) k_batch(KArgs A) {
                 load_tile<R>(sm0, pa, sg, tbase, tn);
                 load_tile<R>(sm1, pb, sg, tbase, tn);
                 tile_wait();
-                exec_segment<R, 2, true, FULL>(A, tiles, c.kt, sg, s_ops, s_cf, t == 0);
+                exec_segment<R, 2, true>(A, tiles, c.kt, sg, s_ops, s_cf, t == 0);
                 store_tile<R>(pa, sm0, sg, tbase, tn);
                 store_tile<R>(pb, sm1, sg, tbase, tn);
                 __syncthreads();
@@ -1457,6 +1417,8 @@ __global__ void k_onehot_dy(double *dy, const DCirc *circs, uint32_t ncirc, uint
         for (uint32_t o = 0; o < circs[c].nobs; ++o) dy[circs[c].out_begin + o] = (o == obs) ? 1.0 : 0.0;
 }
 
+#include "sv_batch_tiles.cuh"
+
 // ---------------------------------------------------------------------------
 // host side
 struct Config {
@@ -1486,8 +1448,12 @@ struct Batch {
     uint32_t ncirc = 0;
     Config cfg;
     bool use_graphs = false;
-    bool full = false;  // the program holds two-wire dense steps or generators
-    uint32_t last_launches = 0;
+    bool full = false;  // some gate needs k_batch (two-wire dense, double excitation, wide matrix)
+    uint32_t launched = 0;  // kernels enqueued by the call being recorded
+    uint32_t last_launches = 0, graph_launches[2] = {0, 0};
+    std::unique_ptr<tiles::Program> tp;  // the level program (not full)
+    cudaStream_t side[4] = {};           // narrower circuit classes of the level program
+    cudaEvent_t fork = nullptr, join[4] = {};
 
     // circuit descriptions kept for re-planning
     std::vector<uint32_t> nq;
@@ -1534,6 +1500,11 @@ struct Batch {
         if (g_forward) cudaGraphExecDestroy(g_forward);
         if (g_vjp) cudaGraphExecDestroy(g_vjp);
         for (void *p : allocs) cudaFree(p);
+        for (int k = 0; k < 4; ++k) {
+            if (side[k]) cudaStreamDestroy(side[k]);
+            if (join[k]) cudaEventDestroy(join[k]);
+        }
+        if (fork) cudaEventDestroy(fork);
         if (own) cudaStreamDestroy(own);
     }
     template <typename T> T *dalloc(size_t count) {
@@ -1548,6 +1519,8 @@ struct Batch {
         for (void *p : allocs) cudaFree(p);
         allocs.clear();
     }
+    // values per gradient slot: one per warp in k_batch
+    int grad_words() const { return full ? cfg.threads / 32 : 1; }
     size_t amp() const { return dtype == B200SV_C64 ? 8 : 16; }
 };
 
@@ -2014,12 +1987,9 @@ Planned plan(const Batch &B, const Config &cfg, bool vjp) {
     return P;
 }
 
-template <typename R> const void *batch_kernel_r(int mode, bool full) {
-    if (full) return mode ? (const void *)k_batch<R, 1, true> : (const void *)k_batch<R, 0, true>;
-    return mode ? (const void *)k_batch<R, 1, false> : (const void *)k_batch<R, 0, false>;
-}
-const void *batch_kernel(int dtype, int mode, bool full) {
-    return dtype == B200SV_C64 ? batch_kernel_r<float>(mode, full) : batch_kernel_r<double>(mode, full);
+const void *batch_kernel(int dtype, int mode) {
+    if (dtype == B200SV_C64) return mode ? (const void *)k_batch<float, 1> : (const void *)k_batch<float, 0>;
+    return mode ? (const void *)k_batch<double, 1> : (const void *)k_batch<double, 0>;
 }
 
 template <typename T> void upload(Batch &B, T *&dst, const std::vector<T> &src) {
@@ -2028,12 +1998,26 @@ template <typename T> void upload(Batch &B, T *&dst, const std::vector<T> &src) 
         B200SV_CUDA(cudaMemcpy(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
 }
 
+#include "sv_batch_levels.hpp"
+
 // Build the device program for a configuration (both forward and VJP share it:
 // the VJP layout is a superset).
 void build_program(Batch &B, const Config &cfg) {
     B.free_program();
-    Planned P = plan(B, cfg, true);
     B.cfg = cfg;
+    B.tp.reset();
+    B.full = false;
+    for (const auto &ops : B.hops)
+        for (const HostOp &h : ops) B.full = B.full || !tiles::serves(h);
+    Planned P;
+    if (B.full) {
+        P = plan(B, cfg, true);
+    } else {
+        P.consts.reserve(1024);
+        push_const(P, {});  // slot 0 unused
+        if (B.dtype == B200SV_C64) tiles::build<float>(B, P);
+        else tiles::build<double>(B, P);
+    }
     upload(B, B.d_circs, P.circs);
     upload(B, B.d_segs, P.segs);
     upload(B, B.d_ops, P.ops);
@@ -2047,8 +2031,7 @@ void build_program(Batch &B, const Config &cfg) {
     B.d_pool_a = B.dalloc<unsigned char>(B.pool_a_bytes);
     B.d_pool_b = B.dalloc<unsigned char>(B.pool_b_bytes);
     B.ngslots = (uint32_t)P.gscale.size();
-    const int nw = cfg.threads / 32;
-    B.d_gradw = B.dalloc<double>((size_t)B.ngslots * nw);
+    B.d_gradw = B.dalloc<double>((size_t)B.ngslots * B.grad_words());
     upload(B, B.d_gscale, P.gscale);
     // CSR param -> gslots
     std::vector<uint32_t> rowptr(B.nparams + 1, 0), cols;
@@ -2090,6 +2073,10 @@ void build_program(Batch &B, const Config &cfg) {
     B.d_dy_in = B.dalloc<double>(B.total_obs);
     B.d_out = B.dalloc<double>(B.total_obs);
     B.d_grad = B.dalloc<double>(B.nparams);
+    if (!B.full) {
+        B200SV_CUDA(cudaDeviceSynchronize());
+        return;
+    }
     B.smem_bytes = (size_t)2 * (size_t(1) << P.max_kt) * B.amp();
     int dev = 0, maxsm = 0, nsm = sm_count();
     B200SV_CUDA(cudaGetDevice(&dev));
@@ -2098,14 +2085,9 @@ void build_program(Batch &B, const Config &cfg) {
                                kMaxSegOpsStaged * (sizeof(DOp) + 4 * B.amp());
     if (B.smem_bytes + static_smem > (size_t)maxsm)
         throw Unsupported("batch: tile does not fit in shared memory; lower kt");
-    B.full = false;
-    for (const DOp &d : P.ops)
-        if (d.form == F_MAT2 || d.form == F_PAIR4 || d.form == F_MATK || (d.gform == G_MAT && d.gk == 2) ||
-            d.gform == G_PAIR4)
-            B.full = true;
     int per_sm = 1 << 30;
     for (int mode = 0; mode < 2; ++mode) {
-        const void *k = batch_kernel(B.dtype, mode, B.full);
+        const void *k = batch_kernel(B.dtype, mode);
         B200SV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B.smem_bytes));
         int m = 0;
         B200SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k, cfg.threads, B.smem_bytes));
@@ -2122,9 +2104,16 @@ void launch_trig(Batch &B, const double *params, cudaStream_t st) {
     const uint64_t nb = std::min<uint64_t>((B.nparams + 255) / 256, 4096);
     k_trig<<<(unsigned)nb, 256, 0, st>>>(params, B.nparams, B.d_cs);
     B200SV_CUDA(cudaGetLastError());
+    B.launched++;
 }
 
 void launch_main(Batch &B, int mode, const double *dy, double *out, const int *reuse, cudaStream_t st) {
+    if (!B.full) {
+        const bool f = B.dtype == B200SV_C64;
+        if (mode == 0) f ? tiles::forward<float>(B, out, st) : tiles::forward<double>(B, out, st);
+        else f ? tiles::reverse<float>(B, dy, reuse, st) : tiles::reverse<double>(B, dy, reuse, st);
+        return;
+    }
     KArgs A{};
     A.circs = B.d_circs;
     A.segs = B.d_segs;
@@ -2151,14 +2140,16 @@ void launch_main(Batch &B, int mode, const double *dy, double *out, const int *r
             k_rev_coeffs<double><<<nb, 256, 0, st>>>(B.d_ops, B.nops_total, B.d_cs, B.d_consts,
                                                       static_cast<C<double>(*)[4]>(B.d_rcf));
         B200SV_CUDA(cudaGetLastError());
+        B.launched++;
     }
     int mk = 1;
     for (auto &c : B.h_circs) mk = std::max<int>(mk, (int)c.kt);
     A.max_kt = mk;
     B200SV_CUDA(cudaMemsetAsync(B.d_counter, 0, sizeof(uint32_t), st));
     void *args[] = {&A};
-    const void *k = batch_kernel(B.dtype, mode, B.full);
+    const void *k = batch_kernel(B.dtype, mode);
     B200SV_CUDA(cudaLaunchKernel(k, dim3(B.grid), dim3(B.cfg.threads), args, B.smem_bytes, st));
+    B.launched++;
 }
 
 // Forward: expectation values; the final states of circuits wider than a tile stay
@@ -2182,20 +2173,24 @@ void enqueue_vjp(Batch &B, cudaStream_t st) {
         const uint64_t nb = std::min<uint64_t>((B.nparams + 255) / 256, 4096);
         k_params_equal<<<(unsigned)nb, 256, 0, st>>>(B.d_params_in, B.d_params_fwd, B.nparams, B.d_reuse);
         B200SV_CUDA(cudaGetLastError());
+        B.launched++;
     }
     launch_main(B, 1, B.d_dy_in, nullptr, B.d_reuse, st);
     B200SV_CUDA(cudaMemsetAsync(B.d_fwd_valid, 0, sizeof(int), st));
-    const int nw = B.cfg.threads / 32;
+    const int nw = B.grad_words();
     const uint64_t np = std::max<uint64_t>(B.nparams, 1);
     k_grad_params<<<(unsigned)std::min<uint64_t>((np + 255) / 256, 4096), 256, 0, st>>>(
         B.d_rowptr, B.d_cols, B.d_gscale, B.d_gradw, nw, B.nparams, B.d_grad);
     B200SV_CUDA(cudaGetLastError());
+    B.launched++;
 }
 
-template <class F> void run_maybe_graph(Batch &B, cudaGraphExec_t &exec, F &&enqueue) {
+template <class F> void run_maybe_graph(Batch &B, cudaGraphExec_t &exec, uint32_t &count, F &&enqueue) {
     cudaStream_t st = B.stream();
+    B.launched = 0;
     if (!B.use_graphs) {
         enqueue(st);
+        B.last_launches = B.launched;
         return;
     }
     if (!exec) {
@@ -2215,8 +2210,10 @@ template <class F> void run_maybe_graph(Batch &B, cudaGraphExec_t &exec, F &&enq
         const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
         cudaGraphDestroy(g);
         B200SV_CUDA(e);
+        count = B.launched;
     }
     B200SV_CUDA(cudaGraphLaunch(exec, st));
+    B.last_launches = count;
 }
 
 }  // namespace batch
@@ -2249,6 +2246,11 @@ int b200sv_batch_create(int dtype, const b200sv_batch_circuit *circuits, uint32_
         B->ncirc = ncircuits;
         B200SV_CUDA(cudaGetDevice(&B->device));
         B200SV_CUDA(cudaStreamCreateWithFlags(&B->own, cudaStreamNonBlocking));
+        for (int k = 0; k < 4; ++k) {
+            B200SV_CUDA(cudaStreamCreateWithFlags(&B->side[k], cudaStreamNonBlocking));
+            B200SV_CUDA(cudaEventCreateWithFlags(&B->join[k], cudaEventDisableTiming));
+        }
+        B200SV_CUDA(cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming));
         for (uint32_t c = 0; c < ncircuits; ++c) {
             const b200sv_batch_circuit &bc = circuits[c];
             if (bc.num_qubits < 1 || bc.num_qubits > 30) throw ArgError("batch circuits have 1..30 qubits");
@@ -2335,9 +2337,8 @@ int b200sv_batch_forward(b200sv_batch_handle bh, const double *params, double *o
         cudaStream_t st = B.stream();
         if (B.nparams)
             B200SV_CUDA(cudaMemcpyAsync(B.d_params_in, params, B.nparams * sizeof(double), cudaMemcpyDeviceToDevice, st));
-        run_maybe_graph(B, B.g_forward, [&](cudaStream_t s) { enqueue_forward(B, s); });
+        run_maybe_graph(B, B.g_forward, B.graph_launches[0], [&](cudaStream_t s) { enqueue_forward(B, s); });
         B200SV_CUDA(cudaMemcpyAsync(out, B.d_out, B.total_obs * sizeof(double), cudaMemcpyDeviceToDevice, st));
-        B.last_launches = 2;  // k_trig, k_batch
     });
 }
 
@@ -2350,10 +2351,9 @@ int b200sv_batch_vjp(b200sv_batch_handle bh, const double *params, const double 
         if (B.nparams)
             B200SV_CUDA(cudaMemcpyAsync(B.d_params_in, params, B.nparams * sizeof(double), cudaMemcpyDeviceToDevice, st));
         B200SV_CUDA(cudaMemcpyAsync(B.d_dy_in, dy, B.total_obs * sizeof(double), cudaMemcpyDeviceToDevice, st));
-        run_maybe_graph(B, B.g_vjp, [&](cudaStream_t s) { enqueue_vjp(B, s); });
+        run_maybe_graph(B, B.g_vjp, B.graph_launches[1], [&](cudaStream_t s) { enqueue_vjp(B, s); });
         if (B.nparams)
             B200SV_CUDA(cudaMemcpyAsync(grad, B.d_grad, B.nparams * sizeof(double), cudaMemcpyDeviceToDevice, st));
-        B.last_launches = 5;  // k_trig, k_params_equal, k_rev_coeffs, k_batch, k_grad_params
     });
 }
 
@@ -2367,8 +2367,8 @@ int b200sv_batch_jacobian(b200sv_batch_handle bh, const double *params, double *
             B200SV_CUDA(cudaMemcpyAsync(B.d_params_in, params, B.nparams * sizeof(double), cudaMemcpyDeviceToDevice, st));
         uint32_t maxobs = 0;
         for (auto n : B.nobs) maxobs = std::max(maxobs, n);
-        const int nw = B.cfg.threads / 32;
-        uint32_t launches = 1;
+        const int nw = B.grad_words();
+        B.launched = 0;
         B200SV_CUDA(cudaMemsetAsync(B.d_fwd_valid, 0, sizeof(int), st));
         launch_trig(B, B.d_params_in, st);
         for (uint32_t o = 0; o < maxobs; ++o) {
@@ -2379,9 +2379,9 @@ int b200sv_batch_jacobian(b200sv_batch_handle bh, const double *params, double *
                     B.d_gscale, B.d_gradw, nw, B.ngslots, o, B.d_gslot_circ, B.d_circs, B.d_jac_base,
                     B.d_gslot_col, B.d_circ_ncols, jac);
             B200SV_CUDA(cudaGetLastError());
-            launches += 4;  // k_onehot_dy, k_rev_coeffs, k_batch, k_grad_scatter
+            B.launched += 2;  // k_onehot_dy, k_grad_scatter
         }
-        B.last_launches = launches;
+        B.last_launches = B.launched;
     });
 }
 
@@ -2395,8 +2395,10 @@ int b200sv_batch_autotune(b200sv_batch_handle bh, const double *params, int *cho
         std::vector<Config> cands;
         const int kts_c64[] = {11, 12, 13};
         const int kts_c128[] = {10, 11, 12};
-        for (int th : {256, 512})
+        for (int th : {256, 512}) {
+            if (!B.full && th != 256) continue;  // the level program's block size follows from the tile
             for (int i = 0; i < 3; ++i) cands.push_back(Config{th, B.dtype == B200SV_C64 ? kts_c64[i] : kts_c128[i]});
+        }
         float best = 1e30f;
         int best_i = -1;
         std::vector<double> saved_params(B.nparams);

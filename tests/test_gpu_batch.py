@@ -463,3 +463,71 @@ def hea_batch_small_many_obs():
     circuits[0] = dict(circuits[0], observables=obs0[:37])
     circuits[1] = dict(circuits[1], observables=[[(1.0, "Z", [q])] for q in range(5)])
     return circuits, params
+
+
+def level_batch(widths, seed=77):
+    """Random circuits of every gate the level engine serves, one per width."""
+    rng = np.random.default_rng(seed)
+    kinds = {"RX": (1, 1), "RY": (1, 1), "RZ": (1, 1), "PhaseShift": (1, 1), "Hadamard": (1, 0), "PauliX": (1, 0),
+             "PauliY": (1, 0), "S": (1, 0), "T": (1, 0), "CNOT": (2, 0), "CZ": (2, 0), "CY": (2, 0), "SWAP": (2, 0),
+             "CRX": (2, 1), "CRY": (2, 1), "CRZ": (2, 1), "ControlledPhaseShift": (2, 1), "IsingZZ": (2, 1),
+             "Toffoli": (3, 0), "CSWAP": (3, 0), "MultiRZ": (0, 1), "Identity": (1, 0)}
+    circuits, params = [], []
+    for n in widths:
+        names = [k for k, (w, _) in kinds.items() if w <= n]
+        ops, pidx = [], []
+        for _ in range(90):
+            name = names[int(rng.integers(len(names)))]
+            w, p = kinds[name]
+            w = w or int(rng.integers(1, min(n, 12) + 1))
+            bound = p and rng.random() < 0.25  # a constant angle
+            ops.append((name, [int(x) for x in rng.choice(n, w, replace=False)], bool(rng.random() < 0.3),
+                        [float(rng.uniform(0, 6))] if bound else []))
+            pidx.append(len(params) if p and not bound else -1)
+            if p and not bound:
+                params.append(float(rng.uniform(0, 2 * np.pi)))
+        u = np.linalg.qr(rng.normal(size=(2, 2)) + 1j * rng.normal(size=(2, 2)))[0]
+        ops.insert(45, ("QubitUnitary", [n // 2], False, [], u))
+        pidx.insert(45, -1)
+        obs = [[(1.0, "Z", [0])], [(0.7, "X", [n - 1]), (-0.4, "Z", [n // 2]), (0.2, "I", [0])], [(0.5, "Y", [n // 2])]]
+        if n >= 3:
+            obs.append([(0.9, "XYZ", [0, n // 2, n - 1]), (0.3, "YY", [0, n - 1]), (-1.1, "ZZ", [1, n - 1])])
+        circuits.append({"num_qubits": n, "ops": ops, "param_index": pidx, "observables": obs})
+    return circuits, np.array(params)
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+@pytest.mark.parametrize("widths", [(1, 2, 3), (7, 8, 9, 10, 11), (12, 13), (14, 15, 4, 14)])
+def test_batch_level_engine_every_gate(dtype, widths):
+    """Every gate of the level engine at widths around its tiles (a tile padded to a warp, one tile of
+    the state's own size, several tiles): outputs, VJP after a forward and on its own, and the
+    Jacobian, against the oracle."""
+    import torch
+    import lq_oracle as O
+    from lightning_b200.batch import BatchedCircuits
+    from lightning_b200.workloads import bind, obs_terms
+    circuits, params = level_batch(widths)
+    eng = BatchedCircuits(circuits, len(params), dtype=dtype)
+    p = torch.tensor(params, device="cuda")
+    dy = np.random.default_rng(3).normal(size=eng.total_obs)
+    out = eng.forward(p)
+    g = eng.vjp(p, torch.tensor(dy, device="cuda"))
+    alone = eng.vjp(p, torch.tensor(dy, device="cuda"))
+    jac = eng.jacobian(p).cpu().numpy()
+    assert torch.equal(g, alone)
+    tol = 1e-12 if dtype == np.complex128 else 2e-5
+    want_g, at, jat = np.zeros(len(params)), 0, 0
+    for c in circuits:
+        n, ops = c["num_qubits"], bind(c, params)
+        obs = [obs_terms(o) for o in c["observables"]]
+        psi = O.run_circuit(n, ops)
+        got = out[at:at + len(obs)].cpu().numpy()
+        assert np.abs(got - [O.expval(psi, o) for o in obs]).max() < tol
+        slots = [q for q in c["param_index"] if q >= 0]
+        which = [k for k, i in enumerate(i for i, op in enumerate(ops) if op[3]) if c["param_index"][i] >= 0]
+        J = O.adjoint_jacobian(psi, ops, obs, which)
+        want_g[slots] += dy[at:at + len(obs)] @ J
+        size = len(obs) * len(slots)
+        assert np.abs(jac[jat:jat + size].reshape(len(obs), -1) - J).max() < GRAD_TOL[dtype]
+        at, jat = at + len(obs), jat + size
+    assert np.abs(g.cpu().numpy() - want_g).max() < GRAD_TOL[dtype]
