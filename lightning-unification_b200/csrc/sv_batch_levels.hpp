@@ -16,10 +16,13 @@ bool serves(const HostOp &h) {
 // A step of a circuit: a run of single-wire gates on one bit, or one gate.
 struct Step {
     SKind kind = S_NONE;
-    bool swap = false, sign = false, diag = false, grad = false, wide = false;
+    bool swap = false, sign = false, grad = false, wide = false;
     std::vector<uint32_t> mems;     // op indices, in order
     std::vector<uint32_t> ctl, tgt; // state bits
     uint64_t mask = 0, targets = 0; // bits touched; bits that must be register bits
+    uint64_t flip = 0;              // bits on which the step is not diagonal: steps commute when every
+                                    // bit they share is diagonal in both
+    bool linear = false;            // CNOT, SWAP: between phases, in the tile's address map
     uint32_t dsign = 0;
 };
 
@@ -34,7 +37,6 @@ std::vector<Step> make_steps(const std::vector<HostOp> &ops, uint32_t n) {
             if (last[b] < 0 || (out[last[b]].kind != S_RUN && out[last[b]].kind != S_DIAGRUN)) {
                 Step s;
                 s.kind = S_DIAGRUN;
-                s.diag = true;
                 s.tgt = {b};
                 s.mask = uint64_t(1) << b;
                 last[b] = (int)out.size();
@@ -44,7 +46,7 @@ std::vector<Step> make_steps(const std::vector<HostOp> &ops, uint32_t n) {
             s.mems.push_back(i);
             if (h.form != F_DIAG) {
                 s.kind = S_RUN;
-                s.diag = false;
+                s.flip = s.mask;
             }
             s.grad = s.grad || h.diff;
             continue;
@@ -58,16 +60,17 @@ std::vector<Step> make_steps(const std::vector<HostOp> &ops, uint32_t n) {
         for (auto b : h.bits) s.mask |= uint64_t(1) << b;
         if (h.form == F_PARITY) {
             s.kind = S_PARITY;
-            s.diag = s.wide = true;
+            s.wide = true;
         } else if (h.form == F_SWAP) {
             s.swap = true;
-            for (auto b : s.tgt) s.targets |= uint64_t(1) << b;
+            for (auto b : s.tgt) s.flip |= uint64_t(1) << b;
+            s.linear = s.ctl.size() + s.tgt.size() == 2;
+            if (!s.linear) s.targets = s.flip;
         } else if (h.form == F_MAT1) {
             s.kind = S_DENSE;
-            s.targets = uint64_t(1) << s.tgt[0];
+            s.targets = s.flip = uint64_t(1) << s.tgt[0];
         } else {
             s.kind = S_DIAG;
-            s.diag = true;
             const bool cst = h.gate == kConstGate, all = h.nt == 0 && cst && h.cmat[0] == cd(-1, 0),
                        one = h.nt == 1 && cst && h.cmat[0] == cd(1, 0) && h.cmat[1] == cd(-1, 0);
             if (h.bits.size() == 2 && (all || one)) {  // CZ: a sign where both bits are set
@@ -146,14 +149,14 @@ template <typename R, bool REV> void plan_dir(Builder &B, Plan &P, uint32_t n, i
     while (left > 0 || (!REV && D.segs.empty())) {
         while (first < ns && done[first]) ++first;
         // the segment: every later step that fits the tile and commutes with the steps left out
-        uint64_t used = 0, any = 0, nondiag = 0;
+        uint64_t used = 0, any = 0, flipped = 0;  // of the steps left out
         int nops = 0, ncf = 0, ngr = 0;
         std::vector<uint32_t> take;
         for (size_t j = first; j < ns; ++j) {
             if (done[j]) continue;
             const Step &s = step(j);
             const uint64_t need = s.wide ? 0 : s.mask;
-            const bool fits = !(s.mask & (s.diag ? nondiag : any)) && __builtin_popcountll(used | need | low) <= kt &&
+            const bool fits = !(s.flip & any) && !(s.mask & flipped) && __builtin_popcountll(used | need | low) <= kt &&
                               nops < kMaxTOps && ncf + coef_slots(s, REV) <= kMaxTCoefs &&
                               ngr + (REV && s.grad ? 1 : 0) <= kMaxTGrads;
             if (fits) {
@@ -166,8 +169,8 @@ template <typename R, bool REV> void plan_dir(Builder &B, Plan &P, uint32_t n, i
                 --left;
             } else {
                 any |= s.mask;
-                if (!s.diag) nondiag |= s.mask;
-                if (nondiag == (uint64_t(1) << n) - 1) break;  // everything later is blocked
+                flipped |= s.flip;
+                if (flipped == (uint64_t(1) << n) - 1) break;  // everything later is blocked
             }
         }
         if (take.empty() && left > 0) throw Unsupported("batch: gate wider than the tile");
@@ -190,43 +193,70 @@ template <typename R, bool REV> void plan_dir(Builder &B, Plan &P, uint32_t n, i
         sg.op_begin = (uint32_t)B.ops.size();
         sg.coef_begin = D.ncoef;
         std::vector<uint32_t> grads;
-        // phases: every ready step whose targets fit the register bits, until nothing moves
+        // phases: the ready CNOTs and SWAPs go into the address map, then every ready step whose
+        // targets fit the register bits, until nothing moves
         std::vector<char> out(take.size(), 0);
         size_t rest = take.size();
+        uint16_t place[12];  // of each tile bit, before the swizzle
+        for (int b = 0; b < 12; ++b) place[b] = (uint16_t)(1u << b);
         while (rest > 0) {
             uint32_t rmask = 0;
             std::vector<uint32_t> cur;
-            for (bool progress = true; progress;) {
-                progress = false;
-                uint64_t la = 0, ln = 0;
-                for (size_t i = 0; i < take.size(); ++i) {
-                    if (out[i]) continue;
-                    const Step &s = step(take[i]);
-                    uint32_t need = 0;
-                    for (uint32_t x = 0; x < n; ++x)
-                        if ((targets(s) >> x) & 1) need |= 1u << loc[x];
-                    if (!(s.mask & (s.diag ? ln : la)) && __builtin_popcount(rmask | need) <= G::a) {
-                        rmask |= need;
-                        cur.push_back(take[i]);
-                        out[i] = 1;
-                        --rest;
-                        progress = true;
-                    } else {
-                        la |= s.mask;
-                        if (!s.diag) ln |= s.mask;
+            for (bool linear : {true, false}) {
+                for (bool progress = true; progress;) {
+                    progress = false;
+                    uint64_t la = 0, lf = 0;
+                    for (size_t i = 0; i < take.size(); ++i) {
+                        if (out[i]) continue;
+                        const Step &s = step(take[i]);
+                        uint32_t need = 0;
+                        for (uint32_t x = 0; x < n; ++x)
+                            if ((targets(s) >> x) & 1) need |= 1u << loc[x];
+                        if (s.linear == linear && !(s.flip & la) && !(s.mask & lf) &&
+                            __builtin_popcount(rmask | need) <= G::a) {
+                            out[i] = 1;
+                            --rest;
+                            progress = true;
+                            if (!linear) {
+                                rmask |= need;
+                                cur.push_back(take[i]);
+                            } else if (s.ctl.size() == 1) {
+                                place[loc[s.ctl[0]]] ^= place[loc[s.tgt[0]]];
+                            } else {
+                                std::swap(place[loc[s.tgt[0]]], place[loc[s.tgt[1]]]);
+                            }
+                        } else {
+                            la |= s.mask;
+                            lf |= s.flip;
+                        }
                     }
                 }
             }
+            if (cur.empty()) continue;  // the segment ends in CNOTs
             for (int b = kt - 1; b >= 0 && __builtin_popcount(rmask) < G::a; --b) rmask |= 1u << b;
             TPhase ph{};
             ph.op_begin = (uint16_t)(B.ops.size() - sg.op_begin);
             ph.nops = (uint16_t)cur.size();
             std::vector<int> rpos(32, -1);
+            std::vector<int> reg;  // register j's tile bit: fewest steps first (Regs)
             for (int b = 0, j = 0; b < kt; ++b)
                 if ((rmask >> b) & 1) {
-                    rpos[b] = j;
+                    reg.push_back(b);
                     ph.rb[j++] = (uint8_t)b;
                 }
+            auto uses = [&](int b) {
+                int c = 0;
+                for (uint32_t j : cur) c += (int)((targets(step(j)) >> sg.lbits[b]) & 1);
+                return c;
+            };
+            std::stable_sort(reg.begin(), reg.end(), [&](int x, int y) { return uses(x) < uses(y); });
+            for (int j = 0; j < G::a; ++j) {
+                rpos[reg[j]] = j;
+                ph.rt[j] = (uint8_t)reg[j];
+                ph.rcol[j] = (uint16_t)tswz<R>(place[reg[j]]);
+            }
+            for (int b = 0, j = 0; b < kt; ++b)
+                if (!((rmask >> b) & 1)) ph.tcol[j++] = (uint16_t)tswz<R>(place[b]);
             B.phases.push_back(ph);
             for (uint32_t j : cur) {
                 const Step &s = step(j);
@@ -328,6 +358,7 @@ template <typename R, bool REV> void plan_dir(Builder &B, Plan &P, uint32_t n, i
                 B.ops.push_back(o);
             }
         }
+        for (int b = 0; b < 12; ++b) sg.fcol[b] = (uint16_t)tswz<R>(place[b]);
         sg.nph = (uint32_t)B.phases.size() - sg.ph_begin;
         sg.nops = (uint32_t)B.ops.size() - sg.op_begin;
         sg.ncoef = D.ncoef - sg.coef_begin;

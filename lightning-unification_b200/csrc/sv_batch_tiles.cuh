@@ -9,7 +9,7 @@
 // (circuits x tiles) independent pieces of work and nothing waits on another CTA.  One wide
 // circuit spreads over the whole GPU this way: a training step over 192 circuits of 10-18 qubits,
 // complex128, went from 121.5 ms (one CTA per circuit: the widest circuits' chains of tiles ran alone
-// at the end) to 7.4 ms, and the 1024-circuit step of 16 qubits, complex64, from 70.2 to 28.5 ms (fewer
+// at the end) to 7.4 ms, and the 1024-circuit step of 16 qubits, complex64, from 70.2 to 23.9 ms (fewer
 // barriers and shared-memory passes between steps, three 256-thread CTAs an SM instead of one of 512).
 // Circuits narrower than a tile are one tile of their own size in CTAs of fewer threads,
 // launched beside the wide ones.
@@ -71,15 +71,25 @@ struct alignas(16) TOp {
     uint8_t p0, p1, p2, pad;
     uint32_t dsign;        // T_DIAG with a gradient: generator entry of index i in bits 2i (1: +1, 2: -1)
 };
+// CNOT and SWAP steps move no data.  A segment keeps a GF(2)-linear map from the tile position of an
+// amplitude to the place where it lies in shared memory; a CNOT between phases replaces the column of
+// its control bit by (control column XOR target column), and the tile's store reads through the last
+// map.  A phase loads and stores its amplitudes through its map: places, not positions, so no thread
+// touches another's amplitudes and no extra barrier is needed.
 struct TPhase {
     uint16_t op_begin, nops;
-    uint8_t rb[4];  // register bits (tile positions, ascending)
+    uint8_t rb[4];     // register bits (tile positions, ascending)
+    uint8_t rt[4];     // tile position of register bit j
+    uint16_t tcol[8];  // place of each thread index bit (swizzled)
+    uint16_t rcol[4];  // place of each register bit (swizzled)
+    uint32_t pad;
 };
 struct alignas(16) TSeg {
     uint32_t ph_begin, nph, op_begin, nops;
     uint32_t coef_begin, ncoef, ngrad;
     uint8_t lbits[16];
     uint8_t gbits[32];
+    uint16_t fcol[12];  // places of the tile bits when the tile is stored (swizzled)
     uint8_t ng, kt, pad[2];
 };
 struct alignas(16) Job {
@@ -146,75 +156,176 @@ template <typename R> __device__ __forceinline__ C<R> flip_sign(C<R> v, uint32_t
     }
 }
 
+// Two FP32 values in one 64-bit register (the paired FP32 instructions' operand).  As float2 the halves
+// are separate registers to the compiler, which then moved the whole state on every step (335 moves a
+// step); a 64-bit value keeps its pair from step to step.
+using pair2 = unsigned long long;
+__device__ __forceinline__ pair2 pk(float x, float y) {
+    pair2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpk(pair2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ pair2 mul2(pair2 a, pair2 b) {
+    pair2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair2 fma2(pair2 a, pair2 b, pair2 c) {
+    pair2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// A thread's amplitudes.  complex64 keeps real and imaginary parts apart and packs the two
+// amplitudes that differ in register bit 0, so that the paired FP32 instructions work on two
+// amplitude pairs at once without swapping or broadcasting any amplitude part; steps on register
+// bit 0 itself use scalar FMAs (the planner gives that bit to the wire with the fewest steps).  Per
+// differentiated 2x2 step on 16 + 16 amplitudes: 128 paired FMAs for both states and 60 for the four
+// sums, against 128 + 64 register swaps and 112 scalar operations with (re, im) pairs; with CNOTs in the
+// address map the 1024-circuit step went from 28.5 to 23.9 ms.
+template <typename R, int A> struct Regs {
+    C<R> v[A];
+    __device__ __forceinline__ C<R> get(int g) const { return v[g]; }
+    __device__ __forceinline__ void set(int g, C<R> x) { v[g] = x; }
+};
+template <int A> struct Regs<float, A> {
+    pair2 re[A / 2], im[A / 2];
+    __device__ __forceinline__ float2 get(int g) const {
+        const float2 r = unpk(re[g >> 1]), i = unpk(im[g >> 1]);
+        return (g & 1) ? make_float2(r.y, i.y) : make_float2(r.x, i.x);
+    }
+    __device__ __forceinline__ void set(int g, float2 x) {
+        const float2 r = unpk(re[g >> 1]), i = unpk(im[g >> 1]);
+        re[g >> 1] = (g & 1) ? pk(r.x, x.x) : pk(x.x, r.y);
+        im[g >> 1] = (g & 1) ? pk(i.x, x.y) : pk(x.y, i.y);
+    }
+};
+
+// ys = M (x, y) on every pair of the register bit; four roundings a component
 template <typename R, int A, int BIT, bool CTL>
-__device__ __forceinline__ void t_dense(C<R> (&v)[A], uint32_t creg, const C<R> (&m)[4]) {
+__device__ __forceinline__ void t_dense(Regs<R, A> &v, uint32_t creg, const C<R> (&m)[4]) {
     constexpr int B = 1 << BIT;
+    if constexpr (sizeof(R) == 4 && BIT > 0 && !CTL) {
+        pair2 mr[4], mi[4], mn[4];
 #pragma unroll
-    for (int g = 0; g < A; ++g) {
-        if (g & B) continue;
-        if (CTL && ((uint32_t)g & creg) != creg) continue;
-        const C<R> x = v[g], y = v[g | B];
-        v[g] = mac2<R>(m[0], x, m[1], y);
-        v[g | B] = mac2<R>(m[2], x, m[3], y);
+        for (int i = 0; i < 4; ++i) {
+            mr[i] = pk(m[i].x, m[i].x);
+            mi[i] = pk(m[i].y, m[i].y);
+            mn[i] = pk(-m[i].y, -m[i].y);
+        }
+#pragma unroll
+        for (int h = 0; h < A / 2; ++h) {
+            if (h & (B >> 1)) continue;
+            const int k = h | (B >> 1);
+            const pair2 xr = v.re[h], xi = v.im[h], yr = v.re[k], yi = v.im[k];
+            v.re[h] = fma2(mn[1], yi, fma2(mr[1], yr, fma2(mn[0], xi, mul2(mr[0], xr))));
+            v.im[h] = fma2(mi[1], yr, fma2(mr[1], yi, fma2(mi[0], xr, mul2(mr[0], xi))));
+            v.re[k] = fma2(mn[3], yi, fma2(mr[3], yr, fma2(mn[2], xi, mul2(mr[2], xr))));
+            v.im[k] = fma2(mi[3], yr, fma2(mr[3], yi, fma2(mi[2], xr, mul2(mr[2], xi))));
+        }
+    } else {
+#pragma unroll
+        for (int g = 0; g < A; ++g) {
+            if (g & B) continue;
+            if (CTL && ((uint32_t)g & creg) != creg) continue;
+            const C<R> x = v.get(g), y = v.get(g | B);
+            C<R> p, q;
+            p.x = fma(-m[1].y, y.y, fma(m[1].x, y.x, fma(-m[0].y, x.y, m[0].x * x.x)));
+            p.y = fma(m[1].y, y.x, fma(m[1].x, y.y, fma(m[0].y, x.x, m[0].x * x.y)));
+            q.x = fma(-m[3].y, y.y, fma(m[3].x, y.x, fma(-m[2].y, x.y, m[2].x * x.x)));
+            q.y = fma(m[3].y, y.x, fma(m[3].x, y.y, fma(m[2].y, x.x, m[2].x * x.y)));
+            v.set(g, p);
+            v.set(g | B, q);
+        }
     }
 }
-// the four sums of a differentiated step on register bit BIT
+// the four sums of a differentiated step on register bit BIT: each pair's values in the state's
+// precision, the sums in FP64
 template <typename R, int A, int BIT, bool CTL>
-__device__ __forceinline__ void t_cross(const C<R> (&v)[A], const C<R> (&w)[A], uint32_t creg, double (&s)[4]) {
+__device__ __forceinline__ void t_cross(const Regs<R, A> &v, const Regs<R, A> &w, uint32_t creg, double (&s)[4]) {
     constexpr int B = 1 << BIT;
+    if constexpr (sizeof(R) == 4 && BIT > 0 && !CTL) {
+        const pair2 minus = pk(-1.0f, -1.0f);
 #pragma unroll
-    for (int g = 0; g < A; ++g) {
-        if (g & B) continue;
-        if (CTL && ((uint32_t)g & creg) != creg) continue;
-        const C<R> a0 = v[g], a1 = v[g | B], b0 = w[g], b1 = w[g | B];
-        s[0] += (double)fma(b0.x, a0.y, -(b0.y * a0.x));
-        s[1] += (double)fma(b1.x, a1.y, -(b1.y * a1.x));
-        s[2] += (double)(fma(b0.x, a1.y, -(b0.y * a1.x)) + fma(b1.x, a0.y, -(b1.y * a0.x)));
-        s[3] += (double)(fma(b0.x, a1.x, b0.y * a1.y) - fma(b1.x, a0.x, b1.y * a0.y));
+        for (int h = 0; h < A / 2; ++h) {
+            if (h & (B >> 1)) continue;
+            const int k = h | (B >> 1);
+            const pair2 a0r = v.re[h], a0i = v.im[h], a1r = v.re[k], a1i = v.im[k];
+            const pair2 b0r = w.re[h], b0i = w.im[h], b1r = w.re[k], b1i = w.im[k];
+            const pair2 n0i = mul2(b0i, minus), n1i = mul2(b1i, minus), n1r = mul2(b1r, minus);
+            const float2 x1 = unpk(fma2(b0r, a0i, mul2(n0i, a0r)));
+            const float2 x2 = unpk(fma2(b1r, a1i, mul2(n1i, a1r)));
+            const float2 s1 = unpk(fma2(n1i, a0r, fma2(b1r, a0i, fma2(n0i, a1r, mul2(b0r, a1i)))));
+            const float2 s2 = unpk(fma2(n1i, a0i, fma2(n1r, a0r, fma2(b0i, a1i, mul2(b0r, a1r)))));
+            s[0] += (double)x1.x;
+            s[1] += (double)x2.x;
+            s[2] += (double)s1.x;
+            s[3] += (double)s2.x;
+            s[0] += (double)x1.y;
+            s[1] += (double)x2.y;
+            s[2] += (double)s1.y;
+            s[3] += (double)s2.y;
+        }
+    } else {
+#pragma unroll
+        for (int g = 0; g < A; ++g) {
+            if (g & B) continue;
+            if (CTL && ((uint32_t)g & creg) != creg) continue;
+            const C<R> a0 = v.get(g), a1 = v.get(g | B), b0 = w.get(g), b1 = w.get(g | B);
+            s[0] += (double)fma(b0.x, a0.y, -(b0.y * a0.x));
+            s[1] += (double)fma(b1.x, a1.y, -(b1.y * a1.x));
+            s[2] += (double)fma(-b1.y, a0.x, fma(b1.x, a0.y, fma(-b0.y, a1.x, b0.x * a1.y)));
+            s[3] += (double)fma(-b1.y, a0.y, fma(-b1.x, a0.x, fma(b0.y, a1.y, b0.x * a1.x)));
+        }
     }
 }
 template <typename R, int A, int BIT>
-__device__ __forceinline__ void t_diag1(C<R> (&v)[A], C<R> f0, C<R> f1) {
+__device__ __forceinline__ void t_diag1(Regs<R, A> &v, C<R> f0, C<R> f1) {
 #pragma unroll
-    for (int g = 0; g < A; ++g) v[g] = tprod<R>((g >> BIT) & 1 ? f1 : f0, v[g]);
+    for (int g = 0; g < A; ++g) v.set(g, tprod<R>((g >> BIT) & 1 ? f1 : f0, v.get(g)));
 }
-template <typename R, int A, int MASK> __device__ __forceinline__ void t_sign(C<R> (&v)[A], uint32_t neg) {
+template <typename R, int A, int MASK> __device__ __forceinline__ void t_sign(Regs<R, A> &v, uint32_t neg) {
 #pragma unroll
     for (int g = 0; g < A; ++g)
-        if ((g & MASK) == MASK) v[g] = flip_sign<R>(v[g], neg);
+        if ((g & MASK) == MASK) v.set(g, flip_sign<R>(v.get(g), neg));
 }
-template <typename R, int A, int BIT, int CMASK> __device__ __forceinline__ void t_cx(C<R> (&v)[A], bool on) {
+template <typename R, int A, int BIT, int CMASK> __device__ __forceinline__ void t_cx(Regs<R, A> &v, bool on) {
     constexpr int B = 1 << BIT;
 #pragma unroll
     for (int g = 0; g < A; ++g) {
         if ((g & B) || (g & CMASK) != CMASK) continue;
-        const C<R> x = v[g], y = v[g | B];
-        v[g] = on ? y : x;
-        v[g | B] = on ? x : y;
+        const C<R> x = v.get(g), y = v.get(g | B);
+        v.set(g, on ? y : x);
+        v.set(g | B, on ? x : y);
     }
 }
 template <typename R, int A, int BIT>
-__device__ __forceinline__ void t_cxg(C<R> (&v)[A], uint32_t creg, bool on) {
+__device__ __forceinline__ void t_cxg(Regs<R, A> &v, uint32_t creg, bool on) {
     constexpr int B = 1 << BIT;
 #pragma unroll
     for (int g = 0; g < A; ++g) {
         if (g & B) continue;
         const bool d = on && ((uint32_t)g & creg) == creg;
-        const C<R> x = v[g], y = v[g | B];
-        v[g] = d ? y : x;
-        v[g | B] = d ? x : y;
+        const C<R> x = v.get(g), y = v.get(g | B);
+        v.set(g, d ? y : x);
+        v.set(g | B, d ? x : y);
     }
 }
 template <typename R, int A, int MASK>
-__device__ __forceinline__ void t_swap(C<R> (&v)[A], uint32_t creg, bool on) {
+__device__ __forceinline__ void t_swap(Regs<R, A> &v, uint32_t creg, bool on) {
     constexpr int LO = low_of(MASK), HI = MASK ^ LO;
 #pragma unroll
     for (int g = 0; g < A; ++g) {
         if (g & MASK) continue;
         const bool d = on && ((uint32_t)g & creg) == creg;
-        const C<R> x = v[g | LO], y = v[g | HI];
-        v[g | LO] = d ? y : x;
-        v[g | HI] = d ? x : y;
+        const C<R> x = v.get(g | LO), y = v.get(g | HI);
+        v.set(g | LO, d ? y : x);
+        v.set(g | HI, d ? x : y);
     }
 }
 
@@ -244,7 +355,7 @@ __device__ __forceinline__ void add_sums(double *sacc, uint32_t row, const doubl
 
 // One step on the thread's amplitudes of NS states (w is v where there is one state).
 template <typename R, int A, int NS>
-__device__ __forceinline__ void t_step(C<R> (&v)[A], C<R> (&w)[A], const TOp &op, const C<R> *__restrict__ scf,
+__device__ __forceinline__ void t_step(Regs<R, A> &v, Regs<R, A> &w, const TOp &op, const C<R> *__restrict__ scf,
                                        double *sacc, uint32_t base, uint64_t tbase, const uint32_t (&rbit)[4], C<R> &tf,
                                        bool &has_tf, uint32_t &neg) {
     const C<R> *cf = scf + op.coef;
@@ -256,6 +367,27 @@ __device__ __forceinline__ void t_step(C<R> (&v)[A], C<R> (&w)[A], const TOp &op
             if ((g >> j) & 1) l |= rbit[j];
         return l;
     };
+    // the codes nearly every step has, ahead of the others: a two-level branch instead of a search
+    // through the whole table
+    if ((op.code & ~3) == T_DENSE) {
+        const C<R> m[4] = {cf[0], cf[1], cf[2], cf[3]};
+        const bool grad = NS == 2 && op.grad;
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+#define TILE_DENSE(b)                                                                                          \
+    if constexpr ((1 << b) < A) {                                                                              \
+        if (grad) t_cross<R, A, b, false>(v, w, 0, s);                                                         \
+        t_dense<R, A, b, false>(v, 0, m);                                                                      \
+        if (NS == 2) t_dense<R, A, b, false>(w, 0, m);                                                         \
+    }
+        if (op.code & 2) {
+            if (op.code & 1) { TILE_DENSE(3) } else { TILE_DENSE(2) }
+        } else {
+            if (op.code & 1) { TILE_DENSE(1) } else { TILE_DENSE(0) }
+        }
+#undef TILE_DENSE
+        if (grad) add_sums(sacc, op.grad - 1u, s);
+        return;
+    }
     switch (op.code) {
     case T_DIAG_T: {
         const uint32_t idx = (((base >> op.p0) & 1u) << 2) | (((base >> op.p1) & 1u) << 1) | ((base >> op.p2) & 1u);
@@ -279,12 +411,13 @@ __device__ __forceinline__ void t_step(C<R> (&v)[A], C<R> (&w)[A], const TOp &op
             const uint32_t idx = (((x >> op.p0) & 1u) << 2) | (((x >> op.p1) & 1u) << 1) | ((x >> op.p2) & 1u);
             if (grad) {
                 const uint32_t d = (op.dsign >> (2 * idx)) & 3u;
-                const double im = (double)fma(w[g].x, v[g].y, -(w[g].y * v[g].x));
+                const C<R> a = v.get(g), b = w.get(g);
+                const double im = (double)fma(b.x, a.y, -(b.y * a.x));
                 s[0] += d == 1u ? im : d == 2u ? -im : 0.0;
             }
             const C<R> f = cf[idx];
-            v[g] = tprod<R>(f, v[g]);
-            if (NS == 2) w[g] = tprod<R>(f, w[g]);
+            v.set(g, tprod<R>(f, v.get(g)));
+            if (NS == 2) w.set(g, tprod<R>(f, w.get(g)));
         }
         if (grad) add_sums(sacc, op.grad - 1u, s);
         break;
@@ -298,12 +431,13 @@ __device__ __forceinline__ void t_step(C<R> (&v)[A], C<R> (&w)[A], const TOp &op
         for (int g = 0; g < A; ++g) {
             const bool odd = ((__popc(position(g) & op.pm) + tp) & 1) != 0;
             if (grad) {
-                const double im = (double)fma(w[g].x, v[g].y, -(w[g].y * v[g].x));
+                const C<R> a = v.get(g), b = w.get(g);
+                const double im = (double)fma(b.x, a.y, -(b.y * a.x));
                 s[0] += odd ? -im : im;
             }
             const C<R> f = odd ? f1 : f0;
-            v[g] = tprod<R>(f, v[g]);
-            if (NS == 2) w[g] = tprod<R>(f, w[g]);
+            v.set(g, tprod<R>(f, v.get(g)));
+            if (NS == 2) w.set(g, tprod<R>(f, w.get(g)));
         }
         if (grad) add_sums(sacc, op.grad - 1u, s);
         break;
@@ -322,18 +456,6 @@ __device__ __forceinline__ void t_step(C<R> (&v)[A], C<R> (&w)[A], const TOp &op
             const uint32_t sg = on ? 0x80000000u : 0u;                                                         \
             t_sign<R, A, 1 << b>(v, sg);                                                                       \
             if (NS == 2) t_sign<R, A, 1 << b>(w, sg);                                                          \
-        }                                                                                                      \
-        break;                                                                                                 \
-    case T_DENSE + b:                                                                                          \
-        if constexpr ((1 << b) < A) {                                                                          \
-            const C<R> m[4] = {cf[0], cf[1], cf[2], cf[3]};                                                    \
-            if (NS == 2 && op.grad) {                                                                          \
-                double s[4] = {0.0, 0.0, 0.0, 0.0};                                                            \
-                t_cross<R, A, b, false>(v, w, 0, s);                                                           \
-                add_sums(sacc, op.grad - 1u, s);                                                               \
-            }                                                                                                  \
-            t_dense<R, A, b, false>(v, 0, m);                                                                  \
-            if (NS == 2) t_dense<R, A, b, false>(w, 0, m);                                                     \
         }                                                                                                      \
         break;                                                                                                 \
     case T_DENSEC + b:                                                                                         \
@@ -473,27 +595,41 @@ __global__ void __launch_bounds__(kTThreads, TGeo<R, REV>::minb) k_tiles(TArgs a
         __syncthreads();
         for (uint32_t p = 0; p < sg.nph; ++p) {
             const TPhase ph = sph[p];
-            uint32_t base = threadIdx.x, rbit[4] = {0, 0, 0, 0}, rs[4];
+            uint32_t base = threadIdx.x, sbase = 0, rbit[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int j = 0; j < G::a; ++j) {
-                rbit[j] = 1u << ph.rb[j];
-                const uint32_t low = base & (rbit[j] - 1u);
+                rbit[j] = 1u << ph.rt[j];
+                const uint32_t low = base & ((1u << ph.rb[j]) - 1u);
                 base = ((base ^ low) << 1) | low;
-                rs[j] = tswz<R>(rbit[j]);
             }
-            const uint32_t sbase = tswz<R>(base);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sbase ^= (threadIdx.x >> j) & 1u ? ph.tcol[j] : 0u;
             auto at = [&](int g) {
                 uint32_t x = sbase;
 #pragma unroll
                 for (int j = 0; j < G::a; ++j)
-                    if ((g >> j) & 1) x ^= rs[j];
+                    if ((g >> j) & 1) x ^= ph.rcol[j];
                 return x;
             };
-            C<R> v[A], w[A];
+            Regs<R, A> v, w;
+            if constexpr (sizeof(R) == 4) {
 #pragma unroll
-            for (int g = 0; g < A; ++g) {
-                v[g] = sl[at(g)];
-                if (REV) w[g] = sb[at(g)];
+                for (int g = 0; g < A; g += 2) {
+                    const C<R> x = sl[at(g)], y = sl[at(g + 1)];
+                    v.re[g / 2] = pk(x.x, y.x);
+                    v.im[g / 2] = pk(x.y, y.y);
+                    if (REV) {
+                        const C<R> p = sb[at(g)], q = sb[at(g + 1)];
+                        w.re[g / 2] = pk(p.x, q.x);
+                        w.im[g / 2] = pk(p.y, q.y);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int g = 0; g < A; ++g) {
+                    v.set(g, sl[at(g)]);
+                    if (REV) w.set(g, sb[at(g)]);
+                }
             }
             C<R> tf = mk<R>(1, 0);
             bool has_tf = false;
@@ -503,24 +639,40 @@ __global__ void __launch_bounds__(kTThreads, TGeo<R, REV>::minb) k_tiles(TArgs a
             if (has_tf) {
 #pragma unroll
                 for (int g = 0; g < A; ++g) {
-                    v[g] = tprod<R>(tf, v[g]);
-                    if (REV) w[g] = tprod<R>(tf, w[g]);
+                    v.set(g, tprod<R>(tf, v.get(g)));
+                    if (REV) w.set(g, tprod<R>(tf, w.get(g)));
                 }
             }
 #pragma unroll
             for (int g = 0; g < A; ++g) {
-                sl[at(g)] = flip_sign<R>(v[g], neg);
-                if (REV) sb[at(g)] = flip_sign<R>(w[g], neg);
+                sl[at(g)] = flip_sign<R>(v.get(g), neg);
+                if (REV) sb[at(g)] = flip_sign<R>(w.get(g), neg);
             }
             __syncthreads();
         }
         if (!(jb.flags & 2u)) {
+            constexpr int LV = V == 2 ? 1 : 0;
+            const int lt = 31 - __clz((int)NT);
+            uint32_t f0 = 0;
+            for (int i = 0; i < lt; ++i) f0 ^= (threadIdx.x >> i) & 1u ? sg.fcol[LV + i] : 0u;
+            auto chunk = [&](const C<R> *t, uint32_t f) {
+                if constexpr (V == 2) {
+                    const C<R> x = t[f], y = t[f ^ sg.fcol[0]];
+                    return make_float4(x.x, x.y, y.x, y.y);
+                } else {
+                    return *reinterpret_cast<const float4 *>(t + f);
+                }
+            };
 #pragma unroll
             for (int j = 0; j < PER; ++j) {
                 const uint64_t x = tbase | lo | s_hi[j];
+                uint32_t f = f0;
+#pragma unroll
+                for (int i = 0; (1 << i) < PER; ++i)
+                    if ((j >> i) & 1) f ^= sg.fcol[LV + lt + i];
                 if (x < namp) {
-                    *reinterpret_cast<float4 *>(ga + x) = *reinterpret_cast<const float4 *>(sl + sw(j));
-                    if (REV) *reinterpret_cast<float4 *>(gb + x) = *reinterpret_cast<const float4 *>(sb + sw(j));
+                    *reinterpret_cast<float4 *>(ga + x) = chunk(sl, f);
+                    if (REV) *reinterpret_cast<float4 *>(gb + x) = chunk(sb, f);
                 }
             }
         }
