@@ -26,10 +26,14 @@
 
 #include "../../include/b200sv.h"
 #include "sv_device.cuh"
+#include "sv_plan.hpp"
+#include "sv_steps.cuh"
 #include "sv_internal.hpp"
 
 namespace b200sv {
 namespace batch {
+
+using steps::cmul1;
 
 // F_PAIR4: the double-excitation family, a 2x2 block on rows 0011 / 1100 of each 16-row group of
 // four target bits, the other rows scaled by gamma.  F_MATK: a constant dense matrix on 3 or 4
@@ -97,10 +101,6 @@ constexpr int kMaxSegOpsStaged = 160;  // ops of a segment staged in shared memo
 // structure of a single-wire matrix, used to spend fewer instructions per amplitude pair
 enum MKind : uint8_t { MK_GENERAL = 0, MK_DIAG = 1, MK_PHASE1 = 2, MK_REAL = 3, MK_SWAP = 4, MK_RX = 5 };
 
-// single complex product m * v (FMA-formed components)
-template <typename R> __device__ __forceinline__ C<R> cmul1(C<R> m, C<R> v) {
-    return mk<R>(fma(m.x, v.x, -(m.y * v.y)), fma(m.x, v.y, m.y * v.x));
-}
 // a*x + b*y for real coefficients, accurate to about one rounding: the product b*y is
 // split exactly with an FMA (TwoProduct) and its error added back after the second FMA.
 template <typename R> __device__ __forceinline__ R dot2r(R a, R x, R b, R y) {

@@ -13,19 +13,6 @@ bool serves(const HostOp &h) {
     }
 }
 
-// A step of a circuit: a run of single-wire gates on one bit, or one gate.
-struct Step {
-    SKind kind = S_NONE;
-    bool swap = false, sign = false, grad = false, wide = false;
-    std::vector<uint32_t> mems;     // op indices, in order
-    std::vector<uint32_t> ctl, tgt; // state bits
-    uint64_t mask = 0, targets = 0; // bits touched; bits that must be register bits
-    uint64_t flip = 0;              // bits on which the step is not diagonal: steps commute when every
-                                    // bit they share is diagonal in both
-    bool linear = false;            // CNOT, SWAP: between phases, in the tile's address map
-    uint32_t dsign = 0;
-};
-
 std::vector<Step> make_steps(const std::vector<HostOp> &ops, uint32_t n) {
     std::vector<Step> out;
     std::vector<int> last(n, -1);  // latest step on each bit
@@ -60,7 +47,6 @@ std::vector<Step> make_steps(const std::vector<HostOp> &ops, uint32_t n) {
         for (auto b : h.bits) s.mask |= uint64_t(1) << b;
         if (h.form == F_PARITY) {
             s.kind = S_PARITY;
-            s.wide = true;
         } else if (h.form == F_SWAP) {
             s.swap = true;
             for (auto b : s.tgt) s.flip |= uint64_t(1) << b;
@@ -105,268 +91,40 @@ struct Plan {
 };
 
 struct Builder {
-    std::vector<TSeg> segs;
-    std::vector<TPhase> phases;
-    std::vector<TOp> ops;
+    Records rec;
     std::vector<CoefStep> steps;
     std::vector<uint32_t> mem_list;
 };
 
-int coef_slots(const Step &s, bool rev) {
-    switch (s.kind) {
-    case S_RUN: case S_DENSE: return 4;
-    case S_DIAGRUN: return rev && s.grad ? 4 : 8;
-    case S_DIAG: return 8;
-    case S_PARITY: return 2;
-    default: return 0;
-    }
-}
-
-// Segments and phases of one direction.  A diagonal run with a gradient is a 2x2 step of the reverse
-// sweep (its sums go over register pairs).
+// Segments and phases of one direction.
 template <typename R, bool REV> void plan_dir(Builder &B, Plan &P, uint32_t n, int kt_cap) {
-    using G = TGeo<R, REV>;
     PlanDir &D = P.dir[REV ? 1 : 0];
-    const int kt = std::max(std::min({(int)n, (int)G::kt, kt_cap}), G::a + 5);
-    const bool tiled = (int)n > kt;
-    const uint64_t low = tiled ? (uint64_t(1) << G::reserve) - 1 : 0;
     std::vector<uint32_t> order(P.steps.size());
     std::iota(order.begin(), order.end(), 0u);
-    if (REV) std::reverse(order.begin(), order.end());
-    const size_t ns = order.size();
-    auto step = [&](size_t i) -> const Step & { return P.steps[order[i]]; };
-    auto targets = [&](const Step &s) { return REV && s.kind == S_DIAGRUN && s.grad ? s.mask : s.targets; };
-    std::vector<char> done(ns, 0);
-    size_t left = ns, first = 0;
     if (REV) {  // steps past the last differentiated one are not needed
-        size_t lastg = 0;
-        for (size_t i = 0; i < ns; ++i)
-            if (step(i).grad) lastg = i + 1;
-        for (size_t i = lastg; i < ns; ++i) done[i] = 1;
-        left = lastg;
+        std::reverse(order.begin(), order.end());
+        while (!order.empty() && !P.steps[order.back()].grad) order.pop_back();
     }
     D.step_begin = (uint32_t)B.steps.size();
-    while (left > 0 || (!REV && D.segs.empty())) {
-        while (first < ns && done[first]) ++first;
-        // the segment: every later step that fits the tile and commutes with the steps left out
-        uint64_t used = 0, any = 0, flipped = 0;  // of the steps left out
-        int nops = 0, ncf = 0, ngr = 0;
-        std::vector<uint32_t> take;
-        for (size_t j = first; j < ns; ++j) {
-            if (done[j]) continue;
-            const Step &s = step(j);
-            const uint64_t need = s.wide ? 0 : s.mask;
-            const bool fits = !(s.flip & any) && !(s.mask & flipped) && __builtin_popcountll(used | need | low) <= kt &&
-                              nops < kMaxTOps && ncf + coef_slots(s, REV) <= kMaxTCoefs &&
-                              ngr + (REV && s.grad ? 1 : 0) <= kMaxTGrads;
-            if (fits) {
-                used |= need;
-                ++nops;
-                ncf += coef_slots(s, REV);
-                ngr += REV && s.grad ? 1 : 0;
-                take.push_back((uint32_t)j);
-                done[j] = 1;
-                --left;
-            } else {
-                any |= s.mask;
-                flipped |= s.flip;
-                if (flipped == (uint64_t(1) << n) - 1) break;  // everything later is blocked
-            }
-        }
-        if (take.empty() && left > 0) throw Unsupported("batch: gate wider than the tile");
-        TSeg sg{};
-        std::vector<int> loc(n, -1);
-        uint64_t inl = used | low;
-        for (uint32_t x = 0; x < n && __builtin_popcountll(inl) < kt; ++x) inl |= uint64_t(1) << x;
-        int nl = 0;
-        for (uint32_t x = 0; x < n; ++x) {
-            if ((inl >> x) & 1) {
-                loc[x] = nl;
-                sg.lbits[nl++] = (uint8_t)x;
-            } else {
-                sg.gbits[sg.ng++] = (uint8_t)x;
-            }
-        }
-        for (uint32_t x = n; nl < kt; ++x) sg.lbits[nl++] = (uint8_t)x;  // padding above the state
-        sg.kt = (uint8_t)kt;
-        sg.ph_begin = (uint32_t)B.phases.size();
-        sg.op_begin = (uint32_t)B.ops.size();
-        sg.coef_begin = D.ncoef;
-        std::vector<uint32_t> grads;
-        // phases: the ready CNOTs and SWAPs go into the address map, then every ready step whose
-        // targets fit the register bits, until nothing moves
-        std::vector<char> out(take.size(), 0);
-        size_t rest = take.size();
-        uint16_t place[12];  // of each tile bit, before the swizzle
-        for (int b = 0; b < 12; ++b) place[b] = (uint16_t)(1u << b);
-        while (rest > 0) {
-            uint32_t rmask = 0;
-            std::vector<uint32_t> cur;
-            for (bool linear : {true, false}) {
-                for (bool progress = true; progress;) {
-                    progress = false;
-                    uint64_t la = 0, lf = 0;
-                    for (size_t i = 0; i < take.size(); ++i) {
-                        if (out[i]) continue;
-                        const Step &s = step(take[i]);
-                        uint32_t need = 0;
-                        for (uint32_t x = 0; x < n; ++x)
-                            if ((targets(s) >> x) & 1) need |= 1u << loc[x];
-                        if (s.linear == linear && !(s.flip & la) && !(s.mask & lf) &&
-                            __builtin_popcount(rmask | need) <= G::a) {
-                            out[i] = 1;
-                            --rest;
-                            progress = true;
-                            if (!linear) {
-                                rmask |= need;
-                                cur.push_back(take[i]);
-                            } else if (s.ctl.size() == 1) {
-                                place[loc[s.ctl[0]]] ^= place[loc[s.tgt[0]]];
-                            } else {
-                                std::swap(place[loc[s.tgt[0]]], place[loc[s.tgt[1]]]);
-                            }
-                        } else {
-                            la |= s.mask;
-                            lf |= s.flip;
-                        }
-                    }
-                }
-            }
-            if (cur.empty()) continue;  // the segment ends in CNOTs
-            for (int b = kt - 1; b >= 0 && __builtin_popcount(rmask) < G::a; --b) rmask |= 1u << b;
-            TPhase ph{};
-            ph.op_begin = (uint16_t)(B.ops.size() - sg.op_begin);
-            ph.nops = (uint16_t)cur.size();
-            std::vector<int> rpos(32, -1);
-            std::vector<int> reg;  // register j's tile bit: fewest steps first (Regs)
-            for (int b = 0, j = 0; b < kt; ++b)
-                if ((rmask >> b) & 1) {
-                    reg.push_back(b);
-                    ph.rb[j++] = (uint8_t)b;
-                }
-            auto uses = [&](int b) {
-                int c = 0;
-                for (uint32_t j : cur) c += (int)((targets(step(j)) >> sg.lbits[b]) & 1);
-                return c;
-            };
-            std::stable_sort(reg.begin(), reg.end(), [&](int x, int y) { return uses(x) < uses(y); });
-            for (int j = 0; j < G::a; ++j) {
-                rpos[reg[j]] = j;
-                ph.rt[j] = (uint8_t)reg[j];
-                ph.rcol[j] = (uint16_t)tswz<R>(place[reg[j]]);
-            }
-            for (int b = 0, j = 0; b < kt; ++b)
-                if (!((rmask >> b) & 1)) ph.tcol[j++] = (uint16_t)tswz<R>(place[b]);
-            B.phases.push_back(ph);
-            for (uint32_t j : cur) {
-                const Step &s = step(j);
-                TOp o{};
-                CoefStep c{};
-                c.kind = s.kind;
-                if (REV && s.kind == S_DIAGRUN && s.grad) c.kind = S_RUN;
-                c.mem_begin = (uint32_t)B.mem_list.size();
-                c.nmem = (uint16_t)s.mems.size();
-                c.coef = D.ncoef;
-                o.coef = (uint16_t)(D.ncoef - sg.coef_begin);
-                o.p0 = o.p1 = o.p2 = 31;
-                if (REV && s.grad) {
-                    grads.push_back(order[j]);
-                    o.grad = (uint16_t)grads.size();
-                }
-                auto control = [&](const std::vector<uint32_t> &bits) {
-                    for (auto x : bits) {
-                        if (rpos[loc[x]] >= 0) o.creg |= (uint16_t)(1 << rpos[loc[x]]);
-                        else o.cthr |= 1u << loc[x];
-                    }
-                };
-                auto pair_index = [](int m) {
-                    for (int i = 0; i < 6; ++i)
-                        if (pair_mask(i) == m) return i;
-                    return 0;
-                };
-                if (s.sign) {
-                    control(s.ctl);
-                    control(s.tgt);
-                    const int nr = __builtin_popcount(o.creg);
-                    o.code = nr == 0 ? T_SIGN_T : nr == 1 ? T_SIGN1 + __builtin_ctz(o.creg) : T_SIGN2 + pair_index(o.creg);
-                } else if (s.swap) {
-                    control(s.ctl);
-                    if (s.tgt.size() == 1) {
-                        const int t = rpos[loc[s.tgt[0]]], nr = __builtin_popcount(o.creg);
-                        o.code = nr == 0   ? T_CX_T + t
-                                 : nr == 1 ? T_CX_R + 4 * t + __builtin_ctz(o.creg)
-                                           : T_CX_G + t;
-                    } else {
-                        o.code = T_SWAP + pair_index((1 << rpos[loc[s.tgt[0]]]) | (1 << rpos[loc[s.tgt[1]]]));
-                    }
-                } else if (c.kind == S_RUN) {
-                    o.code = T_DENSE + rpos[loc[s.tgt[0]]];
-                } else if (s.kind == S_DENSE) {
-                    control(s.ctl);
-                    o.code = T_DENSEC + rpos[loc[s.tgt[0]]];
-                } else if (s.kind == S_DIAGRUN) {
-                    const int b = loc[s.tgt[0]];
-                    if (rpos[b] >= 0) o.code = T_DIAG1 + rpos[b];
-                    else o.code = T_DIAG_T;
-                    o.p2 = (uint8_t)b;
-                } else if (s.kind == S_PARITY) {
-                    for (auto x : s.tgt) {
-                        if (loc[x] >= 0) o.pm |= 1u << loc[x];
-                        else o.pmg |= uint64_t(1) << x;
-                    }
-                    o.code = (o.pm & rmask) == 0 && !o.grad ? T_PAR_T : T_PAR;
-                } else {  // S_DIAG: index over the gate's bits, targets first
-                    std::vector<uint32_t> L = s.tgt;
-                    L.insert(L.end(), s.ctl.begin(), s.ctl.end());
-                    c.nt = (uint8_t)s.tgt.size();
-                    c.nbits = (uint8_t)L.size();
-                    int reg = -1, nr = 0;
-                    for (size_t q = 0; q < L.size(); ++q)
-                        if (rpos[loc[L[q]]] >= 0) {
-                            reg = (int)q;
-                            ++nr;
-                        }
-                    uint8_t pos[3] = {31, 31, 31};
-                    c.src[0] = c.src[1] = c.src[2] = 255;
-                    if (nr == 1 && !o.grad) {  // the register bit last
-                        int at = 0;
-                        for (size_t q = 0; q < L.size(); ++q) {
-                            const int j3 = (int)q == reg ? 2 : at++;
-                            pos[j3] = (uint8_t)loc[L[q]];
-                            c.src[j3] = (uint8_t)q;
-                        }
-                        o.code = T_DIAG1 + rpos[loc[L[reg]]];
-                    } else {
-                        uint32_t ds = 0;
-                        for (size_t q = 0; q < L.size(); ++q) {
-                            pos[q] = (uint8_t)loc[L[q]];
-                            c.src[q] = (uint8_t)q;
-                        }
-                        // the generator's index has the gate's bits lowest; the table's has them highest
-                        for (int e = 0; e < 8; ++e)
-                            ds |= ((s.dsign >> (2 * (e >> (3 - (int)L.size())))) & 3u) << (2 * e);
-                        o.dsign = ds;
-                        o.code = nr == 0 && !o.grad ? T_DIAG_T : T_DIAG;
-                    }
-                    o.p0 = pos[0];
-                    o.p1 = pos[1];
-                    o.p2 = pos[2];
-                }
-                for (auto m : s.mems) B.mem_list.push_back(m);
-                D.ncoef += (uint32_t)coef_slots(s, REV);
-                B.steps.push_back(c);
-                B.ops.push_back(o);
-            }
-        }
-        for (int b = 0; b < 12; ++b) sg.fcol[b] = (uint16_t)tswz<R>(place[b]);
-        sg.nph = (uint32_t)B.phases.size() - sg.ph_begin;
-        sg.nops = (uint32_t)B.ops.size() - sg.op_begin;
-        sg.ncoef = D.ncoef - sg.coef_begin;
-        sg.ngrad = (uint32_t)grads.size();
-        D.segs.push_back((uint32_t)B.segs.size());
-        D.grad_steps.push_back(grads);
-        B.segs.push_back(sg);
+    B.rec.ncoef = 0;
+    auto coef = [&](uint32_t si, SKind kind, const TOp &, const uint8_t *src, const int *, uint32_t at) {
+        const Step &s = P.steps[si];
+        CoefStep c{};
+        c.kind = kind;
+        c.mem_begin = (uint32_t)B.mem_list.size();
+        c.nmem = (uint16_t)s.mems.size();
+        c.coef = at;
+        c.nt = (uint8_t)s.tgt.size();
+        c.nbits = (uint8_t)(s.tgt.size() + s.ctl.size());
+        for (int j = 0; j < 3; ++j) c.src[j] = src[j];
+        for (auto m : s.mems) B.mem_list.push_back(m);
+        B.steps.push_back(c);
+    };
+    for (const Piece &p : plan_segments<R, REV>(P.steps, order, n, kt_cap, !REV, kMaxTCoefs, B.rec, coef)) {
+        D.segs.push_back((uint32_t)p.seg);
+        D.grad_steps.push_back(p.grads);
     }
+    D.ncoef = B.rec.ncoef + (B.rec.ncoef & 1);
     D.step_count = (uint32_t)B.steps.size() - D.step_begin;
 }
 
@@ -388,11 +146,6 @@ std::string structure_key(const std::vector<HostOp> &ops, uint32_t n) {
     return k;
 }
 
-template <typename R, bool REV> size_t seg_smem(const TSeg &s) {
-    return (REV ? 2 : 1) * (sizeof(C<R>) << s.kt) + s.nops * sizeof(TOp) + s.ncoef * sizeof(C<R>) +
-           s.nph * sizeof(TPhase) + (REV ? (size_t)s.ngrad * 4 * kTWarps * sizeof(double) : 0);
-}
-
 template <typename R, bool REV>
 void make_launches(Batch &B, Program &T, const Builder &bd, const std::vector<Plan> &plans,
                    const std::vector<uint32_t> &plan_of, std::vector<Job> &jobs, std::vector<GradRef> &refs,
@@ -407,7 +160,7 @@ void make_launches(Batch &B, Program &T, const Builder &bd, const std::vector<Pl
         uint64_t tiles = 0;
         for (uint32_t c = 0; c < B.ncirc; ++c) {
             const PlanDir &D = plans[plan_of[c]].dir[dir];
-            if (l < D.segs.size()) tiles += uint64_t(1) << std::max(0, (int)B.nq[c] - (int)bd.segs[D.segs[l]].kt);
+            if (l < D.segs.size()) tiles += uint64_t(1) << std::max(0, (int)B.nq[c] - (int)bd.rec.segs[D.segs[l]].kt);
         }
         uint64_t per = 1;
         while (per * 2 * 8 * (uint64_t)(sm_count() * G::minb) <= tiles) per *= 2;
@@ -421,7 +174,7 @@ void make_launches(Batch &B, Program &T, const Builder &bd, const std::vector<Pl
         for (uint32_t c = 0; c < B.ncirc; ++c) {
             const PlanDir &D = plans[plan_of[c]].dir[dir];
             if (l >= D.segs.size()) continue;
-            const TSeg &s = bd.segs[D.segs[l]];
+            const TSeg &s = bd.rec.segs[D.segs[l]];
             const uint64_t nt = uint64_t(1) << std::max(0, (int)B.nq[c] - (int)s.kt);
             const uint64_t nparts = (nt + per - 1) / per;
             for (uint64_t p = 0; p < nparts; ++p) {
@@ -563,9 +316,9 @@ template <typename R> void build(Batch &B, Planned &P) {
     }
     T.nchunks = (uint32_t)chunks.size();
     upload(B, T.circs, circs);
-    upload(B, T.segs, bd.segs);
-    upload(B, T.phases, bd.phases);
-    upload(B, T.ops, bd.ops);
+    upload(B, T.segs, bd.rec.segs);
+    upload(B, T.phases, bd.rec.phases);
+    upload(B, T.ops, bd.rec.ops);
     upload(B, T.jobs, jobs);
     upload(B, T.mems, mems);
     upload(B, T.mem_base, mem_base);

@@ -25,6 +25,7 @@
 // H_k = A_k^dagger G_k A_k, A_k the product of the inverses undone before it.
 
 namespace tiles {
+using namespace steps;
 
 // One gate of one circuit, as its coefficients are formed (per circuit; the plan is shared by all
 // circuits of the same structure).
@@ -34,7 +35,6 @@ struct Mem {
     uint32_t cidx;
 };
 
-enum SKind : uint8_t { S_RUN = 0, S_DIAGRUN = 1, S_DENSE = 2, S_DIAG = 3, S_PARITY = 4, S_NONE = 5 };
 // How a step's coefficients are formed: members in op order, index into the plan's member list.
 struct CoefStep {
     uint32_t mem_begin, coef;  // coef: position in the circuit's coefficient array of this direction
@@ -43,55 +43,6 @@ struct CoefStep {
     uint8_t src[3];            // S_DIAG: index bit (2 - j) of the table is the gate's bit src[j] (255: none)
 };
 
-// Step codes; + register bit, or + index of a register bit pair (pair_index).
-enum TCode : uint16_t {
-    T_DIAG_T = 0,    // diagonal table on thread bits: one factor for the thread
-    T_PAR_T = 1,     // parity on thread bits
-    T_DIAG = 2,      // diagonal table on any bits
-    T_PAR = 3,       // parity on any bits
-    T_SIGN_T = 4,    // -1 where every control bit (all thread bits) is set
-    T_DIAG1 = 8,     // table whose lowest index bit is the register bit, the others thread bits
-    T_SIGN1 = 12,    // -1: one register bit and thread bits
-    T_DENSE = 16,    // 2x2 on the register bit
-    T_DENSEC = 20,   // with controls
-    T_CX_T = 24,     // swap along the register bit, controls all thread bits
-    T_CX_G = 28,     // swap along the register bit, any controls
-    T_SIGN2 = 32,    // -1: two register bits and thread bits
-    T_SWAP = 40,     // exchange of a pair of register bits, any controls
-    T_CX_R = 48,     // + target * 4 + control: swap along target, control one register bit (and thread bits)
-};
-
-struct alignas(16) TOp {
-    uint16_t code, coef;   // coef: position in the segment's coefficients
-    uint16_t creg;         // controls among the register bits
-    uint16_t grad;         // 1 + gradient row of the segment, 0: not differentiated
-    uint32_t cthr;         // controls among the thread bits (tile positions)
-    uint32_t pm;           // parity: tile bits
-    uint64_t pmg;          // parity: state bits outside the tile
-    uint8_t p0, p1, p2, pad;
-    uint32_t dsign;        // T_DIAG with a gradient: generator entry of index i in bits 2i (1: +1, 2: -1)
-};
-// CNOT and SWAP steps move no data.  A segment keeps a GF(2)-linear map from the tile position of an
-// amplitude to the place where it lies in shared memory; a CNOT between phases replaces the column of
-// its control bit by (control column XOR target column), and the tile's store reads through the last
-// map.  A phase loads and stores its amplitudes through its map: places, not positions, so no thread
-// touches another's amplitudes and no extra barrier is needed.
-struct TPhase {
-    uint16_t op_begin, nops;
-    uint8_t rb[4];     // register bits (tile positions, ascending)
-    uint8_t rt[4];     // tile position of register bit j
-    uint16_t tcol[8];  // place of each thread index bit (swizzled)
-    uint16_t rcol[4];  // place of each register bit (swizzled)
-    uint32_t pad;
-};
-struct alignas(16) TSeg {
-    uint32_t ph_begin, nph, op_begin, nops;
-    uint32_t coef_begin, ncoef, ngrad;
-    uint8_t lbits[16];
-    uint8_t gbits[32];
-    uint16_t fcol[12];  // places of the tile bits when the tile is stored (swizzled)
-    uint8_t ng, kt, pad[2];
-};
 struct alignas(16) Job {
     uint32_t seg, circ;
     uint32_t tile0, ntiles;
@@ -107,28 +58,7 @@ struct TCirc {
     uint32_t term_begin, nterms, nobs, out_begin;
 };
 
-template <typename R, bool REV> struct TGeo;
-template <> struct TGeo<float, false> { static constexpr int kt = 12, a = 4, A = 16, reserve = 4, minb = 3; };
-template <> struct TGeo<float, true> { static constexpr int kt = 12, a = 4, A = 16, reserve = 4, minb = 2; };
-template <> struct TGeo<double, false> { static constexpr int kt = 12, a = 4, A = 16, reserve = 3, minb = 2; };
-template <> struct TGeo<double, true> { static constexpr int kt = 11, a = 3, A = 8, reserve = 3, minb = 2; };
-constexpr int kTThreads = 256;
-constexpr int kTWarps = kTThreads / 32;
-constexpr int kMaxTOps = 160, kMaxTCoefs = 640, kMaxTGrads = 64;
 constexpr int kChunkBits = 12;  // amplitudes of one block of the measurement kernels: 16 a thread
-
-// Shared-memory position of tile amplitude l (linear over XOR): the lowest bits take the XOR of the
-// next six, so lanes that differ in any five tile bits spread over the banks for nearly every choice
-// of register bits.  complex64 keeps bit 0 in place: 16-byte pairs stay together.
-template <typename R> __host__ __device__ __forceinline__ uint32_t tswz(uint32_t l) {
-    if constexpr (sizeof(R) == 8) return l ^ ((l >> 3) & 7u) ^ ((l >> 6) & 7u);
-    else return l ^ (((l >> 4) & 7u) << 1) ^ (((l >> 7) & 7u) << 1);
-}
-
-__host__ __device__ constexpr int pair_mask(int i) {
-    return i == 0 ? 3 : i == 1 ? 5 : i == 2 ? 6 : i == 3 ? 9 : i == 4 ? 10 : 12;
-}
-__host__ __device__ constexpr int low_of(int m) { return m & -m; }
 
 struct TArgs {
     const Job *jobs;
@@ -142,393 +72,6 @@ struct TArgs {
     const int *skip;  // forward inside a VJP: nonzero when pool A already holds the states
 };
 
-// ---- steps in registers ----------------------------------------------------------------------
-template <typename R> __device__ __forceinline__ C<R> tprod(C<R> m, C<R> v) { return cmul1<R>(m, v); }
-template <> __device__ __forceinline__ float2 tprod<float>(float2 m, float2 v) { return cmul2(m, v); }
-
-template <typename R> __device__ __forceinline__ C<R> flip_sign(C<R> v, uint32_t neg) {  // neg: 0 or 1 << 31
-    if constexpr (sizeof(R) == 4) {
-        return make_float2(__uint_as_float(__float_as_uint(v.x) ^ neg), __uint_as_float(__float_as_uint(v.y) ^ neg));
-    } else {
-        const int h = (int)neg;
-        return make_double2(__hiloint2double(__double2hiint(v.x) ^ h, __double2loint(v.x)),
-                            __hiloint2double(__double2hiint(v.y) ^ h, __double2loint(v.y)));
-    }
-}
-
-// Two FP32 values in one 64-bit register (the paired FP32 instructions' operand).  As float2 the halves
-// are separate registers to the compiler, which then moved the whole state on every step (335 moves a
-// step); a 64-bit value keeps its pair from step to step.
-using pair2 = unsigned long long;
-__device__ __forceinline__ pair2 pk(float x, float y) {
-    pair2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 unpk(pair2 a) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
-    return r;
-}
-__device__ __forceinline__ pair2 mul2(pair2 a, pair2 b) {
-    pair2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ pair2 fma2(pair2 a, pair2 b, pair2 c) {
-    pair2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
-// A thread's amplitudes.  complex64 keeps real and imaginary parts apart and packs the two
-// amplitudes that differ in register bit 0, so that the paired FP32 instructions work on two
-// amplitude pairs at once without swapping or broadcasting any amplitude part; steps on register
-// bit 0 itself use scalar FMAs (the planner gives that bit to the wire with the fewest steps).  Per
-// differentiated 2x2 step on 16 + 16 amplitudes: 128 paired FMAs for both states and 60 for the four
-// sums, against 128 + 64 register swaps and 112 scalar operations with (re, im) pairs; with CNOTs in the
-// address map the 1024-circuit step went from 28.5 to 23.9 ms.
-template <typename R, int A> struct Regs {
-    C<R> v[A];
-    __device__ __forceinline__ C<R> get(int g) const { return v[g]; }
-    __device__ __forceinline__ void set(int g, C<R> x) { v[g] = x; }
-};
-template <int A> struct Regs<float, A> {
-    pair2 re[A / 2], im[A / 2];
-    __device__ __forceinline__ float2 get(int g) const {
-        const float2 r = unpk(re[g >> 1]), i = unpk(im[g >> 1]);
-        return (g & 1) ? make_float2(r.y, i.y) : make_float2(r.x, i.x);
-    }
-    __device__ __forceinline__ void set(int g, float2 x) {
-        const float2 r = unpk(re[g >> 1]), i = unpk(im[g >> 1]);
-        re[g >> 1] = (g & 1) ? pk(r.x, x.x) : pk(x.x, r.y);
-        im[g >> 1] = (g & 1) ? pk(i.x, x.y) : pk(x.y, i.y);
-    }
-};
-
-// ys = M (x, y) on every pair of the register bit; four roundings a component
-template <typename R, int A, int BIT, bool CTL>
-__device__ __forceinline__ void t_dense(Regs<R, A> &v, uint32_t creg, const C<R> (&m)[4]) {
-    constexpr int B = 1 << BIT;
-    if constexpr (sizeof(R) == 4 && BIT > 0 && !CTL) {
-        pair2 mr[4], mi[4], mn[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            mr[i] = pk(m[i].x, m[i].x);
-            mi[i] = pk(m[i].y, m[i].y);
-            mn[i] = pk(-m[i].y, -m[i].y);
-        }
-#pragma unroll
-        for (int h = 0; h < A / 2; ++h) {
-            if (h & (B >> 1)) continue;
-            const int k = h | (B >> 1);
-            const pair2 xr = v.re[h], xi = v.im[h], yr = v.re[k], yi = v.im[k];
-            v.re[h] = fma2(mn[1], yi, fma2(mr[1], yr, fma2(mn[0], xi, mul2(mr[0], xr))));
-            v.im[h] = fma2(mi[1], yr, fma2(mr[1], yi, fma2(mi[0], xr, mul2(mr[0], xi))));
-            v.re[k] = fma2(mn[3], yi, fma2(mr[3], yr, fma2(mn[2], xi, mul2(mr[2], xr))));
-            v.im[k] = fma2(mi[3], yr, fma2(mr[3], yi, fma2(mi[2], xr, mul2(mr[2], xi))));
-        }
-    } else {
-#pragma unroll
-        for (int g = 0; g < A; ++g) {
-            if (g & B) continue;
-            if (CTL && ((uint32_t)g & creg) != creg) continue;
-            const C<R> x = v.get(g), y = v.get(g | B);
-            C<R> p, q;
-            p.x = fma(-m[1].y, y.y, fma(m[1].x, y.x, fma(-m[0].y, x.y, m[0].x * x.x)));
-            p.y = fma(m[1].y, y.x, fma(m[1].x, y.y, fma(m[0].y, x.x, m[0].x * x.y)));
-            q.x = fma(-m[3].y, y.y, fma(m[3].x, y.x, fma(-m[2].y, x.y, m[2].x * x.x)));
-            q.y = fma(m[3].y, y.x, fma(m[3].x, y.y, fma(m[2].y, x.x, m[2].x * x.y)));
-            v.set(g, p);
-            v.set(g | B, q);
-        }
-    }
-}
-// the four sums of a differentiated step on register bit BIT: each pair's values in the state's
-// precision, the sums in FP64
-template <typename R, int A, int BIT, bool CTL>
-__device__ __forceinline__ void t_cross(const Regs<R, A> &v, const Regs<R, A> &w, uint32_t creg, double (&s)[4]) {
-    constexpr int B = 1 << BIT;
-    if constexpr (sizeof(R) == 4 && BIT > 0 && !CTL) {
-        const pair2 minus = pk(-1.0f, -1.0f);
-#pragma unroll
-        for (int h = 0; h < A / 2; ++h) {
-            if (h & (B >> 1)) continue;
-            const int k = h | (B >> 1);
-            const pair2 a0r = v.re[h], a0i = v.im[h], a1r = v.re[k], a1i = v.im[k];
-            const pair2 b0r = w.re[h], b0i = w.im[h], b1r = w.re[k], b1i = w.im[k];
-            const pair2 n0i = mul2(b0i, minus), n1i = mul2(b1i, minus), n1r = mul2(b1r, minus);
-            const float2 x1 = unpk(fma2(b0r, a0i, mul2(n0i, a0r)));
-            const float2 x2 = unpk(fma2(b1r, a1i, mul2(n1i, a1r)));
-            const float2 s1 = unpk(fma2(n1i, a0r, fma2(b1r, a0i, fma2(n0i, a1r, mul2(b0r, a1i)))));
-            const float2 s2 = unpk(fma2(n1i, a0i, fma2(n1r, a0r, fma2(b0i, a1i, mul2(b0r, a1r)))));
-            s[0] += (double)x1.x;
-            s[1] += (double)x2.x;
-            s[2] += (double)s1.x;
-            s[3] += (double)s2.x;
-            s[0] += (double)x1.y;
-            s[1] += (double)x2.y;
-            s[2] += (double)s1.y;
-            s[3] += (double)s2.y;
-        }
-    } else {
-#pragma unroll
-        for (int g = 0; g < A; ++g) {
-            if (g & B) continue;
-            if (CTL && ((uint32_t)g & creg) != creg) continue;
-            const C<R> a0 = v.get(g), a1 = v.get(g | B), b0 = w.get(g), b1 = w.get(g | B);
-            s[0] += (double)fma(b0.x, a0.y, -(b0.y * a0.x));
-            s[1] += (double)fma(b1.x, a1.y, -(b1.y * a1.x));
-            s[2] += (double)fma(-b1.y, a0.x, fma(b1.x, a0.y, fma(-b0.y, a1.x, b0.x * a1.y)));
-            s[3] += (double)fma(-b1.y, a0.y, fma(-b1.x, a0.x, fma(b0.y, a1.y, b0.x * a1.x)));
-        }
-    }
-}
-template <typename R, int A, int BIT>
-__device__ __forceinline__ void t_diag1(Regs<R, A> &v, C<R> f0, C<R> f1) {
-#pragma unroll
-    for (int g = 0; g < A; ++g) v.set(g, tprod<R>((g >> BIT) & 1 ? f1 : f0, v.get(g)));
-}
-template <typename R, int A, int MASK> __device__ __forceinline__ void t_sign(Regs<R, A> &v, uint32_t neg) {
-#pragma unroll
-    for (int g = 0; g < A; ++g)
-        if ((g & MASK) == MASK) v.set(g, flip_sign<R>(v.get(g), neg));
-}
-template <typename R, int A, int BIT, int CMASK> __device__ __forceinline__ void t_cx(Regs<R, A> &v, bool on) {
-    constexpr int B = 1 << BIT;
-#pragma unroll
-    for (int g = 0; g < A; ++g) {
-        if ((g & B) || (g & CMASK) != CMASK) continue;
-        const C<R> x = v.get(g), y = v.get(g | B);
-        v.set(g, on ? y : x);
-        v.set(g | B, on ? x : y);
-    }
-}
-template <typename R, int A, int BIT>
-__device__ __forceinline__ void t_cxg(Regs<R, A> &v, uint32_t creg, bool on) {
-    constexpr int B = 1 << BIT;
-#pragma unroll
-    for (int g = 0; g < A; ++g) {
-        if (g & B) continue;
-        const bool d = on && ((uint32_t)g & creg) == creg;
-        const C<R> x = v.get(g), y = v.get(g | B);
-        v.set(g, d ? y : x);
-        v.set(g | B, d ? x : y);
-    }
-}
-template <typename R, int A, int MASK>
-__device__ __forceinline__ void t_swap(Regs<R, A> &v, uint32_t creg, bool on) {
-    constexpr int LO = low_of(MASK), HI = MASK ^ LO;
-#pragma unroll
-    for (int g = 0; g < A; ++g) {
-        if (g & MASK) continue;
-        const bool d = on && ((uint32_t)g & creg) == creg;
-        const C<R> x = v.get(g | LO), y = v.get(g | HI);
-        v.set(g | LO, d ? y : x);
-        v.set(g | HI, d ? x : y);
-    }
-}
-
-// Sum of each of four values over the warp, with the exchange halving what each lane carries: lane
-// 16 p + 8 q (+ 0..7) ends with the sum of value 2 p + q.  Fixed order.
-__device__ __forceinline__ double reduce4(const double (&s)[4]) {
-    const int lane = threadIdx.x & 31;
-    const bool hi = lane & 16, hq = lane & 8;
-    double k0 = hi ? s[2] : s[0], k1 = hi ? s[3] : s[1];
-    k0 += __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], 16);
-    k1 += __shfl_xor_sync(0xffffffffu, hi ? s[1] : s[3], 16);
-    double r = hq ? k1 : k0;
-    r += __shfl_xor_sync(0xffffffffu, hq ? k0 : k1, 8);
-#pragma unroll
-    for (int off = 4; off > 0; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
-    return r;
-}
-__device__ __forceinline__ void add_sums(double *sacc, uint32_t row, const double (&s)[4]) {
-    const double r = reduce4(s);
-    const int lane = threadIdx.x & 31;
-    if ((lane & 7) == 0) sacc[(row * 4 + (lane >> 3)) * kTWarps + (threadIdx.x >> 5)] += r;
-}
-
-// The register bits b for which a step code exists in this geometry (a of the four).
-#define TILE_EACH_BIT(X) X(0) X(1) X(2) X(3)
-#define TILE_EACH_PAIR(X) X(0) X(1) X(2) X(3) X(4) X(5)
-
-// One step on the thread's amplitudes of NS states (w is v where there is one state).
-template <typename R, int A, int NS>
-__device__ __forceinline__ void t_step(Regs<R, A> &v, Regs<R, A> &w, const TOp &op, const C<R> *__restrict__ scf,
-                                       double *sacc, uint32_t base, uint64_t tbase, const uint32_t (&rbit)[4], C<R> &tf,
-                                       bool &has_tf, uint32_t &neg) {
-    const C<R> *cf = scf + op.coef;
-    const bool on = (base & op.cthr) == op.cthr;
-    auto position = [&](int g) {  // tile position of register g
-        uint32_t l = base;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if ((g >> j) & 1) l |= rbit[j];
-        return l;
-    };
-    // the codes nearly every step has, ahead of the others: a two-level branch instead of a search
-    // through the whole table
-    if ((op.code & ~3) == T_DENSE) {
-        const C<R> m[4] = {cf[0], cf[1], cf[2], cf[3]};
-        const bool grad = NS == 2 && op.grad;
-        double s[4] = {0.0, 0.0, 0.0, 0.0};
-#define TILE_DENSE(b)                                                                                          \
-    if constexpr ((1 << b) < A) {                                                                              \
-        if (grad) t_cross<R, A, b, false>(v, w, 0, s);                                                         \
-        t_dense<R, A, b, false>(v, 0, m);                                                                      \
-        if (NS == 2) t_dense<R, A, b, false>(w, 0, m);                                                         \
-    }
-        if (op.code & 2) {
-            if (op.code & 1) { TILE_DENSE(3) } else { TILE_DENSE(2) }
-        } else {
-            if (op.code & 1) { TILE_DENSE(1) } else { TILE_DENSE(0) }
-        }
-#undef TILE_DENSE
-        if (grad) add_sums(sacc, op.grad - 1u, s);
-        return;
-    }
-    switch (op.code) {
-    case T_DIAG_T: {
-        const uint32_t idx = (((base >> op.p0) & 1u) << 2) | (((base >> op.p1) & 1u) << 1) | ((base >> op.p2) & 1u);
-        tf = has_tf ? tprod<R>(cf[idx], tf) : cf[idx];
-        has_tf = true;
-        break;
-    }
-    case T_PAR_T: {
-        const int par = (__popcll(tbase & op.pmg) + __popc(base & op.pm)) & 1;
-        tf = has_tf ? tprod<R>(cf[par], tf) : cf[par];
-        has_tf = true;
-        break;
-    }
-    case T_SIGN_T: neg ^= on ? 0x80000000u : 0u; break;
-    case T_DIAG: {
-        double s[4] = {0.0, 0.0, 0.0, 0.0};
-        const bool grad = NS == 2 && op.grad;
-#pragma unroll
-        for (int g = 0; g < A; ++g) {
-            const uint32_t x = position(g);
-            const uint32_t idx = (((x >> op.p0) & 1u) << 2) | (((x >> op.p1) & 1u) << 1) | ((x >> op.p2) & 1u);
-            if (grad) {
-                const uint32_t d = (op.dsign >> (2 * idx)) & 3u;
-                const C<R> a = v.get(g), b = w.get(g);
-                const double im = (double)fma(b.x, a.y, -(b.y * a.x));
-                s[0] += d == 1u ? im : d == 2u ? -im : 0.0;
-            }
-            const C<R> f = cf[idx];
-            v.set(g, tprod<R>(f, v.get(g)));
-            if (NS == 2) w.set(g, tprod<R>(f, w.get(g)));
-        }
-        if (grad) add_sums(sacc, op.grad - 1u, s);
-        break;
-    }
-    case T_PAR: {
-        double s[4] = {0.0, 0.0, 0.0, 0.0};
-        const bool grad = NS == 2 && op.grad;
-        const int tp = __popcll(tbase & op.pmg) & 1;
-        const C<R> f0 = cf[0], f1 = cf[1];
-#pragma unroll
-        for (int g = 0; g < A; ++g) {
-            const bool odd = ((__popc(position(g) & op.pm) + tp) & 1) != 0;
-            if (grad) {
-                const C<R> a = v.get(g), b = w.get(g);
-                const double im = (double)fma(b.x, a.y, -(b.y * a.x));
-                s[0] += odd ? -im : im;
-            }
-            const C<R> f = odd ? f1 : f0;
-            v.set(g, tprod<R>(f, v.get(g)));
-            if (NS == 2) w.set(g, tprod<R>(f, w.get(g)));
-        }
-        if (grad) add_sums(sacc, op.grad - 1u, s);
-        break;
-    }
-#define TILE_BIT_CASES(b)                                                                                      \
-    case T_DIAG1 + b:                                                                                          \
-        if constexpr ((1 << b) < A) {                                                                          \
-            const uint32_t i = ((((base >> op.p0) & 1u) << 1) | ((base >> op.p1) & 1u)) * 2u;                  \
-            const C<R> f0 = cf[i], f1 = cf[i + 1];                                                             \
-            t_diag1<R, A, b>(v, f0, f1);                                                                       \
-            if (NS == 2) t_diag1<R, A, b>(w, f0, f1);                                                          \
-        }                                                                                                      \
-        break;                                                                                                 \
-    case T_SIGN1 + b:                                                                                          \
-        if constexpr ((1 << b) < A) {                                                                          \
-            const uint32_t sg = on ? 0x80000000u : 0u;                                                         \
-            t_sign<R, A, 1 << b>(v, sg);                                                                       \
-            if (NS == 2) t_sign<R, A, 1 << b>(w, sg);                                                          \
-        }                                                                                                      \
-        break;                                                                                                 \
-    case T_DENSEC + b:                                                                                         \
-        if constexpr ((1 << b) < A) {                                                                          \
-            const C<R> m[4] = {cf[0], cf[1], cf[2], cf[3]};                                                    \
-            if (NS == 2 && op.grad) {                                                                          \
-                double s[4] = {0.0, 0.0, 0.0, 0.0};                                                            \
-                if (on) t_cross<R, A, b, true>(v, w, op.creg, s);                                              \
-                add_sums(sacc, op.grad - 1u, s);                                                               \
-            }                                                                                                  \
-            if (on) {                                                                                          \
-                t_dense<R, A, b, true>(v, op.creg, m);                                                         \
-                if (NS == 2) t_dense<R, A, b, true>(w, op.creg, m);                                            \
-            }                                                                                                  \
-        }                                                                                                      \
-        break;                                                                                                 \
-    case T_CX_T + b:                                                                                           \
-        if constexpr ((1 << b) < A) {                                                                          \
-            t_cx<R, A, b, 0>(v, on);                                                                           \
-            if (NS == 2) t_cx<R, A, b, 0>(w, on);                                                              \
-        }                                                                                                      \
-        break;                                                                                                 \
-    case T_CX_G + b:                                                                                           \
-        if constexpr ((1 << b) < A) {                                                                          \
-            t_cxg<R, A, b>(v, op.creg, on);                                                                    \
-            if (NS == 2) t_cxg<R, A, b>(w, op.creg, on);                                                       \
-        }                                                                                                      \
-        break;
-        TILE_EACH_BIT(TILE_BIT_CASES)
-#undef TILE_BIT_CASES
-#define TILE_PAIR_CASES(i)                                                                                     \
-    case T_SIGN2 + i:                                                                                          \
-        if constexpr (pair_mask(i) < A) {                                                                      \
-            const uint32_t sg = on ? 0x80000000u : 0u;                                                         \
-            t_sign<R, A, pair_mask(i)>(v, sg);                                                                 \
-            if (NS == 2) t_sign<R, A, pair_mask(i)>(w, sg);                                                    \
-        }                                                                                                      \
-        break;                                                                                                 \
-    case T_SWAP + i:                                                                                           \
-        if constexpr (pair_mask(i) < A) {                                                                      \
-            t_swap<R, A, pair_mask(i)>(v, op.creg, on);                                                        \
-            if (NS == 2) t_swap<R, A, pair_mask(i)>(w, op.creg, on);                                           \
-        }                                                                                                      \
-        break;
-        TILE_EACH_PAIR(TILE_PAIR_CASES)
-#undef TILE_PAIR_CASES
-#define TILE_CX_CASE(t, c)                                                                                     \
-    case T_CX_R + t * 4 + c:                                                                                   \
-        if constexpr (t != c && (1 << t) < A && (1 << c) < A) {                                                \
-            t_cx<R, A, t, 1 << c>(v, on);                                                                      \
-            if (NS == 2) t_cx<R, A, t, 1 << c>(w, on);                                                         \
-        }                                                                                                      \
-        break;
-#define TILE_CX_CASES(t) TILE_CX_CASE(t, 0) TILE_CX_CASE(t, 1) TILE_CX_CASE(t, 2) TILE_CX_CASE(t, 3)
-        TILE_EACH_BIT(TILE_CX_CASES)
-#undef TILE_CX_CASES
-#undef TILE_CX_CASE
-    default: break;
-    }
-}
-
-__device__ __forceinline__ uint64_t spread(uint64_t x, const uint8_t *pos, int nbits) {
-    uint64_t r = 0;
-    for (int i = 0; i < nbits; ++i) r |= ((x >> i) & 1u) << pos[i];
-    return r;
-}
-template <typename T> __device__ __forceinline__ void copy_words(T *dst, const T *src, uint32_t n) {
-    static_assert(sizeof(T) % 8 == 0, "records are whole 8-byte words");
-    const uint2 *s = reinterpret_cast<const uint2 *>(src);
-    uint2 *d = reinterpret_cast<uint2 *>(dst);
-    for (uint32_t i = threadIdx.x; i < n * (uint32_t)(sizeof(T) / 8); i += blockDim.x) d[i] = s[i];
-}
-
 // One job: a few tiles of one circuit's segment.  Forward: one state; REV: lambda (pool A) and the
 // bra (pool B).  256 threads (fewer for narrow circuits) and one tile buffer per state; the two or
 // three CTAs an SM holds overlap one another's tile moves, staging and barriers.
@@ -536,12 +79,9 @@ template <typename R, bool REV>
 __global__ void __launch_bounds__(kTThreads, TGeo<R, REV>::minb) k_tiles(TArgs args) {
     using G = TGeo<R, REV>;
     constexpr int A = G::A, NS = REV ? 2 : 1;
-    constexpr int V = 16 / (int)sizeof(C<R>);
-    constexpr int PER = A / V;
     if (args.skip && *args.skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ TSeg sg;
-    __shared__ uint64_t s_hi[PER];
     const Job jb = args.jobs[blockIdx.x];
     if (threadIdx.x < sizeof(TSeg) / 8)
         reinterpret_cast<uint64_t *>(&sg)[threadIdx.x] = reinterpret_cast<const uint64_t *>(args.segs + jb.seg)[threadIdx.x];
@@ -560,124 +100,11 @@ __global__ void __launch_bounds__(kTThreads, TGeo<R, REV>::minb) k_tiles(TArgs a
     copy_words(sph, args.phases + sg.ph_begin, sg.nph);
     if (REV)
         for (uint32_t i = threadIdx.x; i < sg.ngrad * 4 * kTWarps; i += NT) sacc[i] = 0.0;
-    if (threadIdx.x < PER) s_hi[threadIdx.x] = spread((uint64_t)threadIdx.x * NT * V, sg.lbits, sg.kt);
-    const uint64_t lo = spread((uint64_t)threadIdx.x * V, sg.lbits, sg.kt);
     C<R> *const ga = static_cast<C<R> *>(args.pool_a) + off;
     C<R> *const gb = REV ? static_cast<C<R> *>(args.pool_b) + off : nullptr;
-    auto sw = [&](int j) { return tswz<R>((threadIdx.x + (uint32_t)j * NT) * V); };
-    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
-    for (uint32_t t = jb.tile0; t < jb.tile0 + jb.ntiles; ++t) {
-        const uint64_t tbase = spread(t, sg.gbits, sg.ng);
-        const bool fresh = !REV && (jb.flags & 1u);
-        if (fresh && t != 0) {  // |0..0> has no amplitude here, and a segment keeps zeros
-#pragma unroll
-            for (int j = 0; j < PER; ++j) {
-                const uint64_t x = tbase | lo | s_hi[j];
-                if (x < namp) *reinterpret_cast<float4 *>(ga + x) = z4;
-            }
-            continue;
-        }
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const uint64_t x = tbase | lo | s_hi[j];  // beyond the state in a tile padded to a warp's share
-            if (!fresh && x < namp) {
-                cp_async16(sl + sw(j), ga + x);
-                if (REV) cp_async16(sb + sw(j), gb + x);
-            } else {
-                *reinterpret_cast<float4 *>(sl + sw(j)) = z4;
-                if (REV) *reinterpret_cast<float4 *>(sb + sw(j)) = z4;
-            }
-        }
-        cp_async_commit();
-        cp_async_wait0();
-        if (fresh && threadIdx.x == 0) sl[0] = mk<R>(1, 0);  // thread 0 zeroed position 0 itself
-        __syncthreads();
-        for (uint32_t p = 0; p < sg.nph; ++p) {
-            const TPhase ph = sph[p];
-            uint32_t base = threadIdx.x, sbase = 0, rbit[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int j = 0; j < G::a; ++j) {
-                rbit[j] = 1u << ph.rt[j];
-                const uint32_t low = base & ((1u << ph.rb[j]) - 1u);
-                base = ((base ^ low) << 1) | low;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) sbase ^= (threadIdx.x >> j) & 1u ? ph.tcol[j] : 0u;
-            auto at = [&](int g) {
-                uint32_t x = sbase;
-#pragma unroll
-                for (int j = 0; j < G::a; ++j)
-                    if ((g >> j) & 1) x ^= ph.rcol[j];
-                return x;
-            };
-            Regs<R, A> v, w;
-            if constexpr (sizeof(R) == 4) {
-#pragma unroll
-                for (int g = 0; g < A; g += 2) {
-                    const C<R> x = sl[at(g)], y = sl[at(g + 1)];
-                    v.re[g / 2] = pk(x.x, y.x);
-                    v.im[g / 2] = pk(x.y, y.y);
-                    if (REV) {
-                        const C<R> p = sb[at(g)], q = sb[at(g + 1)];
-                        w.re[g / 2] = pk(p.x, q.x);
-                        w.im[g / 2] = pk(p.y, q.y);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int g = 0; g < A; ++g) {
-                    v.set(g, sl[at(g)]);
-                    if (REV) w.set(g, sb[at(g)]);
-                }
-            }
-            C<R> tf = mk<R>(1, 0);
-            bool has_tf = false;
-            uint32_t neg = 0;
-            for (uint32_t o = ph.op_begin, oe = ph.op_begin + ph.nops; o < oe; ++o)
-                t_step<R, A, NS>(v, w, sop[o], scf, sacc, base, tbase, rbit, tf, has_tf, neg);
-            if (has_tf) {
-#pragma unroll
-                for (int g = 0; g < A; ++g) {
-                    v.set(g, tprod<R>(tf, v.get(g)));
-                    if (REV) w.set(g, tprod<R>(tf, w.get(g)));
-                }
-            }
-#pragma unroll
-            for (int g = 0; g < A; ++g) {
-                sl[at(g)] = flip_sign<R>(v.get(g), neg);
-                if (REV) sb[at(g)] = flip_sign<R>(w.get(g), neg);
-            }
-            __syncthreads();
-        }
-        if (!(jb.flags & 2u)) {
-            constexpr int LV = V == 2 ? 1 : 0;
-            const int lt = 31 - __clz((int)NT);
-            uint32_t f0 = 0;
-            for (int i = 0; i < lt; ++i) f0 ^= (threadIdx.x >> i) & 1u ? sg.fcol[LV + i] : 0u;
-            auto chunk = [&](const C<R> *t, uint32_t f) {
-                if constexpr (V == 2) {
-                    const C<R> x = t[f], y = t[f ^ sg.fcol[0]];
-                    return make_float4(x.x, x.y, y.x, y.y);
-                } else {
-                    return *reinterpret_cast<const float4 *>(t + f);
-                }
-            };
-#pragma unroll
-            for (int j = 0; j < PER; ++j) {
-                const uint64_t x = tbase | lo | s_hi[j];
-                uint32_t f = f0;
-#pragma unroll
-                for (int i = 0; (1 << i) < PER; ++i)
-                    if ((j >> i) & 1) f ^= sg.fcol[LV + lt + i];
-                if (x < namp) {
-                    *reinterpret_cast<float4 *>(ga + x) = chunk(sl, f);
-                    if (REV) *reinterpret_cast<float4 *>(gb + x) = chunk(sb, f);
-                }
-            }
-        }
-        __syncthreads();  // the buffer is refilled next
-    }
+    run_tiles<R, REV, false>(sg, sl, sb, sop, scf, sph, sacc, jb.tile0, uint64_t(jb.tile0) + jb.ntiles, 1,
+                             !REV && (jb.flags & 1u), !(jb.flags & 2u), ga, ga, gb, namp);
     if (REV) {
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < sg.ngrad * 4; i += NT) {

@@ -128,9 +128,8 @@ int sparse_lanes(uint64_t nrows, uint64_t nnz);
 void sample_mcmc(const void *state, uint32_t nq, int dtype, int proposal, uint64_t burnin, uint64_t nshots,
                  uint64_t nchains, uint64_t seed, uint64_t *idx_dev, cudaStream_t st);
 // Fused application of compiled gates to one state (sv_fused.cu): runs of gates that
-// fit a shared-memory tile of 2^fused_tile_bits amplitudes share one pass over the
+// fit a shared-memory tile (sv_plan.hpp) share one pass over the
 // state; other gates go through apply_single, in order.
-int fused_tile_bits(int dtype, uint32_t nq);
 bool fused_worthwhile(int dtype, uint32_t nq, size_t ngates, cudaStream_t st);
 // One step of the adjoint reverse sweep: the inverse of an op and, when the op is
 // differentiated, its generator G with alpha = -2 * scale, and the Jacobian column.
