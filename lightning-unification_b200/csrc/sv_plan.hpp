@@ -194,14 +194,36 @@ std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector
             ph.nops = (uint16_t)cur.size();
             int rpos[32];
             std::vector<int> reg;  // register j's tile bit: fewest steps first (Regs)
-            for (int b = 0, j = 0, t = 0; b < kt; ++b) {
+            std::vector<int> thr;  // thread bit j's tile bit
+            for (int b = 0; b < kt; ++b) {
                 rpos[b] = -1;
-                if ((rmask >> b) & 1) {
-                    reg.push_back(b);
-                    ph.rb[j++] = (uint8_t)b;
-                } else {
-                    ph.tcol[t++] = (uint16_t)tswz<R>(place[b]);
+                ((rmask >> b) & 1 ? reg : thr).push_back(b);
+            }
+            // the thread bits within one wavefront (eight lanes of 16 bytes, sixteen of 8) first, with
+            // places whose bank bits are independent: those lanes hit different banks (27-qubit complex64
+            // circuit 26.4 -> 25.7 ms, 26-qubit complex128 18.9 -> 17.9 ms, against ascending order)
+            {
+                constexpr int q = sizeof(R) == 4 ? 4 : 3;
+                std::vector<int> front, back;
+                uint32_t basis[q] = {0};
+                for (int b : thr) {
+                    uint32_t v = tswz<R>(place[b]) & ((1u << q) - 1);
+                    for (int k = q - 1; k >= 0 && v; --k)
+                        if ((v >> k) & 1) {
+                            if (!basis[k]) {
+                                basis[k] = v;
+                                break;
+                            }
+                            v ^= basis[k];
+                        }
+                    (v ? front : back).push_back(b);
                 }
+                thr = front;
+                thr.insert(thr.end(), back.begin(), back.end());
+            }
+            for (size_t t = 0; t < thr.size(); ++t) {
+                ph.tval[t] = (uint16_t)(1u << thr[t]);
+                ph.tcol[t] = (uint16_t)(tswz<R>(place[thr[t]]) * sizeof(C<R>));
             }
             if (fixed) {
                 for (int j = 0; j < G::a; ++j) reg[j] = loc[fixed->tgt[3 - j]];
@@ -214,8 +236,9 @@ std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector
             for (int j = 0; j < G::a; ++j) {
                 rpos[reg[j]] = j;
                 ph.rt[j] = (uint8_t)reg[j];
-                ph.rcol[j] = (uint16_t)tswz<R>(place[reg[j]]);
+                ph.rcol[j] = (uint16_t)(tswz<R>(place[reg[j]]) * sizeof(C<R>));
             }
+            const size_t at_phase = B.phases.size();
             B.phases.push_back(ph);
             for (uint32_t i : cur) {
                 const uint32_t si = order[take[i]];
@@ -323,13 +346,14 @@ std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector
                     o.p1 = pos[1];
                     o.p2 = pos[2];
                 }
+                if (o.code == T_SIGN_T) B.phases[at_phase].signs = 1;
                 coef(si, kind, o, src, tr, B.ncoef);
                 B.ncoef += (uint32_t)(kind == S_WIDE ? coef_slots<R, REV>(s) - (sizeof(R) == 4 ? 1 : 0)
                                                      : coef_slots<R, REV>(s));
                 B.ops.push_back(o);
             }
         }
-        for (int b = 0; b < 12; ++b) sg.fcol[b] = (uint16_t)tswz<R>(place[b]);
+        for (int b = 0; b < 12; ++b) sg.fcol[b] = (uint16_t)(tswz<R>(place[b]) * sizeof(C<R>));
         sg.nph = (uint32_t)B.phases.size() - sg.ph_begin;
         sg.nops = (uint32_t)B.ops.size() - sg.op_begin;
         sg.ncoef = B.ncoef - sg.coef_begin;

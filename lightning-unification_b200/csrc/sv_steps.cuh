@@ -51,18 +51,21 @@ struct alignas(16) TOp {
 // touches another's amplitudes and no extra barrier is needed.
 struct TPhase {
     uint16_t op_begin, nops;
-    uint8_t rb[4];     // register bits (tile positions, ascending)
     uint8_t rt[4];     // tile position of register bit j
-    uint16_t tcol[8];  // place of each thread index bit (swizzled)
-    uint16_t rcol[4];  // place of each register bit (swizzled)
+    uint16_t tval[8];  // tile bit of each thread index bit: the planner orders them so that the lanes
+                       // of one shared-memory wavefront fall on different banks
+    uint16_t tcol[8];  // its place (swizzled, bytes)
+    uint16_t rcol[4];  // place of each register bit (swizzled, bytes)
+    uint32_t signs;    // some step is a sign on thread bits (T_SIGN_T)
     uint32_t pad;
 };
+static_assert(sizeof(TPhase) == 56, "phases are staged in 8-byte words");
 struct alignas(16) TSeg {
     uint32_t ph_begin, nph, op_begin, nops;
     uint32_t coef_begin, ncoef, ngrad;
     uint8_t lbits[16];
     uint8_t gbits[32];
-    uint16_t fcol[12];  // places of the tile bits when the tile is stored (swizzled)
+    uint16_t fcol[12];  // places of the tile bits when the tile is stored (swizzled, bytes)
     uint8_t ng, kt, pad[2];
 };
 template <typename R, bool REV> struct TGeo;
@@ -614,32 +617,62 @@ __device__ __forceinline__ void run_tiles(const TSeg &sg, C<R> *sl, C<R> *sb, co
     constexpr int A = G::A, NS = REV ? 2 : 1;
     constexpr int V = 16 / (int)sizeof(C<R>);
     constexpr int PER = A / V;
-    __shared__ uint64_t s_hi[PER];
-    const uint32_t NT = blockDim.x;
-    if (threadIdx.x < PER) s_hi[threadIdx.x] = spread((uint64_t)threadIdx.x * NT * V, sg.lbits, sg.kt);
+    // 16-byte chunk j of a thread: chunk threadIdx.x + j * blockDim.x of the tile.  Everything that
+    // depends on j alone comes from one 16-byte broadcast, everything that depends on the thread alone
+    // is formed once, and the tile's base is one bit per lane, so a chunk's move takes about six
+    // instructions besides the access (27 before: a quarter of a light segment's instructions).
+    constexpr int LV = V == 2 ? 1 : 0;
+    struct alignas(16) Chunk {
+        uint64_t off;     // bytes in the state
+        uint32_t sw, f;   // bytes in the tile: when loaded, and where the last map puts it
+    };
+    __shared__ Chunk s_ch[PER];
+    const uint32_t NT = blockDim.x, lane = threadIdx.x & 31;
+    const int lt = 31 - __clz((int)NT);
+    const bool padded = namp < (uint64_t(1) << sg.kt);
+    if (threadIdx.x < PER) {
+        const uint32_t l = threadIdx.x * NT * V;
+        Chunk c;
+        c.off = spread(l, sg.lbits, sg.kt) * sizeof(C<R>);
+        c.sw = tswz<R>(l) * (uint32_t)sizeof(C<R>);
+        c.f = 0;
+        for (int i = 0; (1 << i) < PER; ++i)
+            if ((threadIdx.x >> i) & 1) c.f ^= sg.fcol[LV + lt + i];
+        s_ch[threadIdx.x] = c;
+    }
     const uint64_t lo = spread((uint64_t)threadIdx.x * V, sg.lbits, sg.kt);
-    auto sw = [&](int j) { return tswz<R>((threadIdx.x + (uint32_t)j * NT) * V); };
+    const uint32_t sw0 = tswz<R>(threadIdx.x * V) * (uint32_t)sizeof(C<R>);
+    uint32_t f0 = 0;
+    for (int i = 0; i < lt; ++i) f0 ^= (threadIdx.x >> i) & 1u ? sg.fcol[LV + i] : 0u;
+    const uint32_t gpos = (int)lane < (int)sg.ng ? sg.gbits[lane] : 0u;
+    char *const cl = reinterpret_cast<char *>(sl), *const cb = reinterpret_cast<char *>(sb);
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     for (uint64_t t = t0; t < t1; t += stride) {
-        const uint64_t tbase = spread(t, sg.gbits, sg.ng);
+        const uint64_t mine = (int)lane < (int)sg.ng ? ((t >> lane) & 1u) << gpos : 0u;
+        const uint64_t tbase = (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)mine) |
+                               (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(mine >> 32)) << 32;
+        const uint64_t start = tbase | lo;
+        // beyond the state in a tile padded to a warp's share
+        auto outside = [&](const Chunk &c) { return padded && start + c.off / sizeof(C<R>) >= namp; };
         if (fresh && t != 0) {  // |0..0> has no amplitude here, and a segment keeps zeros
 #pragma unroll
             for (int j = 0; j < PER; ++j) {
-                const uint64_t x = tbase | lo | s_hi[j];
-                if (x < namp) *reinterpret_cast<float4 *>(a_out + x) = z4;
+                const Chunk c = s_ch[j];
+                if (!outside(c)) *reinterpret_cast<float4 *>(reinterpret_cast<char *>(a_out + start) + c.off) = z4;
             }
             continue;
         }
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            const uint64_t x = tbase | lo | s_hi[j];  // beyond the state in a tile padded to a warp's share
-            if (!fresh && x < namp) {
-                cp_async16(sl + sw(j), a_in + x);
-                if (REV) cp_async16(sb + sw(j), b + x);
+            const Chunk c = s_ch[j];
+            const uint32_t at = sw0 ^ c.sw;
+            if (!fresh && !outside(c)) {
+                cp_async16(cl + at, reinterpret_cast<const char *>(a_in + start) + c.off);
+                if (REV) cp_async16(cb + at, reinterpret_cast<const char *>(b + start) + c.off);
             } else {
-                *reinterpret_cast<float4 *>(sl + sw(j)) = z4;
-                if (REV) *reinterpret_cast<float4 *>(sb + sw(j)) = z4;
+                *reinterpret_cast<float4 *>(cl + at) = z4;
+                if (REV) *reinterpret_cast<float4 *>(cb + at) = z4;
             }
         }
         cp_async_commit();
@@ -648,15 +681,15 @@ __device__ __forceinline__ void run_tiles(const TSeg &sg, C<R> *sl, C<R> *sb, co
         __syncthreads();
         for (uint32_t p = 0; p < sg.nph; ++p) {
             const TPhase ph = sph[p];
-            uint32_t base = threadIdx.x, sbase = 0, rbit[4] = {0, 0, 0, 0};
+            uint32_t base = 0, sbase = 0, rbit[4] = {0, 0, 0, 0};
 #pragma unroll
-            for (int j = 0; j < G::a; ++j) {
-                rbit[j] = 1u << ph.rt[j];
-                const uint32_t low = base & ((1u << ph.rb[j]) - 1u);
-                base = ((base ^ low) << 1) | low;
+            for (int j = 0; j < G::a; ++j) rbit[j] = 1u << ph.rt[j];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const bool one = (threadIdx.x >> j) & 1u;
+                base |= one ? ph.tval[j] : 0u;
+                sbase ^= one ? ph.tcol[j] : 0u;
             }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) sbase ^= (threadIdx.x >> j) & 1u ? ph.tcol[j] : 0u;
             auto at = [&](int g) {
                 uint32_t x = sbase;
 #pragma unroll
@@ -664,15 +697,16 @@ __device__ __forceinline__ void run_tiles(const TSeg &sg, C<R> *sl, C<R> *sb, co
                     if ((g >> j) & 1) x ^= ph.rcol[j];
                 return x;
             };
+            auto amp = [](char *t, uint32_t x) -> C<R> & { return *reinterpret_cast<C<R> *>(t + x); };
             Regs<R, A> v, w;
             if constexpr (sizeof(R) == 4) {
 #pragma unroll
                 for (int g = 0; g < A; g += 2) {
-                    const C<R> x = sl[at(g)], y = sl[at(g + 1)];
+                    const C<R> x = amp(cl, at(g)), y = amp(cl, at(g + 1));
                     v.re[g / 2] = pk(x.x, y.x);
                     v.im[g / 2] = pk(x.y, y.y);
                     if (REV) {
-                        const C<R> p = sb[at(g)], q = sb[at(g + 1)];
+                        const C<R> p = amp(cb, at(g)), q = amp(cb, at(g + 1));
                         w.re[g / 2] = pk(p.x, q.x);
                         w.im[g / 2] = pk(p.y, q.y);
                     }
@@ -680,8 +714,8 @@ __device__ __forceinline__ void run_tiles(const TSeg &sg, C<R> *sl, C<R> *sb, co
             } else {
 #pragma unroll
                 for (int g = 0; g < A; ++g) {
-                    v.set(g, sl[at(g)]);
-                    if (REV) w.set(g, sb[at(g)]);
+                    v.set(g, amp(cl, at(g)));
+                    if (REV) w.set(g, amp(cb, at(g)));
                 }
             }
             C<R> tf = mk<R>(1, 0);
@@ -696,21 +730,25 @@ __device__ __forceinline__ void run_tiles(const TSeg &sg, C<R> *sl, C<R> *sb, co
                     if (REV) w.set(g, tprod<R>(tf, w.get(g)));
                 }
             }
+            if (ph.signs) {
+#pragma unroll
+                for (int g = 0; g < A; ++g) {
+                    v.set(g, flip_sign<R>(v.get(g), neg));
+                    if (REV) w.set(g, flip_sign<R>(w.get(g), neg));
+                }
+            }
 #pragma unroll
             for (int g = 0; g < A; ++g) {
-                sl[at(g)] = flip_sign<R>(v.get(g), neg);
-                if (REV) sb[at(g)] = flip_sign<R>(w.get(g), neg);
+                amp(cl, at(g)) = v.get(g);
+                if (REV) amp(cb, at(g)) = w.get(g);
             }
             __syncthreads();
         }
         if (store) {
-            constexpr int LV = V == 2 ? 1 : 0;
-            const int lt = 31 - __clz((int)NT);
-            uint32_t f0 = 0;
-            for (int i = 0; i < lt; ++i) f0 ^= (threadIdx.x >> i) & 1u ? sg.fcol[LV + i] : 0u;
-            auto chunk = [&](const C<R> *t, uint32_t f) {
+            auto chunk = [&](const char *t, uint32_t f) {
                 if constexpr (V == 2) {
-                    const C<R> x = t[f], y = t[f ^ sg.fcol[0]];
+                    const C<R> x = *reinterpret_cast<const C<R> *>(t + f);
+                    const C<R> y = *reinterpret_cast<const C<R> *>(t + (f ^ sg.fcol[0]));
                     return make_float4(x.x, x.y, y.x, y.y);
                 } else {
                     return *reinterpret_cast<const float4 *>(t + f);
@@ -718,15 +756,11 @@ __device__ __forceinline__ void run_tiles(const TSeg &sg, C<R> *sl, C<R> *sb, co
             };
 #pragma unroll
             for (int j = 0; j < PER; ++j) {
-                const uint64_t x = tbase | lo | s_hi[j];
-                uint32_t f = f0;
-#pragma unroll
-                for (int i = 0; (1 << i) < PER; ++i)
-                    if ((j >> i) & 1) f ^= sg.fcol[LV + lt + i];
-                if (x < namp) {
-                    if (a_out) *reinterpret_cast<float4 *>(a_out + x) = chunk(sl, f);
-                    if (REV) *reinterpret_cast<float4 *>(b + x) = chunk(sb, f);
-                }
+                const Chunk c = s_ch[j];
+                if (outside(c)) continue;
+                const uint32_t f = f0 ^ c.f;
+                if (a_out) *reinterpret_cast<float4 *>(reinterpret_cast<char *>(a_out + start) + c.off) = chunk(cl, f);
+                if (REV) *reinterpret_cast<float4 *>(reinterpret_cast<char *>(b + start) + c.off) = chunk(cb, f);
             }
         }
         __syncthreads();  // the buffer is refilled next
