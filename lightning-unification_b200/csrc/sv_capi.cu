@@ -106,7 +106,7 @@ void *scratch(b200sv_state *h, int i) {
 
 void apply_desc(b200sv_state *h, void *const *states, int nstates, const GateDesc &g) {
     if (g.kind == Kind::Dense && g.k >= 3) {
-        size_t need_b = g.k >= 4 ? h->amp_bytes() * g.m.size() : 0;
+        size_t need_b = g.k >= 4 ? sizeof(double2) * g.m.size() : 0;  // FP64 in either precision from 6 wires
         if (h->dtype == B200SV_C64 && dense_tc_applies(h->nq, g)) need_b = std::max(need_b, dense_tc_scratch_bytes(g.k));
         if (need_b) ensure_matrix(h, need_b);
     }

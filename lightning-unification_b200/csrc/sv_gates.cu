@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_dev(States s, DenseDevP<R, K
     }
 }
 
-// Dense blocks on K = 5..10 target bits (compute-bound from K = 5 in FP64): a register-tiled
+// Dense blocks on K = 9 and 10 target bits: a register-tiled
 // complex matrix product.  Each CTA takes tiles of 4096 amplitudes — TG = 4096 / 2^K
 // consecutive groups times all 2^K rows — staged in shared memory with coalesced loads
 // (consecutive threads take consecutive groups), and each thread accumulates a 4 x 4 block
@@ -270,11 +270,10 @@ template <int K> struct TiledShape {
     static constexpr int D = 1 << K;
     static constexpr int TG = kTileAmps / D;        // groups per tile
     static constexpr int RB = D / 4;                // row blocks
-    // matrix columns per staged chunk: the whole matrix when 2^K <= 32, else two buffers of
-    // 1024 entries, filled with cp.async one chunk ahead of the one being multiplied
-    static constexpr bool kResident = D <= 32;
-    static constexpr int CK = kResident ? D : 1024 / D;
-    static constexpr int MSH = kResident ? D * D : 2 * 1024;  // staged matrix entries
+    // matrix columns per staged chunk: two buffers of 1024 entries, filled with cp.async one chunk ahead
+    // of the one being multiplied
+    static constexpr int CK = 1024 / D;
+    static constexpr int MSH = 2 * 1024;  // staged matrix entries
     static_assert(kTiledThreads % TG == 0 && RB * (TG / 4) == kTiledThreads, "tile shape");
 };
 template <typename R, int K> struct TiledP {
@@ -287,7 +286,6 @@ template <typename R, int K>
 __global__ void __launch_bounds__(kTiledThreads, 2) k_dense_tiled(States s, TiledP<R, K> p) {
     using S = TiledShape<K>;
     constexpr int D = S::D, TG = S::TG, RB = S::RB, CK = S::CK, TG4 = TG / 4;
-    constexpr bool kResident = S::kResident;
     constexpr int kPieces = CK * D * (int)sizeof(C<R>) / 16;  // 16-byte pieces per chunk
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C<R> *tile = reinterpret_cast<C<R> *>(smem_raw);
@@ -301,8 +299,6 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_dense_tiled(States s, Tile
     constexpr int QS = kTiledThreads / TG;
     const uint64_t lo = p.ins((uint64_t)(t % TG));
     const int r0 = t / TG;
-    if constexpr (kResident)
-        for (int e = t; e < D * D; e += kTiledThreads) msh[e] = p.mt[e];
     auto stage = [&](int ci) {  // chunk ci (columns ci * CK ...) into buffer ci & 1
         const char *src = reinterpret_cast<const char *>(p.mt + (size_t)ci * CK * D);
         char *dst = reinterpret_cast<char *>(msh + (ci & 1) * CK * D);
@@ -312,23 +308,21 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_dense_tiled(States s, Tile
     for (uint64_t ti = blockIdx.x; ti < p.ntiles; ti += gridDim.x) {
         const uint64_t base = p.ins(ti * TG) | p.cmask | lo;
         __syncthreads();  // the previous tile has been stored and its chunks read
-        if constexpr (!kResident) stage(0);  // in flight during the tile load
+        stage(0);  // in flight during the tile load
 #pragma unroll
         for (int q = 0; q < kTileAmps / kTiledThreads; ++q)
             tile[t + q * kTiledThreads] = sv[base + p.off[r0 + q * QS]];
         __syncthreads();
         CAcc<R> acc[4][4];
         for (int ci = 0; ci < D / CK; ++ci) {
-            if constexpr (!kResident) {
-                if (ci + 1 < D / CK) {
-                    stage(ci + 1);
-                    cp_async_wait1();  // chunk ci has landed (this thread's pieces)
-                } else {
-                    cp_async_wait0();
-                }
-                __syncthreads();  // ... and every thread's
+            if (ci + 1 < D / CK) {
+                stage(ci + 1);
+                cp_async_wait1();  // chunk ci has landed (this thread's pieces)
+            } else {
+                cp_async_wait0();
             }
-            const C<R> *mc = msh + (kResident ? 0 : (ci & 1) * CK * D);
+            __syncthreads();  // ... and every thread's
+            const C<R> *mc = msh + (ci & 1) * CK * D;
             const C<R> *vc = tile + ci * CK * TG;
 #pragma unroll 4
             for (int c = 0; c < CK; ++c) {
@@ -342,7 +336,7 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_dense_tiled(States s, Tile
 #pragma unroll
                     for (int j = 0; j < 4; ++j) acc[i][j].add(m[i], v[j]);
             }
-            if constexpr (!kResident) __syncthreads();  // buffer ci & 1 is refilled by stage(ci + 2)
+            __syncthreads();  // buffer ci & 1 is refilled by stage(ci + 2)
         }
         __syncthreads();  // every thread has read the whole tile
 #pragma unroll
@@ -353,6 +347,121 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_dense_tiled(States s, Tile
 #pragma unroll
         for (int q = 0; q < kTileAmps / kTiledThreads; ++q)
             sv[base + p.off[r0 + q * QS]] = tile[t + q * kTiledThreads];
+    }
+}
+
+// Dense blocks on K = 5..8 target bits on the FP64 matrix instructions (mma m8n8k4).  The tiled kernel
+// above spends an instruction per FP64 FMA and reloads its operands from shared memory every four of
+// them (42-56 % of the FP64 pipe); an m8n8k4 does 256 FMAs and a warp's 16 x 32 block of complex outputs
+// needs six 16-byte loads per 32 of them.  complex64 states (K = 6..8; 3..5 run in sv_tensor.cu) are
+// widened as they enter the tile, so their sums are FP64 and rounded once, where the compensated FP32
+// sums took twice the FP64 pipe's time.  Tiles as in k_dense_tiled; rows of the tile and of the staged
+// matrix are padded by 32 bytes, so that the four columns by two rows (or groups) a quarter-warp loads
+// fall on different banks.  26 qubits, K = 5 / 6 / 7 / 8: complex128 1.12 -> 0.78, 1.79 -> 1.33, 3.19 ->
+// 2.50, 6.56 -> 4.93 ms (28 TFLOP/s at K = 8); complex64 K = 6 / 7 / 8 2.67 -> 1.17, 5.06 -> 2.32, 9.99 ->
+// 4.68 ms (29 TFLOP/s).  K = 4 measured the same as the register kernel (0.59 ms) and stays there.
+template <int K> struct MmaShape {
+    static constexpr int D = 1 << K, TG = kTileAmps / D;
+    static constexpr int WM = TG >= 32 ? 16 : 512 / TG, WN = 512 / WM;  // a warp's rows and groups
+    static constexpr int LDX = TG + 2, LDM = D + 2;                      // padded row lengths
+    static constexpr bool kResident = D <= 32;
+    static constexpr int CK = kResident ? D : 1024 / D;                  // matrix columns per staged chunk
+    static constexpr int MSH = (kResident ? D : 2 * CK) * LDM;
+    static_assert(CK % 4 == 0 && (D / WM) * (TG / WN) * 32 == kTiledThreads, "warp tiles");
+};
+template <int K> struct MmaP {
+    Insert ins;
+    uint64_t cmask, ntiles;
+    uint64_t off[1 << K];
+    const double2 *mt;  // transposed: mt[c * D + r]
+};
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+template <typename R, int K>
+__global__ void __launch_bounds__(kTiledThreads, 2) k_dense_mma(States s, MmaP<K> p) {
+    using S = MmaShape<K>;
+    constexpr int D = S::D, TG = S::TG, CK = S::CK, MI = S::WM / 8, NJ = S::WN / 8;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2 *tile = reinterpret_cast<double2 *>(smem_raw);  // [row][group], rows of LDX
+    double2 *msh = tile + D * S::LDX;                       // [column][row], columns of LDM
+    C<R> *__restrict__ sv = static_cast<C<R> *>(s.p[blockIdx.y]);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int row0 = (warp % (D / S::WM)) * S::WM, col0 = (warp / (D / S::WM)) * S::WN;
+    const int k4 = lane & 3, r8 = lane >> 2;
+    constexpr int QS = kTiledThreads / TG;  // thread t moves group t % TG of rows t / TG + q * QS
+    const uint64_t lo = p.ins((uint64_t)(t % TG));
+    const int mr = t / TG, mg = t % TG;
+    if constexpr (S::kResident)
+        for (int e = t; e < D * D; e += kTiledThreads)
+            msh[(e / D) * S::LDM + e % D] = p.mt[e];
+    auto stage = [&](int ci) {  // chunk ci (columns ci * CK ...) into buffer ci & 1
+        const double2 *src = p.mt + (size_t)ci * CK * D;
+        double2 *dst = msh + (ci & 1) * CK * S::LDM;
+        for (int e = t; e < CK * D; e += kTiledThreads) cp_async16(dst + (e / D) * S::LDM + e % D, src + e);
+        cp_async_commit();
+    };
+    for (uint64_t ti = blockIdx.x; ti < p.ntiles; ti += gridDim.x) {
+        const uint64_t base = p.ins(ti * TG) | p.cmask | lo;
+        __syncthreads();  // the previous tile has been stored and its chunks read
+        if constexpr (!S::kResident) stage(0);  // in flight during the tile load
+#pragma unroll
+        for (int q = 0; q < kTileAmps / kTiledThreads; ++q)
+            tile[(mr + q * QS) * S::LDX + mg] = widen<R>(sv[base + p.off[mr + q * QS]]);
+        __syncthreads();
+        double cr[MI][NJ][2], ci_[MI][NJ][2];
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) cr[i][j][0] = cr[i][j][1] = ci_[i][j][0] = ci_[i][j][1] = 0.0;
+        for (int ci = 0; ci < D / CK; ++ci) {
+            if constexpr (!S::kResident) {
+                if (ci + 1 < D / CK) {
+                    stage(ci + 1);
+                    cp_async_wait1();  // chunk ci has landed (this thread's pieces)
+                } else {
+                    cp_async_wait0();
+                }
+                __syncthreads();  // ... and every thread's
+            }
+            const double2 *mc = msh + (S::kResident ? 0 : (ci & 1) * CK * S::LDM) + k4 * S::LDM + row0 + r8;
+            const double2 *vc = tile + (ci * CK + k4) * S::LDX + col0 + r8;
+#pragma unroll 2
+            for (int c = 0; c < CK; c += 4) {
+                double2 a[MI], b[NJ];
+#pragma unroll
+                for (int i = 0; i < MI; ++i) a[i] = mc[c * S::LDM + i * 8];
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) b[j] = vc[c * S::LDX + j * 8];
+#pragma unroll
+                for (int i = 0; i < MI; ++i)
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) {
+                        dmma(cr[i][j], a[i].x, b[j].x);
+                        dmma(ci_[i][j], a[i].x, b[j].y);
+                        dmma(cr[i][j], -a[i].y, b[j].y);
+                        dmma(ci_[i][j], a[i].y, b[j].x);
+                    }
+            }
+            if constexpr (!S::kResident) __syncthreads();  // buffer ci & 1 is refilled by stage(ci + 2)
+        }
+        __syncthreads();  // every thread has read the whole tile
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    tile[(row0 + i * 8 + r8) * S::LDX + col0 + j * 8 + k4 * 2 + e] =
+                        make_double2(cr[i][j][e], ci_[i][j][e]);
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kTileAmps / kTiledThreads; ++q) {
+            const double2 v = tile[(mr + q * QS) * S::LDX + mg];
+            sv[base + p.off[mr + q * QS]] = mk<R>((R)v.x, (R)v.y);
+        }
     }
 }
 
@@ -541,10 +650,32 @@ bool launch_dense_k(const States &S, int ns, uint32_t nq, const GateDesc &g, voi
             return true;
         }
     }
-    // the tiled kernel where it measured faster than k_dense_dev on a 30-qubit state:
-    // complex128 from K = 5 (17.3 vs 21.0 ms at K = 5; 10.8 vs 9.8 ms at K = 4), complex64,
-    // whose compensated sums cost twice the FP64 ones, from K = 6 (42 vs 61 ms)
-    if constexpr (K >= (sizeof(R) == 8 ? 5 : 6)) {
+    // FP64 matrix instructions: complex128 from K = 5 and complex64 from K = 6 (3..5 went to the tensor
+    // cores above), as far as a tile of whole groups and a chunk of four columns fit
+    if constexpr (K >= (sizeof(R) == 8 ? 5 : 6) && K <= 8) {
+        using Sh = MmaShape<K>;
+        if (ngroups >= (uint64_t)Sh::TG) {
+            constexpr int D = Sh::D;
+            MmaP<K> p{};
+            std::vector<double2> mt((size_t)D * D);
+            for (int r = 0; r < D; ++r)
+                for (int c = 0; c < D; ++c) mt[(size_t)c * D + r] = cvt<double>(g.m[(size_t)r * D + c]);
+            // pageable source: cudaMemcpyAsync stages it before returning
+            B200SV_CUDA(cudaMemcpyAsync(scratch, mt.data(), mt.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
+            p.mt = static_cast<const double2 *>(scratch);
+            p.ins = make_insert(all);
+            p.cmask = ctrl_mask(g.cbits);
+            p.ntiles = ngroups / Sh::TG;
+            fill_offsets(p.off, g.tbits);
+            const int smem = (int)((D * Sh::LDX + Sh::MSH) * sizeof(double2));
+            B200SV_CUDA(cudaFuncSetAttribute(k_dense_mma<R, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            const uint64_t grid = std::min<uint64_t>(p.ntiles, uint64_t(sm_count()) * 2);
+            k_dense_mma<R, K><<<dim3((unsigned)grid, ns), kTiledThreads, smem, st>>>(S, p);
+            return true;
+        }
+        if constexpr (K > 6) return false;
+    }
+    if constexpr (K >= 9) {
         using Sh = TiledShape<K>;
         if (ngroups >= (uint64_t)Sh::TG) {
             constexpr int D = Sh::D;
@@ -565,7 +696,7 @@ bool launch_dense_k(const States &S, int ns, uint32_t nq, const GateDesc &g, voi
             k_dense_tiled<R, K><<<dim3((unsigned)grid, ns), kTiledThreads, smem, st>>>(S, p);
             return true;
         }
-        if constexpr (K > 6) return false;
+        return false;
     }
     if constexpr (sizeof(R) == 4 && K == 2) {
         const bool low2 = g.cbits.empty() && ((g.tbits[0] == 1 && g.tbits[1] == 0) || (g.tbits[0] == 0 && g.tbits[1] == 1));

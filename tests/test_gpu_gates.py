@@ -298,3 +298,27 @@ def test_apply_matrix_tensor_cores_c64(capi, k, n):
         want = O.apply_matrix(st.astype(np.complex128), u.astype(np.complex128), wires, inverse)
         assert np.abs(got - want).max() < TOL[np.complex64], (wires, inverse)
         assert abs(np.linalg.norm(got.astype(np.complex128)) - 1.0) < 1e-5
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+@pytest.mark.parametrize("k", [4, 5, 6, 7, 8])
+@pytest.mark.parametrize("n", [11, 12, 13, 15])
+def test_apply_matrix_fp64_mma(capi, n, k, dtype):
+    """Dense matrices on 4..8 wires (5..8 complex128, 6..8 complex64 on FP64 matrix instructions) around one tile of 4096 amplitudes (smaller states take the kernels
+    without tiles), on the lowest, highest and scattered wires, forward and inverse, against the oracle.
+    FP64 sums of 2^k products of a unitary: 1e-13 a normalised amplitude; complex64 rounds the inputs'
+    products once (the tensor-core widths 4 and 5 keep their bound of 2e-6)."""
+    import lq_oracle as O
+    from lightning_b200.workloads import random_unitary
+    rng = np.random.default_rng(1000 * n + k)
+    psi = (rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n))
+    psi = (psi / np.linalg.norm(psi)).astype(dtype)
+    u = random_unitary(rng, k).astype(dtype)
+    tol = 1e-13 if dtype == np.complex128 else 2e-6 if k < 6 else 1e-7
+    for wires in (list(range(n - k, n)), list(range(k))[::-1], [int(w) for w in rng.choice(n, k, replace=False)]):
+        for inverse in (False, True):
+            sv = capi.StateVector(n, dtype)
+            sv.upload(psi)
+            sv.apply_matrix(u, wires, inverse)
+            want = O.apply_matrix(psi.astype(np.complex128), u.astype(np.complex128), wires, inverse)
+            assert np.abs(sv.download() - want).max() < tol
