@@ -168,9 +168,10 @@ size_t run_offsets_doubles(uint64_t N);
 // O_1 (the CDF at every 32nd index) into the start of work
 template <typename R> void build_run_offsets(const void *psi, uint32_t nq, double *work, cudaStream_t st);
 void philox_uniforms(double *u, uint64_t n, uint64_t seed, cudaStream_t st);
-// inverse-CDF indices for nshots uniforms, CDF entries formed from O_1 and the state
+// inverse-CDF indices for nshots uniforms, CDF entries formed from O_1 (the start of work) and the
+// state; the end of work holds the search table
 template <typename R>
-void sample_runs(const void *psi, uint32_t nq, const double *o1, const double *u, uint64_t nshots, uint64_t *idx,
+void sample_runs(const void *psi, uint32_t nq, double *work, const double *u, uint64_t nshots, uint64_t *idx,
                  cudaStream_t st);
 
 }  // namespace b200sv

@@ -428,3 +428,25 @@ def test_mcmc_reference_golden(kernel):
     got = np.bincount(idx, minlength=8) / 100000
     want = [0.67078706, 0.03062806, 0.0870997, 0.00397696, 0.17564072, 0.00801973, 0.02280642, 0.00104134]
     assert np.abs(got - want).max() < 0.05
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 6, 7, 11, 17, 18])
+def test_sampling_search_levels(capi, n, dtype):
+    """The search's table, probes and bit pass at widths around a run (32 amplitudes) and the table's
+    depth (17 levels), with shot counts on both sides of the table's use: indices equal to the
+    oracle's plain search bit for bit."""
+    import lq_oracle as O
+    rng = np.random.default_rng(60 + n)
+    st = random_state(rng, n, dtype)
+    if n > 5:  # long stretches of equal CDF entries
+        st[: st.size // 3] = 0
+        st[rng.choice(st.size, st.size // 3, replace=False)] = 0
+        st = (st / np.linalg.norm(st.astype(np.complex128))).astype(dtype)
+    sv = capi.StateVector(n, dtype)
+    sv.upload(st)
+    cdf = O.cdf_fixed_order(st)
+    for shots in (1, 5, 4095, 4096, 9001):
+        u = rng.uniform(size=shots)
+        u[:1] = cdf[-1] if shots > 1 else u[:1]
+        assert np.array_equal(sv.sample(shots, uniforms=u), O.sample_kokkos_rule(cdf, u))
