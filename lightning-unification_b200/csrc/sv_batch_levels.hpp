@@ -335,6 +335,8 @@ template <typename R> void build(Batch &B, Planned &P) {
     T.h = B.dalloc<double4>(P.gscale.size());
     T.gpart = B.dalloc<double>(gpart);
     T.opart = B.dalloc<double>(opart);
+    for (const void *m : {(const void *)k_tile_expval<R>, (const void *)k_tile_bra<R>})
+        B200SV_CUDA(cudaFuncSetAttribute(m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem<R>()));
     uint32_t smem[2] = {0, 0};
     for (int d = 0; d < 2; ++d)
         for (const Launch &L : T.launches[d]) smem[d] = std::max(smem[d], L.smem);
@@ -411,7 +413,7 @@ template <typename R> void forward(Batch &B, double *out, cudaStream_t st) {
     launch_coefs<R>(B, 0, st);
     launch_levels<R, false>(B, nullptr, st);
     if (!B.total_obs) return;
-    k_tile_expval<R><<<T.nchunks, kTThreads, 0, st>>>(T.chunks, T.circs, B.d_terms, B.d_pool_a, T.opart);
+    k_tile_expval<R><<<T.nchunks, kTThreads, chunk_smem<R>(), st>>>(T.chunks, T.circs, B.d_terms, B.d_pool_a, T.opart);
     k_tile_outputs<<<(B.total_obs + 7) / 8, 256, 0, st>>>(T.orefs, B.total_obs, T.circs, B.d_terms, T.opart, out);
     B200SV_CUDA(cudaGetLastError());
     B.launched += 2;
@@ -424,7 +426,7 @@ template <typename R> void reverse(Batch &B, const double *dy, const int *reuse,
     launch_levels<R, false>(B, reuse, st);
     if (!B.ngslots) return;
     launch_coefs<R>(B, 1, st);
-    k_tile_bra<R><<<T.nchunks, kTThreads, 0, st>>>(T.chunks, T.circs, B.d_terms, B.d_pool_a, B.d_pool_b, dy);
+    k_tile_bra<R><<<T.nchunks, kTThreads, chunk_smem<R>(), st>>>(T.chunks, T.circs, B.d_terms, B.d_pool_a, B.d_pool_b, dy);
     launch_levels<R, true>(B, nullptr, st);
     k_tile_grads<<<std::max(1u, std::min(4096u, (B.ngslots + 127) / 128)), 128, 0, st>>>(T.grefs, T.h, T.gpart, B.ngslots,
                                                                                       B.d_gradw);
