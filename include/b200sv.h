@@ -166,13 +166,12 @@ int b200sv_apply_matrix(b200sv_handle h, const void *matrix,
 /* applyOperations: a list applied in order on the handle's stream. */
 int b200sv_apply_ops(b200sv_handle h, const b200sv_op *ops, uint32_t nops);
 /* applyOperations with gate fusion: the list is cut into segments whose wires
- * fit in a shared-memory tile (2^12 complex128 / 2^13 complex64 amplitudes, the
- * lowest wires filling the rest so loads coalesce), and each segment is one
- * pass over HBM instead of one pass per gate.  Same results as
- * b200sv_apply_ops to rounding (complex128: 1e-12).  Gates outside the tile
- * forms (more than three wires, dense matrices on three wires) run as their own
- * pass in order.  States narrower than the tile plus 8 wires use the per-gate
- * path. */
+ * fit in a shared-memory tile (2^12 amplitudes, the lowest wires filling the rest
+ * so loads coalesce), and each segment is one pass over HBM instead of one pass per
+ * gate.  Same results as b200sv_apply_ops to rounding (complex128: 1e-12).  Gates
+ * outside the tile forms (dense matrices on four and more wires) run as their own
+ * pass in order.  On states narrower than the tile, lists of fewer than four gates
+ * and streams being captured use one launch per gate. */
 int b200sv_apply_ops_fused(b200sv_handle h, const b200sv_op *ops, uint32_t nops);
 /* applyGenerator (LQ/StateVectorLQubit.hpp:250-275): G applied in place (it is
  * not unitary for projector-type generators); *scale receives the factor of
@@ -315,8 +314,10 @@ int b200sv_vjp_state(b200sv_handle psi, const b200sv_op *ops, uint32_t nops,
                      uint32_t ntrainable, int apply_operations, double *out);
 
 /* ---- batched engine ------------------------------------------------------ */
-/* A batch is a packed pool of independent circuits of uneven width, run by one
- * persistent kernel per step (optionally replayed as a CUDA graph).  Each circuit
+/* A batch is a packed pool of independent circuits of uneven width, run level by
+ * level (one launch takes a segment of every circuit) or, with two-wire dense gates,
+ * double excitations or wider matrices, by one persistent kernel; optionally replayed
+ * as a CUDA graph.  Each circuit
  * is an op list over its own wires 0..n_c-1 starting from |0...0>, followed by
  * an observable given as a Pauli-word sum.  Parameters live in one device array
  * so steps can change angles without rebuilding the batch.  Ops: every gate with at
@@ -357,8 +358,8 @@ int b200sv_batch_vjp(b200sv_batch_handle b, const double *params_device,
  * (the circuit's own referenced params in op order), circuit-major. */
 int b200sv_batch_jacobian(b200sv_batch_handle b, const double *params_device,
                           double *jac_device);
-/* Record the forward / vjp of this batch as CUDA graphs on first use and
- * replay them afterwards (0 = launch directly). */
+/* Record the forward / vjp of this batch as CUDA graphs on their second use and
+ * replay them afterwards (0 = launch directly, as the first use always does). */
 int b200sv_batch_use_graphs(b200sv_batch_handle b, int enable);
 /* Autotuner: times a forward + VJP step (best of three) for each candidate
  * launch shape (threads per CTA x tile width) and keeps the fastest; *chosen

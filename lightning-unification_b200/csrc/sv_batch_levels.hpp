@@ -428,7 +428,7 @@ template <typename R> void reverse(Batch &B, const double *dy, const int *reuse,
     launch_coefs<R>(B, 1, st);
     k_tile_bra<R><<<T.nchunks, kTThreads, chunk_smem<R>(), st>>>(T.chunks, T.circs, B.d_terms, B.d_pool_a, B.d_pool_b, dy);
     launch_levels<R, true>(B, nullptr, st);
-    k_tile_grads<<<std::max(1u, std::min(4096u, (B.ngslots + 127) / 128)), 128, 0, st>>>(T.grefs, T.h, T.gpart, B.ngslots,
+    k_tile_grads<<<std::max(1u, std::min(8192u, (B.ngslots + 15) / 16)), 128, 0, st>>>(T.grefs, T.h, T.gpart, B.ngslots,
                                                                                       B.d_gradw);
     B200SV_CUDA(cudaGetLastError());
     B.launched += 2;
