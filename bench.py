@@ -516,11 +516,11 @@ def matrix_sweep(nq: int, hbm_peak: float, kmax: int = 8, steps: int = 3):
 # grows in proportion to the state.
 RX_DRAM_BYTES_26Q = 1.0738e9 + 1.0144e9
 
-# DRAM bytes (read + write) of the forward and VJP launches of the batched kernel on 148
-# circuits of the batched-adjoint workload, from an ncu capture of `bench.py --case batch`;
-# circuits are independent, so a step's traffic scales with the number of circuits.
-BATCH_DRAM_BYTES_148 = (0.0397e9 + 0.9832e9) + (3.1324e9 + 3.5031e9)
-BATCH_ISSUE_ACTIVE = 0.47  # scheduler cycles issuing, same capture (forward 52 %, VJP 45 %, time-weighted)
+# DRAM bytes (read + write) of every launch of a forward + VJP step on 148 circuits of the
+# batched-adjoint workload, from an ncu capture of `bench.py --case batch`; circuits are
+# independent, so a step's traffic scales with the number of circuits.
+BATCH_DRAM_BYTES_148 = 3.798e9
+BATCH_ISSUE_ACTIVE = 0.53  # scheduler cycles issuing (forward and reverse levels alike)
 
 
 def run_case(args):
@@ -622,7 +622,7 @@ def run_case(args):
 
 def hea_forward(steps: int, warmup: int, ncirc: int = 4096, dtype=np.complex64, cpu: bool = False):
     """Batched hardware-efficient-ansatz forward (n ~ U[10, 20], depth ~ U[4, 16], 3n-term
-    Hamiltonian) in `dtype`, one persistent launch replayed as a CUDA graph, vs a per-circuit
+    Hamiltonian) in `dtype`, its launches replayed as a CUDA graph, vs a per-circuit
     loop through the plain C ABI on a sample (after one untimed circuit per width).  With
     `cpu`, the reference's own lightning.qubit on the host cores over a seeded subset (the
     first 16 circuits: forward, then the Hamiltonian's expectation value as one observable),
@@ -1037,7 +1037,7 @@ def main():
     line = {
         "metric": METRIC, "value": value, "unit": "circuits/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "c64 (fp32-pair compensated gates, fp64 reductions)",
+        "vs_baseline": None, "dtype": "c64 (fp32 amplitudes, gate products formed in fp64, fp64 reductions)",
         "data": "synthetic (seeded)",
         "config": {"workload": "batched adjoint: 1024 circuits x 16 qubits x 8 layers Rot(RZ RY RZ) + CNOT ring "
                                "(range (l mod 15)+1), 16 PauliZ observables, forward + VJP per step",
@@ -1059,13 +1059,13 @@ def main():
         "precision_sampling": precision,
         "roofline": roof,
         "roofline_batch": {
-            "kernel": "k_batch<float,0|1,false> (forward + VJP launch of the headline step)",
+            "kernel": "k_tiles<float,0|1> (segment levels of the headline step)",
             "bound": "issue", "hbm_traffic_per_step": BATCH_DRAM_BYTES_148 * ncirc / 148,
             "hbm_achieved_gbs": BATCH_DRAM_BYTES_148 * ncirc / 148 / (ms * 1e6),
             "hbm_frac": BATCH_DRAM_BYTES_148 * ncirc / 148 / (ms * 1e6) / hbm_peak, "peak_kind": peak_kind,
             "issue_active_frac": BATCH_ISSUE_ACTIVE,
-            "note": "per-circuit states stay in shared memory within a segment; the kernel is bound by "
-                    "instruction issue and latency (ncu: FMA pipe 20-23 %, shared memory 42-49 %), not by HBM"},
+            "note": "a launch runs one segment of every circuit on tiles in registers; bound by "
+                    "instruction issue and latency (ncu: FMA pipe 30-33 %, shared memory 30-46 %), not by HBM"},
         "cpu_baseline": cpu,
         "e2e": {"value": aggregate_rate(world, ncirc, e2e_ms), "unit": "circuits/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
