@@ -73,12 +73,12 @@ struct TArgs {
 };
 
 // One job: a few tiles of one circuit's segment.  Forward: one state; REV: lambda (pool A) and the
-// bra (pool B).  256 threads (fewer for narrow circuits) and one tile buffer per state; the two or
-// three CTAs an SM holds overlap one another's tile moves, staging and barriers.
+// bra (pool B).  256 threads (fewer for narrow circuits); the two or three CTAs an SM holds overlap one
+// another's tile moves, staging and barriers.
 template <typename R, bool REV>
 __global__ void __launch_bounds__(kTThreads, TGeo<R, REV>::minb) k_tiles(TArgs args) {
     using G = TGeo<R, REV>;
-    constexpr int A = G::A, NS = REV ? 2 : 1;
+    constexpr int A = G::A;
     if (args.skip && *args.skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ TSeg sg;
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kTThreads, TGeo<R, REV>::minb) k_tiles(TArgs a
     const uint32_t NT = blockDim.x, TN = NT * A;
     C<R> *const sl = reinterpret_cast<C<R> *>(smem_raw);
     C<R> *const sb = sl + TN;
-    TOp *const sop = reinterpret_cast<TOp *>(smem_raw + NS * sizeof(C<R>) * TN);
+    TOp *const sop = reinterpret_cast<TOp *>(smem_raw + tile_buffers<R, REV>() * sizeof(C<R>) * TN);
     C<R> *const scf = reinterpret_cast<C<R> *>(sop + sg.nops);
     TPhase *const sph = reinterpret_cast<TPhase *>(scf + sg.ncoef);
     double *const sacc = reinterpret_cast<double *>(sph + sg.nph);

@@ -9,7 +9,7 @@
 //
 // Against the previous kernels (512-thread CTAs, one per SM, tiles double-buffered, CNOTs exchanged in
 // registers, complex64 sums compensated in FP32 pairs, products per member in FP64): 200 random gates on
-// 26 qubits complex128 21.8 -> 17.9 ms and on 27 qubits complex64 39.0 -> 25.7 ms (error against 64 bits
+// 26 qubits complex128 21.8 -> 17.9 ms and on 27 qubits complex64 39.0 -> 24.7 ms (error against 64 bits
 // 6.2e-7 -> 5.3e-7), the 600-parameter Jacobian of 20 qubits 6.2 -> 4.1 ms a call.
 #include <algorithm>
 #include <cstring>
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kTThreads, 2) k_state(const C<R> *lam_in, C<R>
     const uint32_t NT = blockDim.x, TN = NT * G::A;
     C<R> *const sl = reinterpret_cast<C<R> *>(smem_raw);
     C<R> *const sb = sl + TN;
-    TOp *const sop = reinterpret_cast<TOp *>(smem_raw + (REV ? 2 : 1) * sizeof(C<R>) * TN);
+    TOp *const sop = reinterpret_cast<TOp *>(smem_raw + tile_buffers<R, REV>() * sizeof(C<R>) * TN);
     C<R> *const scf = reinterpret_cast<C<R> *>(sop + sg.nops);
     TPhase *const sph = reinterpret_cast<TPhase *>(scf + sg.ncoef);
     double *const sacc = reinterpret_cast<double *>(sph + sg.nph);

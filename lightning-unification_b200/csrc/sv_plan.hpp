@@ -366,7 +366,7 @@ std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector
 }
 
 template <typename R, bool REV> size_t seg_smem(const TSeg &s) {
-    return (REV ? 2 : 1) * (sizeof(C<R>) << s.kt) + s.nops * sizeof(TOp) + s.ncoef * sizeof(C<R>) +
+    return tile_buffers<R, REV>() * (sizeof(C<R>) << s.kt) + s.nops * sizeof(TOp) + s.ncoef * sizeof(C<R>) +
            s.nph * sizeof(TPhase) + (REV ? (size_t)s.ngrad * 4 * kTWarps * sizeof(double) : 0);
 }
 
