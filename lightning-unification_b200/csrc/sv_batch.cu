@@ -2089,7 +2089,10 @@ void build_program(Batch &B, const Config &cfg) {
     int per_sm = 1 << 30;
     for (int mode = 0; mode < 2; ++mode) {
         const void *k = batch_kernel(B.dtype, mode);
-        B200SV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B.smem_bytes));
+        // the limit is the function's, shared by every batch: the device's, not this batch's need
+        cudaFuncAttributes fa;
+        B200SV_CUDA(cudaFuncGetAttributes(&fa, k));
+        B200SV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm - (int)fa.sharedSizeBytes));
         int m = 0;
         B200SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k, cfg.threads, B.smem_bytes));
         per_sm = std::min(per_sm, m);

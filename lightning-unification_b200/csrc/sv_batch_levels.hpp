@@ -337,13 +337,10 @@ template <typename R> void build(Batch &B, Planned &P) {
     T.opart = B.dalloc<double>(opart);
     for (const void *m : {(const void *)k_tile_expval<R>, (const void *)k_tile_bra<R>})
         B200SV_CUDA(cudaFuncSetAttribute(m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem<R>()));
-    uint32_t smem[2] = {0, 0};
-    for (int d = 0; d < 2; ++d)
-        for (const Launch &L : T.launches[d]) smem[d] = std::max(smem[d], L.smem);
-    const void *k[2] = {(const void *)k_tiles<R, false>, (const void *)k_tiles<R, true>};
-    for (int d = 0; d < 2; ++d)
-        if (smem[d] > 48 * 1024)
-            B200SV_CUDA(cudaFuncSetAttribute(k[d], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[d]));
+    B200SV_CUDA(cudaFuncSetAttribute(k_tiles<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)max_seg_smem<R, false>(kMaxTCoefs)));
+    B200SV_CUDA(cudaFuncSetAttribute(k_tiles<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)max_seg_smem<R, true>(kMaxTCoefs)));
 }
 
 // coefficients of a direction from this launch's trigonometry

@@ -363,12 +363,10 @@ struct Blob {
     template <typename T> const T *at(size_t off) const { return reinterpret_cast<const T *>(dev + off); }
 };
 
-template <typename R, bool REV> void allow_smem(const Records &rec, size_t &most) {
-    most = 0;
-    for (const TSeg &s : rec.segs) most = std::max(most, seg_smem<R, REV>(s));
-    if (most > 227 * 1024) throw Unsupported("fused segment records exceed shared memory");
-    if (most > 48 * 1024)
-        B200SV_CUDA(cudaFuncSetAttribute(k_state<R, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+template <typename R, bool REV> void allow_smem() {
+    constexpr size_t most = max_seg_smem<R, REV>(kMaxStateCoefs);
+    static_assert(most <= 113 * 1024, "two CTAs an SM");
+    B200SV_CUDA(cudaFuncSetAttribute(k_state<R, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
 }
 // CTAs of a launch: four per resident slot, so that the last ones leave few SMs idle and each stages the
 // segment's records for several tiles
@@ -394,9 +392,8 @@ void run_fused(void *state, uint32_t nq, const std::vector<GateDesc> &descs,
     coefs.resize(rec.ncoef + 2, mk<R>(0, 0));
     Blob blob(st);
     const size_t o_seg = blob.add(rec.segs), o_ph = blob.add(rec.phases), o_op = blob.add(rec.ops), o_cf = blob.add(coefs);
-    size_t smem = 0;
     if (!rec.segs.empty()) {
-        allow_smem<R, false>(rec, smem);
+        allow_smem<R, false>();
         blob.upload();
     }
     for (const Piece &p : pieces) {
@@ -550,9 +547,8 @@ void run_fused_adjoint(void *&lam, void *&lam2, const std::vector<void *> &bras,
     Blob blob(st);
     const size_t o_seg = blob.add(rec.segs), o_ph = blob.add(rec.phases), o_op = blob.add(rec.ops),
                  o_cf = blob.add(coefs), o_br = blob.add(bras), o_gr = blob.add(grads);
-    size_t smem = 0;
     if (!rec.segs.empty()) {
-        allow_smem<R, true>(rec, smem);
+        allow_smem<R, true>();
         blob.upload();
         B200SV_CUDA(cudaMallocAsync((void **)&gpart, std::max<uint64_t>(1, ngpart) * sizeof(double), st));
     }

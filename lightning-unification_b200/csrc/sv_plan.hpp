@@ -369,6 +369,14 @@ template <typename R, bool REV> size_t seg_smem(const TSeg &s) {
     return tile_buffers<R, REV>() * (sizeof(C<R>) << s.kt) + s.nops * sizeof(TOp) + s.ncoef * sizeof(C<R>) +
            s.nph * sizeof(TPhase) + (REV ? (size_t)s.ngrad * 4 * kTWarps * sizeof(double) : 0);
 }
+// The most that any segment takes (a wide step's coefficients may start one further on, a phase holds
+// at least one step).  A kernel's shared-memory limit is set to this and not to one call's or batch's
+// need: the limit belongs to the function, so a later, smaller one would refuse the launches of
+// programs built before it.
+template <typename R, bool REV> constexpr size_t max_seg_smem(int max_coefs) {
+    return tile_buffers<R, REV>() * (sizeof(C<R>) << TGeo<R, REV>::kt) + kMaxTOps * (sizeof(TOp) + sizeof(TPhase)) +
+           (max_coefs + kMaxTOps) * sizeof(C<R>) + (REV ? (size_t)kMaxTGrads * 4 * kTWarps * sizeof(double) : 0);
+}
 
 }  // namespace steps
 }  // namespace b200sv

@@ -531,3 +531,47 @@ def test_batch_level_engine_every_gate(dtype, widths):
         assert np.abs(jac[jat:jat + size].reshape(len(obs), -1) - J).max() < GRAD_TOL[dtype]
         at, jat = at + len(obs), jat + size
     assert np.abs(g.cpu().numpy() - want_g).max() < GRAD_TOL[dtype]
+
+
+def layered_batch(n, layers, gates, ncirc=2, seed=5):
+    """ncirc circuits of `layers` layers of the one-wire `gates` on every wire and a CNOT ring."""
+    rng = np.random.default_rng(seed)
+    circuits, at = [], 0
+    for _ in range(ncirc):
+        ops, pidx = [], []
+        for l in range(layers):
+            for q in range(n):
+                for g in gates:
+                    ops.append((g, [q], False, []))
+                    pidx.append(at)
+                    at += 1
+            for q in range(n):
+                ops.append(("CNOT", [q, (q + 1 + l % (n - 1)) % n], False, []))
+                pidx.append(-1)
+        circuits.append({"num_qubits": n, "ops": ops, "param_index": pidx,
+                         "observables": [[(1.0, "Z", [0]), (0.5, "X", [n - 1])]]})
+    return circuits, rng.uniform(0, 2 * np.pi, at)
+
+
+@pytest.mark.parametrize("wide_gate", [False, True])
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+def test_engines_alive_together(dtype, wide_gate):
+    """Engines keep running after ones that need less shared memory were built: direct calls, recorded
+    graphs and their replays, on both batch kernels."""
+    import torch
+    from lightning_b200.batch import BatchedCircuits
+    engines = []
+    for n, layers in ((13, 7), (13, 6), (13, 1), (6, 1)):
+        circuits, params = layered_batch(n, layers, ("RX", "RY", "RZ"))
+        if wide_gate:
+            for c in circuits:
+                c["ops"].append(("IsingXX", [0, 1], False, [0.3]))
+                c["param_index"].append(-1)
+        eng = BatchedCircuits(circuits, len(params), dtype=dtype)
+        engines.append((eng, circuits, params))
+    for eng, circuits, params in engines:
+        p, dy = torch.tensor(params, device="cuda"), torch.ones(2, dtype=torch.float64, device="cuda")
+        want, gwant = oracle_outputs(circuits, params), oracle_vjp(circuits, params, np.ones(2))
+        for _ in range(3):  # direct, recorded, replayed
+            assert np.abs(eng.forward(p).cpu().numpy() - want).max() < (1e-12 if dtype == np.complex128 else 2e-5)
+            assert np.abs(eng.vjp(p, dy).cpu().numpy() - gwant).max() < GRAD_TOL[dtype]
