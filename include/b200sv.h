@@ -171,7 +171,8 @@ int b200sv_apply_ops(b200sv_handle h, const b200sv_op *ops, uint32_t nops);
  * gate.  Same results as b200sv_apply_ops to rounding (complex128: 1e-12).  Gates
  * outside the tile forms (dense matrices on four and more wires) run as their own
  * pass in order.  On states narrower than the tile, lists of fewer than four gates
- * and streams being captured use one launch per gate. */
+ * use one launch per gate; so does every call on a stream that is being captured,
+ * whose graph may be replayed after the call's own memory is gone. */
 int b200sv_apply_ops_fused(b200sv_handle h, const b200sv_op *ops, uint32_t nops);
 /* applyGenerator (LQ/StateVectorLQubit.hpp:250-275): G applied in place (it is
  * not unitary for projector-type generators); *scale receives the factor of

@@ -581,18 +581,17 @@ void run_fused_adjoint(void *&lam, void *&lam2, const std::vector<void *> &bras,
 }  // namespace
 
 // A state narrower than a tile is fused from four gates on: the records' upload and the launch
-// cost about as much as three gate launches.  While its stream is being captured it stays on the
-// per-gate launches, whose coefficients are kernel arguments: a replay must not read the records
-// from this call's host memory.  From one tile up every call is fused.
+// cost about as much as three gate launches.  From one tile up every call is fused.  While the stream is
+// being captured every width stays on the per-gate launches, whose coefficients are kernel arguments (or
+// kept with the graph, upload_matrix): a replay must not read the records from this call's host memory.
 bool fused_worthwhile(int dtype, uint32_t nq, size_t ngates, cudaStream_t st) {
-    if (nq >= (uint32_t)(dtype == B200SV_C64 ? TGeo<float, false>::kt : TGeo<double, false>::kt)) return true;
-    if (ngates < 4) return false;
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return status == cudaStreamCaptureStatusNone;
+    if (status != cudaStreamCaptureStatusNone) return false;
+    return nq >= (uint32_t)(dtype == B200SV_C64 ? TGeo<float, false>::kt : TGeo<double, false>::kt) || ngates >= 4;
 }
 
 void apply_fused(void *state, uint32_t nq, int dtype, const std::vector<GateDesc> &descs,

@@ -10,6 +10,7 @@
 // and GateImplementationsPI.hpp:248-289 / :785-799 (same index mathematics,
 // revWireParity generalised to any number of inserted bits).
 #include <algorithm>
+#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <vector>
@@ -660,8 +661,7 @@ bool launch_dense_k(const States &S, int ns, uint32_t nq, const GateDesc &g, voi
             std::vector<double2> mt((size_t)D * D);
             for (int r = 0; r < D; ++r)
                 for (int c = 0; c < D; ++c) mt[(size_t)c * D + r] = cvt<double>(g.m[(size_t)r * D + c]);
-            // pageable source: cudaMemcpyAsync stages it before returning
-            B200SV_CUDA(cudaMemcpyAsync(scratch, mt.data(), mt.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
+            upload_matrix(scratch, mt.data(), mt.size() * sizeof(double2), st);
             p.mt = static_cast<const double2 *>(scratch);
             p.ins = make_insert(all);
             p.cmask = ctrl_mask(g.cbits);
@@ -682,8 +682,7 @@ bool launch_dense_k(const States &S, int ns, uint32_t nq, const GateDesc &g, voi
             std::vector<C<R>> mt((size_t)D * D);
             for (int r = 0; r < D; ++r)
                 for (int c = 0; c < D; ++c) mt[(size_t)c * D + r] = cvt<R>(g.m[(size_t)r * D + c]);
-            // pageable source: cudaMemcpyAsync stages it before returning
-            B200SV_CUDA(cudaMemcpyAsync(scratch, mt.data(), mt.size() * sizeof(C<R>), cudaMemcpyHostToDevice, st));
+            upload_matrix(scratch, mt.data(), mt.size() * sizeof(C<R>), st);
             TiledP<R, K> p{};
             p.ins = make_insert(all);
             p.cmask = ctrl_mask(g.cbits);
@@ -737,8 +736,7 @@ bool launch_dense_k(const States &S, int ns, uint32_t nq, const GateDesc &g, voi
         fill_offsets(p.off, g.tbits);
         std::vector<C<R>> hm(g.m.size());
         for (size_t i = 0; i < g.m.size(); ++i) hm[i] = cvt<R>(g.m[i]);
-        // pageable source: cudaMemcpyAsync stages it before returning, so hm may go out of scope
-        B200SV_CUDA(cudaMemcpyAsync(scratch, hm.data(), hm.size() * sizeof(C<R>), cudaMemcpyHostToDevice, st));
+        upload_matrix(scratch, hm.data(), hm.size() * sizeof(C<R>), st);
         p.m = static_cast<const C<R> *>(scratch);
         k_dense_dev<R, K><<<grid_for(ngroups, ns), kThreads, 0, st>>>(S, p);
     }
@@ -815,7 +813,7 @@ void launch_gate(void *const *states, int nstates, uint32_t nq, const GateDesc &
             for (int j = 0; j < g.k; ++j) p.tmask[j] = uint64_t(1) << g.tbits[j];
             std::vector<C<R>> hm(g.m.size());
             for (size_t i = 0; i < g.m.size(); ++i) hm[i] = cvt<R>(g.m[i]);
-            B200SV_CUDA(cudaMemcpyAsync(scratch, hm.data(), hm.size() * sizeof(C<R>), cudaMemcpyHostToDevice, st));
+            upload_matrix(scratch, hm.data(), hm.size() * sizeof(C<R>), st);
             const size_t sm = sizeof(C<R>) << g.k;
             if (sm > 48 * 1024)
                 B200SV_CUDA(cudaFuncSetAttribute(k_dense_big<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -867,6 +865,25 @@ void launch_gate(void *const *states, int nstates, uint32_t nq, const GateDesc &
     default: break;
     }
     B200SV_CUDA(cudaGetLastError());
+}
+
+void upload_matrix(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    B200SV_CUDA(cudaStreamGetCaptureInfo(st, &status, &id, &graph));
+    if (status == cudaStreamCaptureStatusActive) {
+        auto kept = std::make_unique<std::vector<unsigned char>>(static_cast<const unsigned char *>(src),
+                                                                 static_cast<const unsigned char *>(src) + bytes);
+        src = kept->data();
+        cudaUserObject_t object;
+        B200SV_CUDA(cudaUserObjectCreate(
+            &object, kept.get(), [](void *p) { delete static_cast<std::vector<unsigned char> *>(p); }, 1,
+            cudaUserObjectNoDestructorSync));
+        kept.release();
+        B200SV_CUDA(cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove));
+    }
+    B200SV_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
 }
 
 template void launch_gate<float>(void *const *, int, uint32_t, const GateDesc &, void *, cudaStream_t);

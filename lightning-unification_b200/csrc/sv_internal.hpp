@@ -41,6 +41,11 @@ template <typename R>
 void launch_gate(void *const *states, int nstates, uint32_t nq, const GateDesc &g,
                  void *dev_matrix_scratch, cudaStream_t st);
 
+// Stream-ordered copy of a matrix from the call's own host memory (sv_gates.cu).  Pageable memory is staged
+// before cudaMemcpyAsync returns; on a stream being captured the copy happens at every replay, so there a
+// copy of the bytes goes with the graph, which frees it.
+void upload_matrix(void *dst, const void *src, size_t bytes, cudaStream_t st);
+
 // complex64 dense matrices on 3..5 wires on the tensor cores (sv_tensor.cu): applies when
 // the descriptor has no controls and the state holds at least one 128-group tile;
 // `scratch` must hold dense_tc_scratch_bytes(k) bytes (the split real-embedded matrix).

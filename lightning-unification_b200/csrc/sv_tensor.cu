@@ -254,8 +254,7 @@ void launch_tc(float2 *const *states, int ns, uint32_t nq, const GateDesc &g, vo
                     put(1, 2 * r + bb, 2 * c + aa, lo);
                 }
         }
-    // pageable source: cudaMemcpyAsync stages it before returning
-    B200SV_CUDA(cudaMemcpyAsync(scratch, blob.data(), blob.size(), cudaMemcpyHostToDevice, st));
+    upload_matrix(scratch, blob.data(), blob.size(), st);
     TcP p{};
     std::vector<uint32_t> bits = g.tbits;
     std::sort(bits.begin(), bits.end());

@@ -322,3 +322,39 @@ def test_apply_matrix_fp64_mma(capi, n, k, dtype):
             sv.apply_matrix(u, wires, inverse)
             want = O.apply_matrix(psi.astype(np.complex128), u.astype(np.complex128), wires, inverse)
             assert np.abs(sv.download() - want).max() < tol
+
+
+@pytest.mark.parametrize("n,dtype", [(5, np.complex128), (11, np.complex64), (12, np.complex64), (12, np.complex128),
+                                     (14, np.complex64), (14, np.complex128)])
+def test_captured_lists_replay_after_the_call(capi, n, dtype):
+    """apply_ops_fused on a stream being captured, below, at and above the tile width: the graph is replayed
+    after the call's own memory is gone and written over, and applies the list both times."""
+    import torch
+    import lq_oracle as O
+    from lightning_b200.workloads import random_unitary
+    rng = np.random.default_rng(n)
+    ops = []
+    for _ in range(12):
+        ops += [("RX", [int(rng.integers(n))], False, [float(rng.uniform(0, 6))]),
+                ("CNOT", [int(x) for x in rng.choice(n, 2, replace=False)], False, []),
+                ("IsingZZ", [int(x) for x in rng.choice(n, 2, replace=False)], True, [float(rng.uniform(0, 6))])]
+    for k in (2, 3, 4, 5):
+        ops.append(("QubitUnitary", [int(x) for x in rng.choice(n, k, replace=False)], False, [], random_unitary(rng, k)))
+    psi = random_state(rng, n, dtype)
+    sv = capi.StateVector(n, dtype)
+    stream = torch.cuda.Stream()
+    sv.set_stream(stream.cuda_stream)
+    sv.apply_ops(ops)  # the matrix workspace, outside the capture
+    sv.upload(psi)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        sv.apply_ops_fused(ops)
+    want = psi.astype(np.complex128)
+    for _ in range(2):
+        junk = [np.full(s, np.nan) for s in (64, 600, 5000, 40000) for _ in range(20)]
+        with torch.cuda.stream(stream):
+            graph.replay()
+        stream.synchronize()
+        del junk
+        want = O.run_circuit(n, ops, state=want)
+        assert np.abs(sv.download() - want).max() < (1e-12 if dtype == np.complex128 else 2e-5)
