@@ -120,7 +120,7 @@ template <typename R, bool REV> void plan_dir(Builder &B, Plan &P, uint32_t n, i
         for (auto m : s.mems) B.mem_list.push_back(m);
         B.steps.push_back(c);
     };
-    for (const Piece &p : plan_segments<R, REV>(P.steps, order, n, kt_cap, !REV, kMaxTCoefs, B.rec, coef)) {
+    for (const Piece &p : plan_segments<R, REV>(P.steps, order, n, kt_cap, !REV, sizeof(R) == 4, kMaxTCoefs, B.rec, coef)) {
         D.segs.push_back((uint32_t)p.seg);
         D.grad_steps.push_back(p.grads);
     }

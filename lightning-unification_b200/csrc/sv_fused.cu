@@ -388,7 +388,7 @@ void run_fused(void *state, uint32_t nq, const std::vector<GateDesc> &descs,
     auto coef = [&](uint32_t si, SKind kind, const TOp &o, const uint8_t *src, const int *tr, uint32_t at) {
         put_coefs<R>(coefs, gs, all[si], kind, o, src, tr, at);
     };
-    const std::vector<Piece> pieces = plan_segments<R, false>(all, order, nq, 64, false, kMaxStateCoefs, rec, coef);
+    const std::vector<Piece> pieces = plan_segments<R, false>(all, order, nq, 64, false, false, kMaxStateCoefs, rec, coef);
     coefs.resize(rec.ncoef + 2, mk<R>(0, 0));
     Blob blob(st);
     const size_t o_seg = blob.add(rec.segs), o_ph = blob.add(rec.phases), o_op = blob.add(rec.ops), o_cf = blob.add(coefs);
@@ -495,7 +495,7 @@ void run_fused_adjoint(void *&lam, void *&lam2, const std::vector<void *> &bras,
     auto coef = [&](uint32_t si, SKind kind, const TOp &o, const uint8_t *src, const int *tr, uint32_t at) {
         put_coefs<R>(coefs, gs, all[si], kind, o, src, tr, at);
     };
-    const std::vector<Piece> pieces = plan_segments<R, true>(all, order, nq, 64, false, kMaxStateCoefs, rec, coef);
+    const std::vector<Piece> pieces = plan_segments<R, true>(all, order, nq, 64, false, false, kMaxStateCoefs, rec, coef);
     coefs.resize(rec.ncoef + 2, mk<R>(0, 0));
     const uint64_t namp = uint64_t(1) << nq;
     const int kt = tile_bits_of<R, true>(nq, 64);

@@ -77,10 +77,11 @@ template <typename R, bool REV> int tile_bits_of(uint32_t n, int cap) {
 // later one that fits the tile and commutes with the steps left out; each phase first puts the ready
 // CNOTs and SWAPs into the address map and then takes every ready step whose targets fit the
 // register bits.  coef(step index, effective kind, record, index bit sources, register of each target,
-// position) is called once per record; `even_empty` keeps one segment for a circuit without steps.
+// position) is called once per record; `even_empty` keeps one segment for a circuit without steps;
+// `exact_single` gives differentiated steps of one gate the controlled form (t_cross).
 template <typename R, bool REV, typename F>
 std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector<uint32_t> &order, uint32_t n, int cap,
-                                 bool even_empty, int max_coefs, Records &B, F &&coef) {
+                                 bool even_empty, bool exact_single, int max_coefs, Records &B, F &&coef) {
     using G = TGeo<R, REV>;
     const int kt = tile_bits_of<R, REV>(n, cap);
     const bool tiled = (int)n > kt;
@@ -285,7 +286,7 @@ std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector
                         o.code = T_SWAP + pair_index(rm);
                     }
                 } else if (kind == S_RUN) {
-                    o.code = T_DENSE + tr[0];
+                    o.code = (exact_single && o.grad && s.mems.size() == 1 ? T_DENSEC : T_DENSE) + tr[0];
                 } else if (kind == S_DENSE) {
                     control(s.ctl);
                     o.code = T_DENSEC + tr[0];

@@ -301,3 +301,32 @@ def test_fused_narrow_states(capi, n, dtype):
         got = sv.adjoint_jacobian(ops, o, tp)
         assert np.abs(got - O.adjoint_jacobian(st.astype(np.complex128), ops, o, tp)).max() < tol
     assert np.array_equal(sv.download(), st)
+
+
+@pytest.mark.parametrize("n", [6, 12, 14])
+@pytest.mark.parametrize("nobs", [1, 3])
+def test_complex64_generator_products_in_fp64(capi, n, nobs):
+    """The generator products of a complex64 Jacobian are formed and summed in FP64: with one step after the
+    state (a gate of each kind, or a run on one wire) and bras that are sign flips and permutations of it,
+    nothing is rounded to FP32, so the Jacobian is the oracle's on the same amplitudes to FP64 rounding
+    (2^n products of 1e-16; FP32 products miss by 1e-9)."""
+    import lq_oracle as O
+    from conftest import random_state
+    rng = np.random.default_rng(n)
+    psi = random_state(rng, n, np.complex64)
+    sv = capi.StateVector(n, np.complex64)
+    sv.upload(psi)
+    obs = [[(1.0, [("PauliZ", [2])])], [(1.0, [("PauliX", [n - 1]), ("PauliZ", [1])])], [(1.0, [("PauliX", [0])])]]
+    for o in ([obs[:1], obs[1:2]] if nobs == 1 else [obs]):
+        for q in (0, n // 2, n - 1):
+            p = (q + 1) % n
+            for ops in ([("RX", [q], False, [0.4])], [("RY", [q], True, [1.4])], [("RZ", [q], False, [2.4])],
+                        [("PhaseShift", [q], False, [0.9])], [("CRX", [q, p], False, [0.3])],
+                        [("CRY", [p, q], False, [0.8])], [("CRZ", [q, p], False, [1.1])],
+                        [("ControlledPhaseShift", [p, q], False, [0.6])], [("IsingZZ", [q, p], False, [0.7])],
+                        [("MultiRZ", [q, p, (p + 1) % n], False, [0.2])],
+                        [("RX", [q], False, [0.4]), ("RY", [q], False, [1.0]), ("RZ", [q], False, [2.0])]):
+                tp = list(range(len(ops)))
+                got = sv.adjoint_jacobian(ops, o, tp)
+                want = O.adjoint_jacobian(psi.astype(np.complex128), ops, o, tp)
+                assert np.abs(got - want).max() < 1e-13, (q, ops)
