@@ -142,6 +142,40 @@ __device__ __forceinline__ void mul22(const double2 (&x)[4], const double2 (&y)[
 #pragma unroll
         for (int j = 0; j < 2; ++j) r[i * 2 + j] = zadd(zmul(x[i * 2], y[j]), zmul(x[i * 2 + 1], y[2 + j]));
 }
+// A 2x2 matrix in twice FP64's length, h + l.  complex128 runs are multiplied so and rounded once (as the
+// single-state engine does on the host, sv_fused.cu): what their coefficients miss is the same on every
+// amplitude and adds up in the values.
+struct Mat2 {
+    double2 h[4], l[4];
+};
+struct Twofold {  // sum of products with its low part
+    double h, l;
+    __device__ __forceinline__ void add(double a, double al, double b, double bl) {
+        const double p = a * b, u = h + p, z = u - h;
+        l += ((h - (u - z)) + (p - z)) + fma(a, b, -p) + fma(a, bl, al * b);
+        h = u;
+    }
+};
+__device__ __forceinline__ void mul22(const Mat2 &x, Mat2 &y) {  // y = x y
+    Mat2 r;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            Twofold re{0.0, 0.0}, im{0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const double2 a = x.h[i * 2 + k], al = x.l[i * 2 + k], b = y.h[k * 2 + j], bl = y.l[k * 2 + j];
+                re.add(a.x, al.x, b.x, bl.x);
+                re.add(-a.y, -al.y, b.y, bl.y);
+                im.add(a.x, al.x, b.y, bl.y);
+                im.add(a.y, al.y, b.x, bl.x);
+            }
+            r.h[i * 2 + j] = make_double2(re.h + re.l, im.h + im.l);
+            r.l[i * 2 + j] = make_double2(re.l - (r.h[i * 2 + j].x - re.h), im.l - (r.h[i * 2 + j].y - im.h));
+        }
+    y = r;
+}
 // h of generator code 1 X, 2 Y, 3 Z, 4 |1><1| seen through A (H = A^dagger G A)
 __device__ __forceinline__ double4 gen_row(int code, const double2 (&Am)[4]) {
     const double2 z = make_double2(0, 0), one = make_double2(1, 0);
@@ -176,15 +210,21 @@ template <typename R> __global__ void k_tile_coefs(CoefArgs a) {
             const uint32_t *list = a.mem_list + st.mem_begin;
             C<R> *o = out + st.coef;
             if (st.kind == S_RUN || st.kind == S_DIAGRUN) {
-                double2 P[4] = {make_double2(1, 0), make_double2(0, 0), make_double2(0, 0), make_double2(1, 0)};
+                const double2 zero = make_double2(0, 0), one = make_double2(1, 0);
+                Mat2 run{{one, zero, zero, one}, {zero, zero, zero, zero}};
+                double2(&P)[4] = run.h;
                 for (int k = 0; k < st.nmem; ++k) {
                     const Mem &m = mems[list[rev ? st.nmem - 1 - k : k]];
                     if (rev && m.gslot >= 0) a.h[m.gslot] = gen_row(gen_code(m.gate), P);
-                    C<double> q[4];
-                    member_mat<double>(m, a.cs, a.consts, rev, q);
-                    double2 N[4];
-                    mul22(q, P, N);
-                    for (int e = 0; e < 4; ++e) P[e] = N[e];
+                    Mat2 q{{}, {zero, zero, zero, zero}};
+                    member_mat<double>(m, a.cs, a.consts, rev, q.h);
+                    if constexpr (sizeof(R) == 8) {
+                        mul22(q, run);
+                    } else {
+                        double2 N[4];
+                        mul22(q.h, P, N);
+                        for (int e = 0; e < 4; ++e) P[e] = N[e];
+                    }
                 }
                 if (st.kind == S_RUN) {
                     for (int e = 0; e < 4; ++e) o[e] = mk<R>((R)P[e].x, (R)P[e].y);

@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cstring>
 #include <functional>
+#include <type_traits>
 #include <vector>
 
 #include "sv_device.cuh"
@@ -173,6 +174,35 @@ void one_bit_matrix(const GateDesc &g, cd (&m)[4]) {
     }
 }
 
+// Product of a run's gates, rounded once: its rounding is the same on every amplitude and so adds up in the
+// values, where the rounding of single amplitudes averages out.  complex128 products are formed in extended
+// precision (600-parameter Jacobian of 20 qubits: error 2.1e-15 -> 1.3e-15 against gate by gate in 64 bits).
+template <typename R>
+void run_product(const std::vector<const GateDesc *> &gs, const std::vector<uint32_t> &mems, cd (&P)[4]) {
+    using L = std::conditional_t<sizeof(R) == 8, long double, double>;
+    if (mems.size() == 1) return one_bit_matrix(*gs[mems[0]], P);
+    L pr[4] = {1, 0, 0, 1}, pi[4] = {0, 0, 0, 0};
+    for (uint32_t i : mems) {
+        cd m[4];
+        one_bit_matrix(*gs[i], m);
+        L mr[4], mi[4], nr[4], ni[4];
+        for (int e = 0; e < 4; ++e) {
+            mr[e] = m[e].real();
+            mi[e] = m[e].imag();
+        }
+        for (int r = 0; r < 4; r += 2)
+            for (int c = 0; c < 2; ++c) {
+                nr[r + c] = mr[r] * pr[c] - mi[r] * pi[c] + mr[r + 1] * pr[2 + c] - mi[r + 1] * pi[2 + c];
+                ni[r + c] = mr[r] * pi[c] + mi[r] * pr[c] + mr[r + 1] * pi[2 + c] + mi[r + 1] * pr[2 + c];
+            }
+        for (int e = 0; e < 4; ++e) {
+            pr[e] = nr[e];
+            pi[e] = ni[e];
+        }
+    }
+    for (int e = 0; e < 4; ++e) P[e] = cd((double)pr[e], (double)pi[e]);
+}
+
 // Steps of a gate list in order.  `extra(i, step)` completes the step of gate i (gradients) and says
 // whether the gate may use a tile form.
 template <typename F>
@@ -266,14 +296,8 @@ void put_coefs(std::vector<C<R>> &out, const std::vector<const GateDesc *> &gs, 
     const GateDesc &g = *gs[s.mems[0]];
     switch (kind) {
     case S_RUN: case S_DIAGRUN: {
-        cd P[4] = {1, 0, 0, 1};
-        for (uint32_t i : s.mems) {
-            cd m[4], N[4];
-            one_bit_matrix(*gs[i], m);
-            for (int r = 0; r < 2; ++r)
-                for (int c = 0; c < 2; ++c) N[r * 2 + c] = m[r * 2] * P[c] + m[r * 2 + 1] * P[2 + c];
-            for (int e = 0; e < 4; ++e) P[e] = N[e];
-        }
+        cd P[4];
+        run_product<R>(gs, s.mems, P);
         if (kind == S_RUN) for (uint32_t e = 0; e < 4; ++e) put(e, P[e]);
         else for (uint32_t e = 0; e < 8; ++e) put(e, P[(e & 1) * 3]);
         break;

@@ -143,3 +143,35 @@ def test_qft_inverse_known_answer_large(capi, n, dtype):
     slack = 1e-12 if c128 else 1e-5
     assert np.all(lo - slack < u) and np.all(u <= hi + slack)
     sv.close()
+
+
+@pytest.mark.gpu
+def test_run_product_rounded_once(capi):
+    """A run of 999 rotations on one wire is applied as one matrix, their product rounded once: from |0> the
+    amplitudes are the extended-precision product's first column to half a unit in the last place (u = 1.1e-16
+    a component), and a batch's <X>, <Y>, <Z> of it, six roundings of values up to 1, to 1e-15.  A product
+    rounded after every gate misses by 5e-15."""
+    import math
+    import torch
+    from lightning_b200.batch import BatchedCircuits
+    rng = np.random.default_rng(12)
+    n, ops, col = 6, [], np.array([1, 0], dtype=np.clongdouble)
+    for i in range(999):
+        t = float(rng.uniform(0, 2 * np.pi))
+        c, s = math.cos(t / 2), math.sin(t / 2)
+        name = ("RX", "RY", "RZ")[i % 3]
+        ops.append((name, [0], False, [t]))
+        m = {"RX": [[c, -1j * s], [-1j * s, c]], "RY": [[c, -s], [s, c]],
+             "RZ": [[complex(c, -s), 0], [0, complex(c, s)]]}[name]
+        col = np.array(m, dtype=np.clongdouble) @ col
+    sv = capi.StateVector(n)
+    sv.apply_ops_fused(ops)
+    got = sv.download()[[0, 1 << (n - 1)]].astype(np.clongdouble)
+    for g, w in ((got.real, col.real), (got.imag, col.imag)):
+        assert (np.abs(g - w) <= 1.12e-16 * np.abs(w)).all()
+    eng = BatchedCircuits([{"num_qubits": n, "ops": ops, "param_index": [-1] * len(ops),
+                            "observables": [[(1.0, p, [0])] for p in "XYZ"]}], 0, dtype=np.complex128)
+    z = 2 * np.conj(col[0]) * col[1]
+    want = [z.real, z.imag, abs(col[0]) ** 2 - abs(col[1]) ** 2]
+    out = eng.forward(torch.empty(0, dtype=torch.float64, device="cuda")).cpu().numpy()
+    assert np.abs(out - np.array(want, dtype=np.longdouble)).max() < 1e-15
