@@ -146,19 +146,20 @@ std::string structure_key(const std::vector<HostOp> &ops, uint32_t n) {
     return k;
 }
 
+// Launches of one direction over the circuits `members` (a wave).
 template <typename R, bool REV>
-void make_launches(Batch &B, Program &T, const Builder &bd, const std::vector<Plan> &plans,
-                   const std::vector<uint32_t> &plan_of, std::vector<Job> &jobs, std::vector<GradRef> &refs,
-                   const std::vector<std::vector<int64_t>> &gslots, uint64_t &gpart) {
+void make_launches(Batch &B, Wave &W, const std::vector<uint32_t> &members, const Builder &bd,
+                   const std::vector<Plan> &plans, const std::vector<uint32_t> &plan_of, std::vector<Job> &jobs,
+                   std::vector<GradRef> &refs, const std::vector<std::vector<int64_t>> &gslots, uint64_t &gpart) {
     using G = TGeo<R, REV>;
     constexpr int dir = REV ? 1 : 0;
     size_t levels = 0;
-    for (const Plan &p : plans) levels = std::max(levels, p.dir[dir].segs.size());
+    for (uint32_t c : members) levels = std::max(levels, plans[plan_of[c]].dir[dir].segs.size());
     for (size_t l = 0; l < levels; ++l) {
         // tiles a job takes: eight jobs for every CTA the GPU holds, so that the last ones to finish
         // leave few SMs idle, and no more, since a job stages its segment's records once
         uint64_t tiles = 0;
-        for (uint32_t c = 0; c < B.ncirc; ++c) {
+        for (uint32_t c : members) {
             const PlanDir &D = plans[plan_of[c]].dir[dir];
             if (l < D.segs.size()) tiles += uint64_t(1) << std::max(0, (int)B.nq[c] - (int)bd.rec.segs[D.segs[l]].kt);
         }
@@ -171,7 +172,7 @@ void make_launches(Batch &B, Program &T, const Builder &bd, const std::vector<Pl
             uint64_t cost;
         };
         std::vector<Ref> list;
-        for (uint32_t c = 0; c < B.ncirc; ++c) {
+        for (uint32_t c : members) {
             const PlanDir &D = plans[plan_of[c]].dir[dir];
             if (l >= D.segs.size()) continue;
             const TSeg &s = bd.rec.segs[D.segs[l]];
@@ -212,7 +213,7 @@ void make_launches(Batch &B, Program &T, const Builder &bd, const std::vector<Pl
                 L.smem = std::max(L.smem, (uint32_t)list[i].smem);
                 ++L.njobs;
             }
-            T.launches[dir].push_back(L);
+            W.launches[dir].push_back(L);
         }
     }
 }
@@ -229,9 +230,34 @@ template <typename R> void build(Batch &B, Planned &P) {
     std::vector<uint64_t> mem_base(B.ncirc);
     std::vector<std::vector<int64_t>> gslots(B.ncirc);
     std::vector<uint32_t> sbegin[2], scount[2];
-    uint64_t pool = 0, ncoef[2] = {0, 0};
+    uint64_t ncoef[2] = {0, 0};
     uint32_t out_begin = 0;
     const int kt_old = B.dtype == B200SV_C64 ? 13 : 12;  // the widest gate a batch takes
+    // Places of the states.  k_batch holds states up to kt_old wires in shared memory, so a batch of any number
+    // of narrow circuits fits; here they share kNarrowPool bytes and take turns in waves where they need
+    // more (100 000 circuits of 12 qubits complex64 would take 3.3 GB in each pool).  Wider states, which
+    // k_batch keeps in memory too, have places of their own.
+    auto narrow = [&](uint32_t c) { return (int)B.nq[c] <= kt_old; };
+    auto place = [&](uint32_t c) { return std::max<uint64_t>(2, uint64_t(1) << B.nq[c]); };  // 16-byte aligned
+    constexpr uint64_t kShare = kNarrowPool / sizeof(C<R>);
+    uint64_t wide = 0, narrows = 0, pool = 0;
+    for (uint32_t c = 0; c < B.ncirc; ++c) (narrow(c) ? narrows : wide) += place(c);
+    std::vector<std::vector<uint32_t>> members(1);  // circuits of each wave
+    std::vector<uint64_t> off(B.ncirc);
+    for (bool turn : {false, true}) {  // the wide states, then the narrow ones
+        uint64_t at = turn ? wide : 0;
+        for (uint32_t c = 0; c < B.ncirc; ++c) {
+            if (narrow(c) != turn) continue;
+            if (turn && narrows > kShare && (at == wide || at + place(c) > wide + kShare)) {
+                if (!members.back().empty()) members.emplace_back();
+                at = wide;
+            }
+            off[c] = at;
+            at += place(c);
+            pool = std::max(pool, at);
+            members.back().push_back(c);
+        }
+    }
     for (uint32_t c = 0; c < B.ncirc; ++c) {
         const auto &ops = B.hops[c];
         const uint32_t n = B.nq[c];
@@ -250,8 +276,7 @@ template <typename R> void build(Batch &B, Planned &P) {
         plan_of[c] = it->second;
         TCirc &tc = circs[c];
         tc.n = n;
-        tc.off = pool;
-        pool += std::max<uint64_t>(2, uint64_t(1) << n);  // 16-byte aligned states
+        tc.off = off[c];
         tc.term_begin = (uint32_t)P.terms.size();
         for (auto t : B.hterms[c]) P.terms.push_back(t);
         tc.nterms = (uint32_t)B.hterms[c].size();
@@ -297,24 +322,29 @@ template <typename R> void build(Batch &B, Planned &P) {
     }
     std::vector<uint32_t> col(B.ncirc, 0);
     for (auto c : P.gslot_circ) P.gslot_col.push_back(col[c]++);
-    P.pool_a = P.pool_b = pool;
-    // jobs of every launch
+    P.pool_a = pool;
+    P.pool_b = P.gscale.empty() ? 0 : pool;  // bras
+    // jobs of every launch, and the chunks of the measurement kernels, wave by wave
     std::vector<Job> jobs;
     std::vector<GradRef> refs(P.gscale.size());
-    uint64_t gpart = 0;
-    make_launches<R, false>(B, T, bd, plans, plan_of, jobs, refs, gslots, gpart);
-    make_launches<R, true>(B, T, bd, plans, plan_of, jobs, refs, gslots, gpart);
-    // chunks of the measurement kernels
     std::vector<ChunkJob> chunks;
     std::vector<ObsRef> orefs;
-    uint64_t opart = 0;
-    for (uint32_t c = 0; c < B.ncirc; ++c) {
-        const uint32_t nch = B.nq[c] > (uint32_t)kChunkBits ? 1u << (B.nq[c] - kChunkBits) : 1u;
-        for (uint32_t k = 0; k < nch; ++k) chunks.push_back(ChunkJob{c, k, nch, 0, opart});
-        for (uint32_t o = 0; o < B.nobs[c]; ++o) orefs.push_back(ObsRef{opart, c, o, nch, 0});
-        opart += (uint64_t)circs[c].nterms * nch;
+    uint64_t gpart = 0, opart = 0;
+    for (const auto &list : members) {
+        Wave W;
+        W.kept = members.size() == 1 || !narrow(list[0]);
+        make_launches<R, false>(B, W, list, bd, plans, plan_of, jobs, refs, gslots, gpart);
+        make_launches<R, true>(B, W, list, bd, plans, plan_of, jobs, refs, gslots, gpart);
+        W.chunk0 = (uint32_t)chunks.size();
+        for (uint32_t c : list) {
+            const uint32_t nch = B.nq[c] > (uint32_t)kChunkBits ? 1u << (B.nq[c] - kChunkBits) : 1u;
+            for (uint32_t k = 0; k < nch; ++k) chunks.push_back(ChunkJob{c, k, nch, 0, opart});
+            for (uint32_t o = 0; o < B.nobs[c]; ++o) orefs.push_back(ObsRef{opart, c, o, nch, 0});
+            opart += (uint64_t)circs[c].nterms * nch;
+        }
+        W.nchunks = (uint32_t)chunks.size() - W.chunk0;
+        T.waves.push_back(std::move(W));
     }
-    T.nchunks = (uint32_t)chunks.size();
     upload(B, T.circs, circs);
     upload(B, T.segs, bd.rec.segs);
     upload(B, T.phases, bd.rec.phases);
@@ -368,7 +398,7 @@ template <typename R> void launch_coefs(Batch &B, int dir, cudaStream_t st) {
 
 // The levels of a direction: circuits of full tiles in order on the caller's stream, the narrower
 // classes (one level each, as a rule) beside them on the batch's side streams.
-template <typename R, bool REV> void launch_levels(Batch &B, const int *skip, cudaStream_t st) {
+template <typename R, bool REV> void launch_levels(Batch &B, const Wave &W, const int *skip, cudaStream_t st) {
     Program &T = *B.tp;
     TArgs a{};
     a.jobs = T.jobs;
@@ -381,7 +411,7 @@ template <typename R, bool REV> void launch_levels(Batch &B, const int *skip, cu
     a.pool_b = B.d_pool_b;
     a.gpart = T.gpart;
     a.skip = skip;
-    const auto &Ls = T.launches[REV ? 1 : 0];
+    const auto &Ls = W.launches[REV ? 1 : 0];
     if (Ls.empty()) return;
     std::vector<uint32_t> classes;
     for (const Launch &L : Ls)
@@ -408,27 +438,39 @@ template <typename R, bool REV> void launch_levels(Batch &B, const int *skip, cu
 template <typename R> void forward(Batch &B, double *out, cudaStream_t st) {
     Program &T = *B.tp;
     launch_coefs<R>(B, 0, st);
-    launch_levels<R, false>(B, nullptr, st);
+    for (const Wave &W : T.waves) {
+        launch_levels<R, false>(B, W, nullptr, st);
+        if (!B.total_obs) continue;
+        k_tile_expval<R><<<W.nchunks, kTThreads, chunk_smem<R>(), st>>>(T.chunks + W.chunk0, T.circs, B.d_terms,
+                                                                        B.d_pool_a, T.opart);
+        B200SV_CUDA(cudaGetLastError());
+        B.launched++;
+    }
     if (!B.total_obs) return;
-    k_tile_expval<R><<<T.nchunks, kTThreads, chunk_smem<R>(), st>>>(T.chunks, T.circs, B.d_terms, B.d_pool_a, T.opart);
     k_tile_outputs<<<(B.total_obs + 7) / 8, 256, 0, st>>>(T.orefs, B.total_obs, T.circs, B.d_terms, T.opart, out);
     B200SV_CUDA(cudaGetLastError());
-    B.launched += 2;
+    B.launched++;
 }
 
-// gradw[g] for the bra of dy, recomputing the states unless *reuse says pool A holds them
+// gradw[g] for the bra of dy, recomputing the states unless *reuse says pool A holds them (the places of a
+// wave that takes turns hold another wave's)
 template <typename R> void reverse(Batch &B, const double *dy, const int *reuse, cudaStream_t st) {
     Program &T = *B.tp;
-    launch_coefs<R>(B, 0, st);
-    launch_levels<R, false>(B, reuse, st);
     if (!B.ngslots) return;
+    launch_coefs<R>(B, 0, st);
     launch_coefs<R>(B, 1, st);
-    k_tile_bra<R><<<T.nchunks, kTThreads, chunk_smem<R>(), st>>>(T.chunks, T.circs, B.d_terms, B.d_pool_a, B.d_pool_b, dy);
-    launch_levels<R, true>(B, nullptr, st);
+    for (const Wave &W : T.waves) {
+        launch_levels<R, false>(B, W, W.kept ? reuse : nullptr, st);
+        k_tile_bra<R><<<W.nchunks, kTThreads, chunk_smem<R>(), st>>>(T.chunks + W.chunk0, T.circs, B.d_terms,
+                                                                     B.d_pool_a, B.d_pool_b, dy);
+        B200SV_CUDA(cudaGetLastError());
+        B.launched++;
+        launch_levels<R, true>(B, W, nullptr, st);
+    }
     k_tile_grads<<<std::max(1u, std::min(8192u, (B.ngslots + 15) / 16)), 128, 0, st>>>(T.grefs, T.h, T.gpart, B.ngslots,
                                                                                       B.d_gradw);
     B200SV_CUDA(cudaGetLastError());
-    B.launched += 2;
+    B.launched++;
 }
 
 }  // namespace tiles

@@ -532,6 +532,13 @@ __global__ void __launch_bounds__(kTThreads, 2) k_tile_bra(const ChunkJob *__res
 struct Launch {
     uint32_t first, njobs, threads, smem, level;
 };
+// Circuits whose states are in the pools together.
+struct Wave {
+    std::vector<Launch> launches[2];  // forward, reverse: level by level
+    uint32_t chunk0 = 0, nchunks = 0;
+    bool kept = true;                 // no other wave takes its places
+};
+constexpr uint64_t kNarrowPool = uint64_t(256) << 20;
 struct Program {
     TCirc *circs = nullptr;
     TSeg *segs = nullptr;
@@ -548,8 +555,8 @@ struct Program {
     GradRef *grefs = nullptr;
     ChunkJob *chunks = nullptr;
     ObsRef *orefs = nullptr;
-    uint32_t nchunks = 0, max_steps[2] = {};
-    std::vector<Launch> launches[2];  // forward, reverse: level by level
+    uint32_t max_steps[2] = {};
+    std::vector<Wave> waves;
 };
 
 }  // namespace tiles

@@ -575,3 +575,52 @@ def test_engines_alive_together(dtype, wide_gate):
         for _ in range(3):  # direct, recorded, replayed
             assert np.abs(eng.forward(p).cpu().numpy() - want).max() < (1e-12 if dtype == np.complex128 else 2e-5)
             assert np.abs(eng.vjp(p, dy).cpu().numpy() - gwant).max() < GRAD_TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+def test_many_narrow_circuits_take_turns(dtype):
+    """10 000 circuits of one shared-memory state's width, with a few wider and narrower ones: the pools hold a
+    share of them at a time (0.5 GiB; all at once would take 1.3 GB), and values, a VJP after a forward and a
+    VJP on its own are the oracle's for circuits of every turn.  A batch without trainable parameters holds
+    no bras."""
+    import torch
+    from lightning_b200.batch import BatchedCircuits
+    n, count = (13 if dtype == np.complex64 else 12), 10000
+    rng = np.random.default_rng(17)
+    circuits, at = [], 0
+    for c in range(count):
+        w = {3: n + 2, 4000: n + 1, 5000: 4, 9997: n + 2}.get(c, n)
+        a, b, d = (int(x) for x in rng.choice(w, 3, replace=False))
+        ops = [("RY", [a], False, []), ("CNOT", [a, b], False, []), ("RX", [b], False, []), ("CRZ", [b, d], False, []),
+               ("Hadamard", [d], False, []), ("RY", [d], False, [])]
+        circuits.append({"num_qubits": w, "ops": ops, "param_index": [at, -1, at + 1, at + 2, -1, at + 3],
+                         "observables": [[(1.0, "Z", [a]), (0.5, "XY", [b, d])]]})
+        at += 4
+    params = rng.uniform(0, 2 * np.pi, at)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    eng = BatchedCircuits(circuits, at, dtype=dtype)
+    assert free - torch.cuda.mem_get_info()[0] < 0.8e9
+    p, dy = torch.tensor(params, device="cuda"), rng.normal(size=count)
+    dyt = torch.tensor(dy, device="cuda")
+    which = [0, 1, 3, 2047, 4000, 4099, 5000, 7777, 9997, 9999]
+    some = [circuits[c] for c in which]
+    want, gwant = oracle_outputs(some, params), oracle_vjp(some, params, dy[which])
+    slots = np.concatenate([np.arange(4 * c, 4 * c + 4) for c in which])
+    for _ in range(3):  # direct, recorded, replayed
+        out = eng.forward(p).cpu().numpy()
+        grads = [eng.vjp(p, dyt).cpu().numpy() for _ in range(2)]  # after the forward, and on its own
+        assert np.abs(out[which] - want).max() < (1e-12 if dtype == np.complex128 else 2e-5)
+        assert np.array_equal(grads[0], grads[1])
+        assert np.abs(grads[0][slots] - gwant[slots]).max() < GRAD_TOL[dtype]
+    jac = eng.jacobian(p).cpu().numpy()
+    assert np.abs(jac[slots] * np.repeat(dy[which], 4) - gwant[slots]).max() < GRAD_TOL[dtype]
+    eng.close()
+    fixed = [dict(c, param_index=[-1] * 6, ops=[(o[0], o[1], False, [0.3] if o[0] in ("RY", "RX", "CRZ") else [])
+                                                for o in c["ops"]]) for c in circuits]
+    free = torch.cuda.mem_get_info()[0]
+    eng = BatchedCircuits(fixed, 0, dtype=dtype)
+    assert free - torch.cuda.mem_get_info()[0] < 0.4e9
+    out = eng.forward(torch.empty(0, dtype=torch.float64, device="cuda")).cpu().numpy()
+    want = oracle_outputs([fixed[c] for c in which], params)
+    assert np.abs(out[which] - want).max() < (1e-12 if dtype == np.complex128 else 2e-5)
