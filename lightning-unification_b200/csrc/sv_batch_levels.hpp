@@ -112,7 +112,7 @@ template <typename R, bool REV> void plan_dir(Builder &B, Plan &P, uint32_t n, i
         CoefStep c{};
         c.kind = kind;
         c.mem_begin = (uint32_t)B.mem_list.size();
-        c.nmem = (uint16_t)s.mems.size();
+        c.nmem = (uint32_t)s.mems.size();
         c.coef = at;
         c.nt = (uint8_t)s.tgt.size();
         c.nbits = (uint8_t)(s.tgt.size() + s.ctl.size());

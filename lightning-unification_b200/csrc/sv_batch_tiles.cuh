@@ -37,8 +37,8 @@ struct Mem {
 
 // How a step's coefficients are formed: members in op order, index into the plan's member list.
 struct CoefStep {
-    uint32_t mem_begin, coef;  // coef: position in the circuit's coefficient array of this direction
-    uint16_t nmem;
+    uint32_t mem_begin, nmem;  // a run has any number of members
+    uint32_t coef;             // position in the circuit's coefficient array of this direction
     uint8_t kind, nt, nbits;   // S_DIAG: target count, index bits
     uint8_t src[3];            // S_DIAG: index bit (2 - j) of the table is the gate's bit src[j] (255: none)
 };
@@ -213,7 +213,7 @@ template <typename R> __global__ void k_tile_coefs(CoefArgs a) {
                 const double2 zero = make_double2(0, 0), one = make_double2(1, 0);
                 Mat2 run{{one, zero, zero, one}, {zero, zero, zero, zero}};
                 double2(&P)[4] = run.h;
-                for (int k = 0; k < st.nmem; ++k) {
+                for (uint32_t k = 0; k < st.nmem; ++k) {
                     const Mem &m = mems[list[rev ? st.nmem - 1 - k : k]];
                     if (rev && m.gslot >= 0) a.h[m.gslot] = gen_row(gen_code(m.gate), P);
                     Mat2 q{{}, {zero, zero, zero, zero}};

@@ -624,3 +624,24 @@ def test_many_narrow_circuits_take_turns(dtype):
     out = eng.forward(torch.empty(0, dtype=torch.float64, device="cuda")).cpu().numpy()
     want = oracle_outputs([fixed[c] for c in which], params)
     assert np.abs(out[which] - want).max() < (1e-12 if dtype == np.complex128 else 2e-5)
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+def test_run_of_more_gates_than_a_16_bit_count(dtype):
+    """66 000 gates on one wire, one run: values and the gradients of its first and last gate."""
+    import torch
+    from lightning_b200.batch import BatchedCircuits
+    rng = np.random.default_rng(2)
+    kinds = ("RX", "RY", "RZ")
+    ops = [(kinds[i % 3], [1], False, [float(rng.uniform(0, 2 * np.pi))]) for i in range(66000)]
+    ops = [("RY", [1], False, [])] + ops + [("RX", [1], False, []), ("CNOT", [1, 0], False, [])]
+    c = {"num_qubits": 3, "ops": ops, "param_index": [0] + [-1] * 66000 + [1, -1],
+         "observables": [[(1.0, "Z", [0]), (0.5, "Y", [1])]]}
+    params = np.array([0.4, 1.9])
+    eng = BatchedCircuits([c], 2, dtype=dtype)
+    p = torch.tensor(params, device="cuda")
+    assert abs(eng.forward(p).item() - oracle_outputs([c], params)[0]) < (1e-11 if dtype == np.complex128 else 2e-5)
+    g = eng.vjp(p, torch.ones(1, dtype=torch.float64, device="cuda")).cpu().numpy()
+    # shift rule: exact for one rotation
+    want = [(oracle_outputs([c], params + s)[0] - oracle_outputs([c], params - s)[0]) / 2 for s in np.pi / 2 * np.eye(2)]
+    assert np.abs(g - want).max() < (1e-11 if dtype == np.complex128 else 2e-5)
