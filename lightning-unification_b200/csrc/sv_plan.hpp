@@ -23,6 +23,8 @@ enum SKind : uint8_t {
     S_PAIR4 = 8,    // excitation block on four bits
 };
 
+constexpr int kLookAhead = 4096;  // steps a segment leaves out before it is closed
+
 // A step of a circuit.  Two steps commute when every bit they share is diagonal in both (flip).
 struct Step {
     SKind kind = S_NONE;
@@ -101,7 +103,7 @@ std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector
             continue;
         }
         uint64_t used = 0, any = 0, flipped = 0;  // any, flipped: of the steps left out
-        int nops = 0, ncf = 0, ngr = 0;
+        int nops = 0, ncf = 0, ngr = 0, skipped = 0;
         std::vector<uint32_t> take;
         for (size_t j = first; j < ns; ++j) {
             if (done[j]) continue;
@@ -120,7 +122,9 @@ std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector
             } else {
                 any |= s.mask;
                 flipped |= s.flip;
-                if (flipped == every) break;  // everything later is blocked
+                // everything later is blocked, or far away: where some bits are never touched (or all steps
+                // commute) the look-ahead would read the whole list for every segment
+                if (flipped == every || ++skipped == kLookAhead) break;
             }
         }
         if (take.empty() && left > 0) throw Unsupported("gate wider than the tile");

@@ -358,3 +358,23 @@ def test_captured_lists_replay_after_the_call(capi, n, dtype):
         del junk
         want = O.run_circuit(n, ops, state=want)
         assert np.abs(sv.download() - want).max() < (1e-12 if dtype == np.complex128 else 2e-5)
+
+
+def test_long_lists_plan_in_linear_time(capi):
+    """A list on a few wires of a wider state: eight times the gates take about eight times as long (a planner that
+    looks through the rest of the list for every segment took 30 times as long)."""
+    import time
+    n, took = 14, []
+    for count in (50000, 400000):
+        ops = [(("CRX", "CRY", "CRZ")[i % 3], [(i * 7) % 3, (i * 7 + 1 + i % 2) % 3], False, [0.1]) for i in range(count)]
+        ol = capi.OpList(ops, np.complex128)
+        sv = capi.StateVector(n)
+        best = np.inf
+        for _ in range(2):
+            t = time.perf_counter()
+            sv.apply_ops_fused(ol)
+            sv.synchronize()
+            best = min(best, time.perf_counter() - t)
+        took.append(best)
+        assert abs(sv.norm2() - 1.0) < count * 1e-15
+    assert took[1] < 16 * took[0]
