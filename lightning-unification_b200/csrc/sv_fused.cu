@@ -28,6 +28,9 @@ namespace {
 using namespace steps;
 
 constexpr int kMaxStateCoefs = 1024;
+// Partial sums of a sweep's gradients (64 MiB; a step has four per CTA and bra, 38 KB on a wide state): they are
+// reduced when the next segment's would not fit, so the workspace does not grow with the parameters.
+constexpr uint64_t kMaxGradSums = uint64_t(8) << 20;
 
 struct StateArgs {
     const TSeg *seg;
@@ -528,9 +531,19 @@ void run_fused_adjoint(void *&lam, void *&lam2, const std::vector<void *> &bras,
     // gradient items: members in sweep order, each seen through the inverses before it in its run
     std::vector<GradItem> grads;
     std::vector<uint64_t> gbase(rec.segs.size(), 0);
-    uint64_t ngpart = 0;
+    std::vector<size_t> flush(rec.segs.size(), 0);  // items whose sums are formed after the segment
+    uint64_t ngpart = 0, most_gpart = 0;
+    size_t flushed = 0;
+    int last = -1;
     for (const Piece &p : pieces) {
         if (p.seg < 0) continue;
+        const uint64_t size = (uint64_t)p.grads.size() * 4 * grid * nobs;
+        if (ngpart > 0 && ngpart + size > kMaxGradSums) {
+            flush[last] = grads.size() - flushed;
+            flushed = grads.size();
+            ngpart = 0;
+        }
+        last = p.seg;
         gbase[p.seg] = ngpart;
         for (size_t row = 0; row < p.grads.size(); ++row) {
             Step s = all[p.grads[row]];
@@ -558,8 +571,10 @@ void run_fused_adjoint(void *&lam, void *&lam2, const std::vector<void *> &bras,
                 }
             }
         }
-        ngpart += (uint64_t)p.grads.size() * 4 * grid * nobs;
+        ngpart += size;
+        most_gpart = std::max(most_gpart, ngpart);
     }
+    if (last >= 0) flush[last] = grads.size() - flushed;
     double *gpart = nullptr;
     struct Free {
         double *&p;
@@ -574,8 +589,9 @@ void run_fused_adjoint(void *&lam, void *&lam2, const std::vector<void *> &bras,
     if (!rec.segs.empty()) {
         allow_smem<R, true>();
         blob.upload();
-        B200SV_CUDA(cudaMallocAsync((void **)&gpart, std::max<uint64_t>(1, ngpart) * sizeof(double), st));
+        B200SV_CUDA(cudaMallocAsync((void **)&gpart, std::max<uint64_t>(1, most_gpart) * sizeof(double), st));
     }
+    size_t done = 0;  // items whose sums are formed
     for (const Piece &p : pieces) {
         if (p.seg < 0) {
             exec_single(all[p.step].mems[0]);
@@ -595,10 +611,11 @@ void run_fused_adjoint(void *&lam, void *&lam2, const std::vector<void *> &bras,
             static_cast<const C<R> *>(lam), out, blob.at<C<R> *>(o_br), a);
         B200SV_CUDA(cudaGetLastError());
         if (nobs > 1) std::swap(lam, lam2);
-    }
-    if (!grads.empty()) {
-        k_state_grads<<<dim3((unsigned)grads.size(), nobs), 128, 0, st>>>(blob.at<GradItem>(o_gr), gpart, (int)grid, d_jac);
-        B200SV_CUDA(cudaGetLastError());
+        if (const size_t n = flush[p.seg]) {
+            k_state_grads<<<dim3((unsigned)n, nobs), 128, 0, st>>>(blob.at<GradItem>(o_gr) + done, gpart, (int)grid, d_jac);
+            B200SV_CUDA(cudaGetLastError());
+            done += n;
+        }
     }
 }
 

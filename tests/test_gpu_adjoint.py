@@ -330,3 +330,40 @@ def test_complex64_generator_products_in_fp64(capi, n, nobs):
                 got = sv.adjoint_jacobian(ops, o, tp)
                 want = O.adjoint_jacobian(psi.astype(np.complex128), ops, o, tp)
                 assert np.abs(got - want).max() < 1e-13, (q, ops)
+
+
+def test_gradient_workspace_does_not_grow_with_the_parameters(capi):
+    """20 000 parameters on 20 qubits: the sweep's work memory stays below 200 MB (one partial sum per step and
+    CTA for all of them would take 330), and parameters from all over the list have the shift rule's values,
+    with one and with two observables."""
+    import ctypes
+    rt = ctypes.CDLL("libcudart.so.12")
+    pool, high = ctypes.c_void_p(), ctypes.c_uint64(0)
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    n, count = 20, 20000
+    rng = np.random.default_rng(8)
+    angles = rng.uniform(0, 2 * np.pi, count)
+
+    def circuit(a):
+        return [op for i in range(count) for op in ((("RX", "RY")[i % 2], [i % 6], False, [float(a[i])]),
+                                                    ("CNOT", [i % 6, (i + 1) % 6], False, []))]
+    obs = [[(1.0, [("PauliZ", [2])]), (0.5, [("PauliX", [4])])], [(1.0, [("PauliZ", [0]), ("PauliZ", [1])])]]
+
+    def values(a):
+        sv = capi.StateVector(n)
+        sv.apply_ops_fused(circuit(a))
+        return np.array([sv.expval(o) for o in obs])
+    sv = capi.StateVector(n)
+    ops = circuit(angles)
+    sv.apply_ops_fused(ops)
+    used_high = 8  # cudaMemPoolAttrUsedMemHigh
+    for o in (obs[:1], obs):
+        assert rt.cudaMemPoolSetAttribute(pool, used_high, ctypes.byref(ctypes.c_uint64(0))) == 0
+        jac = sv.adjoint_jacobian(ops, o, list(range(count)))
+        assert rt.cudaMemPoolGetAttribute(pool, used_high, ctypes.byref(high)) == 0
+        assert 0 < high.value < 200e6
+    for k in (0, 1, 63, 64, 5000, 12345, 19999):
+        shift = np.zeros(count)
+        shift[k] = np.pi / 2
+        want = (values(angles + shift) - values(angles - shift)) / 2
+        assert np.abs(jac[:, k] - want).max() < 1e-10  # 40 000 gates of about 1e-16 each way
