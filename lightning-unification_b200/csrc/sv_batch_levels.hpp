@@ -146,11 +146,16 @@ std::string structure_key(const std::vector<HostOp> &ops, uint32_t n) {
     return k;
 }
 
+// Partial sums of the gradients given out so far: of one group, reduced together (k_tile_grads).
+struct GradSums {
+    uint64_t used = 0, most = 0;
+    uint32_t group = 0;
+};
 // Launches of one direction over the circuits `members` (a wave).
 template <typename R, bool REV>
 void make_launches(Batch &B, Wave &W, const std::vector<uint32_t> &members, const Builder &bd,
                    const std::vector<Plan> &plans, const std::vector<uint32_t> &plan_of, std::vector<Job> &jobs,
-                   std::vector<GradRef> &refs, const std::vector<std::vector<int64_t>> &gslots, uint64_t &gpart) {
+                   std::vector<GradRef> &refs, const std::vector<std::vector<int64_t>> &gslots, GradSums &sums) {
     using G = TGeo<R, REV>;
     constexpr int dir = REV ? 1 : 0;
     size_t levels = 0;
@@ -165,6 +170,25 @@ void make_launches(Batch &B, Wave &W, const std::vector<uint32_t> &members, cons
         }
         uint64_t per = 1;
         while (per * 2 * 8 * (uint64_t)(sm_count() * G::minb) <= tiles) per *= 2;
+        auto parts = [&](uint32_t c, const TSeg &s) {
+            return ((uint64_t(1) << std::max(0, (int)B.nq[c] - (int)s.kt)) + per - 1) / per;
+        };
+        if (REV) {
+            uint64_t need = 0;
+            for (uint32_t c : members) {
+                const PlanDir &D = plans[plan_of[c]].dir[dir];
+                if (l >= D.segs.size()) continue;
+                const TSeg &s = bd.rec.segs[D.segs[l]];
+                need += (uint64_t)s.ngrad * 4 * parts(c, s);
+            }
+            const bool full = sums.used > 0 && sums.used + need > kMaxGradSums;
+            if (full) {
+                sums.used = 0;
+                ++sums.group;
+            }
+            if (l == 0 || full) W.spans.push_back(Span{(uint32_t)l, full});
+            sums.most = std::max(sums.most, sums.used + need);
+        }
         struct Ref {
             Job j;
             uint32_t threads;
@@ -177,7 +201,7 @@ void make_launches(Batch &B, Wave &W, const std::vector<uint32_t> &members, cons
             if (l >= D.segs.size()) continue;
             const TSeg &s = bd.rec.segs[D.segs[l]];
             const uint64_t nt = uint64_t(1) << std::max(0, (int)B.nq[c] - (int)s.kt);
-            const uint64_t nparts = (nt + per - 1) / per;
+            const uint64_t nparts = parts(c, s);
             for (uint64_t p = 0; p < nparts; ++p) {
                 Ref r{};
                 r.j.seg = D.segs[l];
@@ -187,7 +211,7 @@ void make_launches(Batch &B, Wave &W, const std::vector<uint32_t> &members, cons
                 r.j.nparts = (uint32_t)nparts;
                 r.j.part = (uint32_t)p;
                 r.j.flags = (!REV && l == 0 ? 1u : 0u) | (REV && l + 1 == D.segs.size() ? 2u : 0u);
-                r.j.gpart = gpart;
+                r.j.gpart = sums.used;
                 r.threads = 1u << (s.kt - G::a);
                 r.smem = seg_smem<R, REV>(s);
                 r.cost = (uint64_t)r.j.ntiles * (s.nops + 2 * s.nph + 1);
@@ -198,8 +222,8 @@ void make_launches(Batch &B, Wave &W, const std::vector<uint32_t> &members, cons
                 for (size_t k = 0; k < rows.size(); ++k)
                     for (uint32_t m : plans[plan_of[c]].steps[rows[k]].mems)
                         if (gslots[c][m] >= 0)
-                            refs[gslots[c][m]] = GradRef{gpart + (uint64_t)k * 4 * nparts, (uint32_t)nparts, 0};
-                gpart += (uint64_t)s.ngrad * 4 * nparts;
+                            refs[gslots[c][m]] = GradRef{sums.used + (uint64_t)k * 4 * nparts, (uint32_t)nparts, sums.group};
+                sums.used += (uint64_t)s.ngrad * 4 * nparts;
             }
         }
         std::stable_sort(list.begin(), list.end(), [](const Ref &a, const Ref &b) {
@@ -329,12 +353,13 @@ template <typename R> void build(Batch &B, Planned &P) {
     std::vector<GradRef> refs(P.gscale.size());
     std::vector<ChunkJob> chunks;
     std::vector<ObsRef> orefs;
-    uint64_t gpart = 0, opart = 0;
+    GradSums sums;
+    uint64_t opart = 0;
     for (const auto &list : members) {
         Wave W;
         W.kept = members.size() == 1 || !narrow(list[0]);
-        make_launches<R, false>(B, W, list, bd, plans, plan_of, jobs, refs, gslots, gpart);
-        make_launches<R, true>(B, W, list, bd, plans, plan_of, jobs, refs, gslots, gpart);
+        make_launches<R, false>(B, W, list, bd, plans, plan_of, jobs, refs, gslots, sums);
+        make_launches<R, true>(B, W, list, bd, plans, plan_of, jobs, refs, gslots, sums);
         W.chunk0 = (uint32_t)chunks.size();
         for (uint32_t c : list) {
             const uint32_t nch = B.nq[c] > (uint32_t)kChunkBits ? 1u << (B.nq[c] - kChunkBits) : 1u;
@@ -363,7 +388,7 @@ template <typename R> void build(Batch &B, Planned &P) {
     upload(B, T.chunks, chunks);
     upload(B, T.orefs, orefs);
     T.h = B.dalloc<double4>(P.gscale.size());
-    T.gpart = B.dalloc<double>(gpart);
+    T.gpart = B.dalloc<double>(sums.most);
     T.opart = B.dalloc<double>(opart);
     for (const void *m : {(const void *)k_tile_expval<R>, (const void *)k_tile_bra<R>})
         B200SV_CUDA(cudaFuncSetAttribute(m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem<R>()));
@@ -396,9 +421,10 @@ template <typename R> void launch_coefs(Batch &B, int dir, cudaStream_t st) {
     B.launched++;
 }
 
-// The levels of a direction: circuits of full tiles in order on the caller's stream, the narrower
+// Levels [l0, l1) of a direction: circuits of full tiles in order on the caller's stream, the narrower
 // classes (one level each, as a rule) beside them on the batch's side streams.
-template <typename R, bool REV> void launch_levels(Batch &B, const Wave &W, const int *skip, cudaStream_t st) {
+template <typename R, bool REV>
+void launch_levels(Batch &B, const Wave &W, uint32_t l0, uint32_t l1, const int *skip, cudaStream_t st) {
     Program &T = *B.tp;
     TArgs a{};
     a.jobs = T.jobs;
@@ -412,16 +438,17 @@ template <typename R, bool REV> void launch_levels(Batch &B, const Wave &W, cons
     a.gpart = T.gpart;
     a.skip = skip;
     const auto &Ls = W.launches[REV ? 1 : 0];
-    if (Ls.empty()) return;
+    auto now = [&](const Launch &L) { return L.level >= l0 && L.level < l1; };
     std::vector<uint32_t> classes;
     for (const Launch &L : Ls)
-        if (std::find(classes.begin(), classes.end(), L.threads) == classes.end()) classes.push_back(L.threads);
+        if (now(L) && std::find(classes.begin(), classes.end(), L.threads) == classes.end())
+            classes.push_back(L.threads);
     if (classes.size() > 1) B200SV_CUDA(cudaEventRecord(B.fork, st));
     for (size_t k = 0; k < classes.size(); ++k) {
         const cudaStream_t s = k == 0 ? st : B.side[k - 1];
         if (k > 0) B200SV_CUDA(cudaStreamWaitEvent(s, B.fork, 0));
         for (const Launch &L : Ls) {
-            if (L.threads != classes[k]) continue;
+            if (!now(L) || L.threads != classes[k]) continue;
             TArgs x = a;
             x.jobs = a.jobs + L.first;
             k_tiles<R, REV><<<L.njobs, L.threads, L.smem, s>>>(x);
@@ -439,7 +466,7 @@ template <typename R> void forward(Batch &B, double *out, cudaStream_t st) {
     Program &T = *B.tp;
     launch_coefs<R>(B, 0, st);
     for (const Wave &W : T.waves) {
-        launch_levels<R, false>(B, W, nullptr, st);
+        launch_levels<R, false>(B, W, 0, ~0u, nullptr, st);
         if (!B.total_obs) continue;
         k_tile_expval<R><<<W.nchunks, kTThreads, chunk_smem<R>(), st>>>(T.chunks + W.chunk0, T.circs, B.d_terms,
                                                                         B.d_pool_a, T.opart);
@@ -457,20 +484,28 @@ template <typename R> void forward(Batch &B, double *out, cudaStream_t st) {
 template <typename R> void reverse(Batch &B, const double *dy, const int *reuse, cudaStream_t st) {
     Program &T = *B.tp;
     if (!B.ngslots) return;
+    uint32_t group = 0;
+    auto grads = [&] {
+        k_tile_grads<<<std::max(1u, std::min(8192u, (B.ngslots + 15) / 16)), 128, 0, st>>>(T.grefs, T.h, T.gpart, B.ngslots,
+                                                                                          group++, B.d_gradw);
+        B200SV_CUDA(cudaGetLastError());
+        B.launched++;
+    };
     launch_coefs<R>(B, 0, st);
     launch_coefs<R>(B, 1, st);
     for (const Wave &W : T.waves) {
-        launch_levels<R, false>(B, W, W.kept ? reuse : nullptr, st);
+        launch_levels<R, false>(B, W, 0, ~0u, W.kept ? reuse : nullptr, st);
         k_tile_bra<R><<<W.nchunks, kTThreads, chunk_smem<R>(), st>>>(T.chunks + W.chunk0, T.circs, B.d_terms,
                                                                      B.d_pool_a, B.d_pool_b, dy);
         B200SV_CUDA(cudaGetLastError());
         B.launched++;
-        launch_levels<R, true>(B, W, nullptr, st);
+        for (size_t i = 0; i < W.spans.size(); ++i) {
+            if (W.spans[i].reduce) grads();
+            const uint32_t end = i + 1 < W.spans.size() ? W.spans[i + 1].level : ~0u;
+            launch_levels<R, true>(B, W, W.spans[i].level, end, nullptr, st);
+        }
     }
-    k_tile_grads<<<std::max(1u, std::min(8192u, (B.ngslots + 15) / 16)), 128, 0, st>>>(T.grefs, T.h, T.gpart, B.ngslots,
-                                                                                      B.d_gradw);
-    B200SV_CUDA(cudaGetLastError());
-    B.launched++;
+    grads();
 }
 
 }  // namespace tiles

@@ -267,19 +267,21 @@ template <typename R> __global__ void k_tile_coefs(CoefArgs a) {
     }
 }
 
-// gradw[g] = h_g . (sums of its step over the segment's parts); eight lanes a gradient, fixed order
+// gradw[g] = h_g . (sums of its step over the segment's parts) for the gradients of a group; eight lanes a
+// gradient, fixed order
 struct GradRef {
     uint64_t base;
-    uint32_t nparts, pad;
+    uint32_t nparts, group;
 };
 __global__ void k_tile_grads(const GradRef *__restrict__ refs, const double4 *__restrict__ h,
-                             const double *__restrict__ gpart, uint32_t n, double *__restrict__ gradw) {
+                             const double *__restrict__ gpart, uint32_t n, uint32_t group, double *__restrict__ gradw) {
     const uint32_t sub = threadIdx.x & 7;
     for (uint32_t g0 = blockIdx.x * (blockDim.x >> 3); g0 < n; g0 += gridDim.x * (blockDim.x >> 3)) {
         const uint32_t g = g0 + (threadIdx.x >> 3);
         double s = 0.0;
-        if (g < n) {
-            const GradRef r = refs[g];
+        const GradRef r = g < n ? refs[g] : GradRef{0, 0, ~0u};
+        const bool mine = g < n && r.group == group;
+        if (mine) {
             const double4 q = h[g];
             const double hv[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -291,7 +293,7 @@ __global__ void k_tile_grads(const GradRef *__restrict__ refs, const double4 *__
         }
 #pragma unroll
         for (int off = 4; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        if (g < n && sub == 0) gradw[g] = s;
+        if (mine && sub == 0) gradw[g] = s;
     }
 }
 
@@ -532,13 +534,20 @@ __global__ void __launch_bounds__(kTThreads, 2) k_tile_bra(const ChunkJob *__res
 struct Launch {
     uint32_t first, njobs, threads, smem, level;
 };
+// Reverse levels from `level` on; reduce: the gradients' partial sums are reduced first, their place is needed.
+struct Span {
+    uint32_t level;
+    bool reduce;
+};
 // Circuits whose states are in the pools together.
 struct Wave {
     std::vector<Launch> launches[2];  // forward, reverse: level by level
+    std::vector<Span> spans;
     uint32_t chunk0 = 0, nchunks = 0;
     bool kept = true;                 // no other wave takes its places
 };
 constexpr uint64_t kNarrowPool = uint64_t(256) << 20;
+constexpr uint64_t kMaxGradSums = uint64_t(32) << 20;  // 256 MiB
 struct Program {
     TCirc *circs = nullptr;
     TSeg *segs = nullptr;

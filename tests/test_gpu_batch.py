@@ -645,3 +645,39 @@ def test_run_of_more_gates_than_a_16_bit_count(dtype):
     # shift rule: exact for one rotation
     want = [(oracle_outputs([c], params + s)[0] - oracle_outputs([c], params - s)[0]) / 2 for s in np.pi / 2 * np.eye(2)]
     assert np.abs(g - want).max() < (1e-11 if dtype == np.complex128 else 2e-5)
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+def test_gradient_sums_of_deep_circuits_take_turns(dtype):
+    """Ten circuits of 20 (complex64: 21) qubits and 100 levels of 64 gradients, with narrower ones beside them:
+    the partial sums (0.5 GB for all levels) are reduced as they fill 256 MiB, and gradients from all over the
+    circuits have the shift rule's values, after a forward, alone and replayed."""
+    import torch
+    from lightning_b200.batch import BatchedCircuits
+    rng = np.random.default_rng(23)
+    circuits, at, first = [], 0, []
+    wide = 21 if dtype == np.complex64 else 20
+    for n, count in [(wide, 6400)] * 10 + [(12, 500), (14, 300), (8, 700)]:
+        ops = [op for i in range(count) for op in ((("RX", "RY")[i % 2], [i % 6], False, []),
+                                                   ("CNOT", [i % 6, (i + 1) % 6], False, []))]
+        circuits.append({"num_qubits": n, "ops": ops, "param_index": [v for i in range(count) for v in (at + i, -1)],
+                         "observables": [[(1.0, "Z", [2]), (0.5, "X", [4])]]})
+        first.append((at, count))
+        at += count
+    params = rng.uniform(0, 2 * np.pi, at)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    eng = BatchedCircuits(circuits, at, dtype=dtype)
+    amp = 16 if dtype == np.complex128 else 8
+    assert free - torch.cuda.mem_get_info()[0] < 2 * amp * (10 << wide) + 0.4e9
+    p, dy = torch.tensor(params, device="cuda"), torch.ones(len(circuits), dtype=torch.float64, device="cuda")
+    eng.forward(p)
+    grads = [eng.vjp(p, dy).cpu().numpy() for _ in range(3)]  # after a forward; recorded; replayed
+    assert np.array_equal(grads[0], grads[1]) and np.array_equal(grads[0], grads[2])
+    tol = 1e-10 if dtype == np.complex128 else 2e-4  # 12 800 gates of about 1e-16 (6e-8) each way
+    for where in (0.0, 0.01, 0.31, 0.5, 0.77, 0.999):  # one parameter of every circuit at a time
+        k = np.array([a + int(where * c) for a, c in first])
+        shift = np.zeros(at)
+        shift[k] = np.pi / 2
+        up, down = (eng.forward(torch.tensor(params + s, device="cuda")).cpu().numpy() for s in (shift, -shift))
+        assert np.abs(grads[0][k] - (up - down) / 2).max() < tol
