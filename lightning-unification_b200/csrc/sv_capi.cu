@@ -1238,15 +1238,18 @@ int b200sv_adjoint_jacobian(b200sv_handle psi, const b200sv_op *ops, uint32_t no
         }
         std::vector<void *> lambda_and_bras{lambda};
         lambda_and_bras.insert(lambda_and_bras.end(), bras.begin(), bras.end());
-        // several bras: a second lambda for the fused passes (the observables' work state where
-        // there was one); without the memory for it the steps run one by one
-        void *lambda2 = tmp;
-        if (nobs > 1 && !lambda2) {
-            if (cudaMallocAsync(&lambda2, h->state_bytes(), st) == cudaSuccess) {
-                bufs.push_back(lambda2);
-            } else {
-                cudaGetLastError();
-                lambda2 = nullptr;
+        // a second lambda where several bras share launches (the observables' work state where there was one);
+        // without the memory for it the bras take turns
+        void *lambda2 = nullptr;
+        if (fused_adjoint_together(h->dtype, h->nq, nobs)) {
+            lambda2 = tmp;
+            if (!lambda2) {
+                if (cudaMallocAsync(&lambda2, h->state_bytes(), st) == cudaSuccess) {
+                    bufs.push_back(lambda2);
+                } else {
+                    cudaGetLastError();
+                    lambda2 = nullptr;
+                }
             }
         }
         // one step: the products (one-wire gates: products and inverse in one pass over the pairs)
@@ -1279,11 +1282,7 @@ int b200sv_adjoint_jacobian(b200sv_handle psi, const b200sv_op *ops, uint32_t no
             lambda_and_bras[0] = lambda;
             apply_desc_multi(h, lambda_and_bras, it.adj);  // lambda and every bra in one launch
         };
-        if (nobs == 1 || (nobs > 1 && nobs <= 65535 && lambda2)) {
-            apply_fused_adjoint(lambda, lambda2, bras, h->nq, h->dtype, items, exec_single, d_jac, st);
-        } else {
-            for (size_t i = 0; i < items.size(); ++i) exec_single(i);
-        }
+        if (nobs) apply_fused_adjoint(lambda, lambda2, bras, h->nq, h->dtype, items, exec_single, d_jac, st);
         std::vector<double> jt((size_t)ntp * nobs);
         if (!jt.empty())
             B200SV_CUDA(cudaMemcpyAsync(jt.data(), d_jac, jt.size() * sizeof(double), cudaMemcpyDeviceToHost, st));

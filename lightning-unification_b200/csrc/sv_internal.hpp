@@ -147,7 +147,9 @@ struct AdjItem {
 };
 // The sweep over lambda and the bras in fused passes; items without a register form run
 // through exec_single(i) in order, on `lambda`.  Products land in d_jac[col * bras + bra].  With
-// several bras lambda moves between `lambda` and `lambda2` (swapped); one bra needs no lambda2.
+// several bras and a lambda2 (fused_adjoint_together), lambda moves between `lambda` and `lambda2` (swapped);
+// without one every bra has launches of its own.
+bool fused_adjoint_together(int dtype, uint32_t nq, uint32_t nobs);
 void apply_fused_adjoint(void *&lambda, void *&lambda2, const std::vector<void *> &bras, uint32_t nq, int dtype,
                          const std::vector<AdjItem> &items, const std::function<void(size_t)> &exec_single,
                          double *d_jac, cudaStream_t st);

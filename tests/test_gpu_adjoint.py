@@ -367,3 +367,38 @@ def test_gradient_workspace_does_not_grow_with_the_parameters(capi):
         shift[k] = np.pi / 2
         want = (values(angles + shift) - values(angles - shift)) / 2
         assert np.abs(jac[:, k] - want).max() < 1e-10  # 40 000 gates of about 1e-16 each way
+
+
+@pytest.mark.parametrize("n,dtype", [(22, np.complex128), (24, np.complex128), (23, np.complex64), (25, np.complex64)])
+def test_several_observables_on_wide_states(capi, n, dtype):
+    """Three observables where their sweeps share launches (22 qubits complex128, 23 complex64) and where each has
+    its own (24, 25), with more tiles than CTAs either way and a matrix that runs on its own between the
+    segments, against the oracle."""
+    import lq_oracle as O
+    from lightning_b200.workloads import random_unitary
+    rng = np.random.default_rng(n)
+    ops = [("RY", [0], False, [0.7]), ("RX", [n - 1], False, [1.3]), ("CNOT", [0, n - 1], False, []),
+           ("CRZ", [n // 2, 3], False, [0.9]), ("QubitUnitary", [1, 8, 12, n - 2], False, [], random_unitary(rng, 4)),
+           ("RX", [5], True, [0.4]), ("RZ", [5], False, [2.1]), ("IsingXX", [2, 9], False, [0.5])]
+    obs = [[(1.0, [("PauliZ", [n - 1])])], [(0.5, [("PauliX", [5])]), (-0.3, [("PauliZ", [0])])],
+           [(1.0, [("PauliY", [9]), ("PauliZ", [3])])]]
+    psi = np.zeros(1 << n, dtype=np.complex128)  # a product state on the wires the circuit touches
+    psi.reshape((2,) * n)[(slice(None),) * 13 + (0,) * (n - 14) + (slice(None),)] = \
+        (rng.normal(size=(2,) * 14) + 1j * rng.normal(size=(2,) * 14)) / 180
+    sv = capi.StateVector(n, dtype)
+    sv.upload(psi.astype(dtype))
+    got = sv.adjoint_jacobian(ops, obs, [0, 1, 2, 3, 4, 5])
+    want = O.adjoint_jacobian(psi.astype(dtype).astype(np.complex128), ops, obs, [0, 1, 2, 3, 4, 5])
+    assert np.abs(got - want).max() < (1e-12 if dtype == np.complex128 else 1e-5)
+
+
+def test_more_observables_than_a_grid_dimension(capi):
+    """65 600 observables on three qubits: rows from both ends equal those of a call with these alone."""
+    ops = [("RX", [0], False, [0.3]), ("CNOT", [0, 1], False, []), ("RY", [2], False, [0.8]), ("CRY", [2, 0], False, [0.5])]
+    kinds = [[(1.0, [(p, [q])])] for p in ("PauliZ", "PauliX", "PauliY") for q in range(3)]
+    sv = capi.StateVector(3)
+    sv.apply_ops_fused(ops)
+    count = 65600
+    got = sv.adjoint_jacobian(ops, [kinds[i % 9] for i in range(count)], [0, 1, 2])
+    want = sv.adjoint_jacobian(ops, kinds, [0, 1, 2])
+    assert np.abs(got - want[np.arange(count) % 9]).max() < 1e-14
