@@ -2405,7 +2405,11 @@ int b200sv_batch_autotune(b200sv_batch_handle bh, const double *params, int *cho
         const int kts_c128[] = {10, 11, 12};
         for (int th : {256, 512}) {
             if (!B.full && th != 256) continue;  // the level program's block size follows from the tile
-            for (int i = 0; i < 3; ++i) cands.push_back(Config{th, B.dtype == B200SV_C64 ? kts_c64[i] : kts_c128[i]});
+            for (int i = 0; i < 3; ++i) {
+                const int kt = B.dtype == B200SV_C64 ? kts_c64[i] : kts_c128[i];
+                if (!B.full && kt > tiles::kMaxTileBits) continue;  // the same program as kMaxTileBits
+                cands.push_back(Config{th, kt});
+            }
         }
         float best = 1e30f;
         int best_i = -1;

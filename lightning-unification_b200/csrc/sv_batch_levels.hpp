@@ -3,6 +3,8 @@
 
 namespace tiles {
 
+constexpr int kMaxTileBits = std::max(TGeo<float, false>::kt, TGeo<double, false>::kt);
+
 // Gates of the level engine: everything but two-wire dense gates, double excitations and matrices on
 // two and more wires.
 bool serves(const HostOp &h) {

@@ -681,3 +681,18 @@ def test_gradient_sums_of_deep_circuits_take_turns(dtype):
         shift[k] = np.pi / 2
         up, down = (eng.forward(torch.tensor(params + s, device="cuda")).cpu().numpy() for s in (shift, -shift))
         assert np.abs(grads[0][k] - (up - down) / 2).max() < tol
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+def test_autotune_times_each_program_once(dtype):
+    """The level engine's tiles have at most 12 bits, so the tuner reports one of them (13 built and timed the
+    12-bit program a second time), and the tuned engine's values are the oracle's."""
+    import torch
+    from lightning_b200.batch import BatchedCircuits
+    circuits, params = layered_batch(12, 8, ("RY", "RZ"), ncirc=3)
+    eng = BatchedCircuits(circuits, len(params), dtype=dtype)
+    p = torch.tensor(params, device="cuda")
+    for _ in range(12):
+        assert eng.autotune(p) in [25600 + kt for kt in (10, 11, 12)]
+    assert np.abs(eng.forward(p).cpu().numpy() - oracle_outputs(circuits, params)).max() < \
+        (1e-12 if dtype == np.complex128 else 2e-5)
