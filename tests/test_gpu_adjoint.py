@@ -217,7 +217,8 @@ def test_adjoint_fused_sweep_every_generator(capi, dtype):
     """A 13-qubit state takes the fused reverse sweep (one observable: a Hamiltonian, the VJP
     form).  Every differentiable gate kind, constant gates and matrices on 1..4 wires, a trainable
     subset with gaps and an early exit; against the oracle's AdjointJacobianLQubit restatement,
-    and against the unfused sweep of the same engine (two observables)."""
+    and against the sweep made of single calls (gate by gate, generator by generator), with one
+    observable and two."""
     import lq_oracle as O
     from lightning_b200.workloads import random_unitary
     rng = np.random.default_rng(1313)
@@ -255,7 +256,26 @@ def test_adjoint_fused_sweep_every_generator(capi, dtype):
     got = sv.adjoint_jacobian(ops, ham, tp)
     tol = 1e-12 if dtype == np.complex128 else 1e-5
     assert np.abs(got - want).max() < tol
-    # unfused sweep of the same engine: two observables
+    # the sweep by single calls: one kernel a gate, a generator applied to a copy, an inner product
+    lam, bra, mu = (capi.StateVector(n, dtype) for _ in range(3))
+    lam.upload(st.astype(dtype))
+    bra.copy_from(lam)
+    bra.apply_observable(ham[0])
+    single, k = np.zeros(len(tp)), npar
+    for op in reversed(ops):
+        if op[3]:
+            k -= 1
+            if k in tp:
+                mu.copy_from(lam)
+                scale = mu.apply_generator(op[0], op[1])
+                single[tp.index(k)] = -2 * scale * (-1 if op[2] else 1) * bra.inner(mu).imag
+        for s in (lam, bra):
+            if len(op) > 4:
+                s.apply_matrix(op[4], op[1], inverse=True)
+            else:
+                s.apply(op[0], op[1], not op[2], op[3])
+    assert np.abs(got[0] - single).max() < tol
+    # two observables
     got2 = sv.adjoint_jacobian(ops, ham + [[(1.0, [("PauliZ", [7])])]], tp)
     assert np.abs(got2[0] - got[0]).max() < tol
     want2 = O.adjoint_jacobian(st, ops, [[(1.0, [("PauliZ", [7])])]], tp)
@@ -402,3 +422,38 @@ def test_more_observables_than_a_grid_dimension(capi):
     got = sv.adjoint_jacobian(ops, [kinds[i % 9] for i in range(count)], [0, 1, 2])
     want = sv.adjoint_jacobian(ops, kinds, [0, 1, 2])
     assert np.abs(got - want[np.arange(count) % 9]).max() < 1e-14
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+@pytest.mark.parametrize("kind", ["steps", "coefficients", "gradients"])
+def test_segments_cut_by_a_limit(capi, kind, dtype):
+    """Lists whose bits fit one tile but whose records do not fit one segment: more steps than it takes (160), more
+    coefficients (1024: three-wire matrices take 64 or 129 each), more differentiated steps (64); the state and
+    the Jacobian against the oracle."""
+    import lq_oracle as O
+    from conftest import random_state
+    from lightning_b200.workloads import random_unitary
+    rng = np.random.default_rng(len(kind))
+    n, ops = 9, []
+    for i in range({"steps": 330, "coefficients": 40, "gradients": 200}[kind]):
+        w = [int(x) for x in rng.choice(n, 3, replace=False)]
+        if kind == "steps":
+            ops.append((("CNOT", "CY", "CZ", "Toffoli")[i % 4], w if i % 4 == 3 else w[:2], False, []))
+        elif kind == "coefficients":
+            ops.append(("QubitUnitary", w, False, [], random_unitary(rng, 3)))
+        else:
+            ops.append((("CRX", "CRY", "CRZ", "IsingZZ")[i % 4], w[:2], bool(i % 3), [float(rng.uniform(0, 6))]))
+        if i % 20 == 0:
+            ops.append(("RY", [w[0]], False, [float(rng.uniform(0, 6))]))
+    psi = random_state(rng, n, dtype)
+    sv = capi.StateVector(n, dtype)
+    sv.upload(psi)
+    sv.apply_ops_fused(ops)
+    want = O.run_circuit(n, ops, state=psi.astype(np.complex128))
+    assert np.abs(sv.download() - want).max() < (1e-12 if dtype == np.complex128 else 2e-5)
+    tp = list(range(sum(1 for op in ops if op[3])))
+    for obs in ([Zs(0)], [Zs(0), [(0.5, [("PauliX", [4])]), (1.0, [("PauliY", [8])])]]):
+        st = sv.download()
+        got = sv.adjoint_jacobian(ops, obs, tp)
+        want = O.adjoint_jacobian(st.astype(np.complex128), ops, obs, tp)
+        assert np.abs(got - want).max() < (1e-12 if dtype == np.complex128 else 1e-5)

@@ -696,3 +696,113 @@ def test_autotune_times_each_program_once(dtype):
         assert eng.autotune(p) in [25600 + kt for kt in (10, 11, 12)]
     assert np.abs(eng.forward(p).cpu().numpy() - oracle_outputs(circuits, params)).max() < \
         (1e-12 if dtype == np.complex128 else 2e-5)
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+@pytest.mark.parametrize("n", [5, 12, 14])
+def test_more_words_than_a_group(dtype, n):
+    """200 Pauli words in one circuit, over several outputs and with one output of 130 (the measurement kernels
+    stage 64 at a time), beside a circuit of one word: values and the VJP against the oracle."""
+    import torch
+    from lightning_b200.batch import BatchedCircuits
+    rng = np.random.default_rng(n)
+    circuits, params = layered_batch(n, 2, ("RY", "RX"), ncirc=2, seed=n)
+    words = []
+    for _ in range(200):
+        w = [int(x) for x in rng.choice(n, int(rng.integers(1, min(n, 5) + 1)), replace=False)]
+        words.append((float(rng.normal()), "".join(rng.choice(list("XYZZ"), len(w))), w))
+    circuits[0]["observables"] = [words[:130], words[130:140], words[140:]]
+    eng = BatchedCircuits(circuits, len(params), dtype=dtype)
+    p = torch.tensor(params, device="cuda")
+    dy = rng.normal(size=4)
+    # an output of 130 words of size one, its gradient likewise: the bounds of one word times their 2-norm
+    scale = np.sqrt(sum(c * c for c, _, _ in words))
+    out = eng.forward(p).cpu().numpy()
+    assert np.abs(out - oracle_outputs(circuits, params)).max() < scale * (1e-12 if dtype == np.complex128 else 2e-5)
+    g = eng.vjp(p, torch.tensor(dy, device="cuda")).cpu().numpy()
+    assert np.abs(g - oracle_vjp(circuits, params, dy)).max() < scale * GRAD_TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+def test_jobs_of_several_tiles(dtype):
+    """So many circuits of 18 qubits, of every gate the level engine serves, that a job takes four tiles forward and
+    in the reverse sweep (two tiles of the 13-qubit ones): values, the VJP after a forward and alone, and the
+    Jacobian, against the oracle for two circuits of each structure and against these for their copies."""
+    import torch
+    import lq_oracle as O
+    from lightning_b200.batch import BatchedCircuits
+    from lightning_b200.workloads import bind, obs_terms
+    shapes, values = level_batch((18, 13, 18), seed=5)
+    jobs = 8 * 3 * torch.cuda.get_device_properties(0).multi_processor_count  # at most three CTAs an SM
+    copies = -(-4 * jobs // (2 * 64))  # 2^6 tiles of 18 qubits
+    rng = np.random.default_rng(6)
+    circuits, params, which = [], [], []
+    sets = []  # two sets of angles for each structure
+    at = 0
+    for c in shapes:
+        k = sum(1 for x in c["param_index"] if x >= 0)
+        sets.append([values[at:at + k], rng.uniform(0, 2 * np.pi, k)])
+        at += k
+    for i in range(copies):
+        for s, c in enumerate(shapes):
+            v = sets[s][i % 2]
+            pidx, k = [], len(params)
+            for x in c["param_index"]:
+                pidx.append(k if x >= 0 else -1)
+                k += x >= 0
+            params += list(v)
+            circuits.append(dict(c, param_index=pidx))
+            which.append((s, i % 2))
+    params = np.array(params)
+    eng = BatchedCircuits(circuits, len(params), dtype=dtype)
+    p = torch.tensor(params, device="cuda")
+    per = [rng.normal(size=len(c["observables"])) for c in shapes]
+    dy = torch.tensor(np.concatenate([per[s] for s, _ in which]), device="cuda")
+    out = eng.forward(p).cpu().numpy()
+    grads = [eng.vjp(p, dy).cpu().numpy() for _ in range(2)]
+    jac = eng.jacobian(p).cpu().numpy()
+    assert np.array_equal(grads[0], grads[1])
+    tol, known, oa, ga, ja = 1e-12 if dtype == np.complex128 else 2e-5, {}, 0, 0, 0
+    for c, key in zip(circuits, which):
+        obs = [obs_terms(o) for o in c["observables"]]
+        slots = [q for q in c["param_index"] if q >= 0]
+        no, ng = len(obs), len(slots)
+        got = (out[oa:oa + no], grads[0][ga:ga + ng], jac[ja:ja + no * ng])
+        oa, ga, ja = oa + no, ga + ng, ja + no * ng
+        if key not in known:
+            ops = bind(c, params)
+            psi = O.run_circuit(c["num_qubits"], ops)
+            trainable = [k for k, i in enumerate(i for i, op in enumerate(ops) if op[3]) if c["param_index"][i] >= 0]
+            J = O.adjoint_jacobian(psi, ops, obs, trainable)
+            assert np.abs(got[0] - [O.expval(psi, o) for o in obs]).max() < tol
+            assert np.abs(got[1] - per[key[0]] @ J).max() < 4 * GRAD_TOL[dtype]  # up to four outputs' errors
+            assert np.abs(got[2].reshape(no, ng) - J).max() < GRAD_TOL[dtype]
+            known[key] = got
+        assert all(np.array_equal(x, y) for x, y in zip(got, known[key]))
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+def test_level_segments_cut_by_a_limit(dtype):
+    """Circuits of one tile whose records do not fit one segment: 300 controlled rotations (64 gradients, 640
+    coefficients a segment) and 400 gates without coefficients (160 steps)."""
+    import torch
+    from lightning_b200.batch import BatchedCircuits
+    rng = np.random.default_rng(40)
+    circuits, at, n = [], 0, 9
+    for names, count in ((("CRX", "CRY", "CRZ", "IsingZZ"), 300), (("CNOT", "CZ", "Toffoli"), 400)):
+        ops, pidx = [("RY", [q], False, []) for q in range(n)], list(range(at, at + n))
+        at += n
+        for i in range(count):
+            name = names[i % len(names)]
+            ops.append((name, [int(x) for x in rng.choice(n, 3 if name == "Toffoli" else 2, replace=False)], False, []))
+            pidx.append(at if count == 300 else -1)
+            at += count == 300
+        circuits.append({"num_qubits": n, "ops": ops, "param_index": pidx,
+                         "observables": [[(1.0, "Z", [0])], [(0.6, "XY", [3, 8])]]})
+    params = rng.uniform(0, 2 * np.pi, at)
+    eng = BatchedCircuits(circuits, at, dtype=dtype)
+    p, dy = torch.tensor(params, device="cuda"), rng.normal(size=4)
+    tol = 1e-12 if dtype == np.complex128 else 2e-5
+    assert np.abs(eng.forward(p).cpu().numpy() - oracle_outputs(circuits, params)).max() < tol
+    g = eng.vjp(p, torch.tensor(dy, device="cuda")).cpu().numpy()
+    assert np.abs(g - oracle_vjp(circuits, params, dy)).max() < 2 * GRAD_TOL[dtype]  # two outputs' errors

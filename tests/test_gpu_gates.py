@@ -378,3 +378,27 @@ def test_long_lists_plan_in_linear_time(capi):
         took.append(best)
         assert abs(sv.norm2() - 1.0) < count * 1e-15
     assert took[1] < 16 * took[0]
+
+
+@pytest.mark.parametrize("n,dtype", [(23, np.complex128), (25, np.complex64)])
+def test_fused_wide_states_equal_gate_by_gate(capi, n, dtype):
+    """Several tiles a CTA (2048 and 8192 tiles for 1184): the fused list against the same gates one by one, whose
+    kernels share nothing with it.  Each side is off by about 1e-15 (complex64 6e-7) of the norm; four times that."""
+    import torch
+    from lightning_b200.workloads import random_unitary
+    rng = np.random.default_rng(n)
+    ops = []
+    for i in range(60):
+        w = [int(x) for x in rng.choice(n, 3, replace=False)]
+        ops.append([("RX", w[:1], False, [float(rng.uniform(0, 6))]), ("Hadamard", w[:1], False, []),
+                    ("CNOT", w[:2], False, []), ("CRZ", w[:2], True, [float(rng.uniform(0, 6))]),
+                    ("Toffoli", w, False, []), ("QubitUnitary", w[:2], False, [], random_unitary(rng, 2)),
+                    ("QubitUnitary", w, False, [], random_unitary(rng, 3)), ("SWAP", w[:2], False, []),
+                    ("MultiRZ", w, False, [float(rng.uniform(0, 6))]), ("CZ", w[:2], False, [])][i % 10])
+    a, b = capi.StateVector(n, dtype), capi.StateVector(n, dtype)
+    a.apply_ops_fused([("RY", [q], False, [float(x)]) for q, x in enumerate(rng.uniform(0, 6, n))])
+    b.copy_from(a)
+    a.apply_ops_fused(ops)
+    b.apply_ops(ops)
+    x, y = (torch.from_numpy(s.download()).cuda() for s in (a, b))
+    assert torch.linalg.vector_norm(x - y).item() < (4e-15 if dtype == np.complex128 else 2.4e-6)
