@@ -1048,15 +1048,6 @@ def main():
                   "path": "C ABI, one gate per launch: apply_ops + 16 Pauli expvals + adjoint VJP"},
         "ratio_vs_plain": value / world / plain_value,
         "max_grad_err_vs_fp64": err,
-        "gate_sweep": sweeps,
-        "matrix_sweep": msweep,
-        "rows_single_state": rows,
-        "rows_next": nxt,
-        "hea_batch_forward": hea,
-        "hea_batch_forward_c128": hea128,
-        "sampling": samp,
-        "plain_20q_layered": plain20,
-        "precision_sampling": precision,
         "roofline": roof,
         "roofline_batch": {
             "kernel": "k_tiles<float,0|1> (segment levels of the headline step)",
@@ -1072,6 +1063,10 @@ def main():
         "gpu_launches": (launches_fwd + launches_vjp) * args.steps,
         "clocks": clk.summary(),
     }
+    # the headline alone on stdout, one line that readers of a log's end get whole; the other rows on stderr
+    print(json.dumps({"gate_sweep": sweeps, "matrix_sweep": msweep, "rows_single_state": rows, "rows_next": nxt,
+                      "hea_batch_forward": hea, "hea_batch_forward_c128": hea128, "sampling": samp,
+                      "plain_20q_layered": plain20, "precision_sampling": precision}), file=sys.stderr, flush=True)
     print(json.dumps(line), flush=True)
     if dist:
         dist.destroy_process_group()
