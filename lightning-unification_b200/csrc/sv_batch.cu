@@ -1,5 +1,7 @@
-// sv_batch.cu — batched engine: thousands of independent circuits of uneven width
-// in one persistent launch.
+// sv_batch.cu — batched engine: thousands of independent circuits of uneven width.
+//
+// Batches of one-wire, diagonal, parity and swap gates run level by level over tiles of all circuits
+// (sv_batch_tiles.cuh, sv_batch_levels.hpp).  The others run in one persistent launch (k_batch), as follows.
 //
 // Each CTA pulls circuits from an atomic work queue (longest first).  A circuit
 // whose state fits in shared memory (2^n <= 2^kt amplitudes per live state) runs

@@ -9,8 +9,9 @@
 // (circuits x tiles) independent pieces of work and nothing waits on another CTA.  One wide
 // circuit spreads over the whole GPU this way: a training step over 192 circuits of 10-18 qubits,
 // complex128, went from 121.5 ms (one CTA per circuit: the widest circuits' chains of tiles ran alone
-// at the end) to 7.4 ms, and the 1024-circuit step of 16 qubits, complex64, from 70.2 to 22.5 ms (fewer
-// barriers and shared-memory passes between steps, three 256-thread CTAs an SM instead of one of 512).
+// at the end) to 6.7 ms, and the 1024-circuit step of 16 qubits, complex64, from 70.2 to 22.3 ms (fewer
+// barriers and shared-memory passes between steps, two 256-thread CTAs an SM, three in the complex64
+// forward sweep, instead of one of 512).
 // Circuits narrower than a tile are one tile of their own size in CTAs of fewer threads,
 // launched beside the wide ones.
 //

@@ -1,10 +1,10 @@
 """torch.autograd.Function over the batched engine.
 
-forward: params -> <O_{c,o}> for every circuit c and observable o (one
-persistent launch).  backward: the adjoint vector-Jacobian product with a
-single bra sum_o dy_o O_o psi per circuit (the Hamiltonian trick the reference
-uses for its vjp, pennylane_lightning/lightning_qubit/lightning_qubit.py:747-772),
-one more persistent launch.  Both run on torch's current stream.
+forward: params -> <O_{c,o}> for every circuit c and observable o.  backward: the
+adjoint vector-Jacobian product with a single bra sum_o dy_o O_o psi per circuit
+(the Hamiltonian trick the reference uses for its vjp,
+pennylane_lightning/lightning_qubit/lightning_qubit.py:747-772).  Both run on
+torch's current stream, replayed as one CUDA graph each from the second call on.
 """
 from __future__ import annotations
 

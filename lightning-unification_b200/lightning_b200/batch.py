@@ -1,4 +1,4 @@
-"""Batched engine: many independent circuits in one persistent launch.
+"""Batched engine: many independent circuits at once, a segment of every circuit per launch.
 
 Python view of ``b200sv_batch_*`` (include/b200sv.h).  Parameters, outputs and
 gradients are torch CUDA tensors (float64); torch provides the device memory

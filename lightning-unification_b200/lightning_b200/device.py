@@ -304,7 +304,7 @@ class LightningQubit:
                                   f"Operations have already been applied on a {self.short_name} device.")
         ops = [op for op in operations if op.name != "Identity"]
         # the fused apply: one pass over the state per run of gates that fit a shared-memory
-        # tile on wide states, one launch per gate on narrow ones (same results to rounding)
+        # tile (a narrow state is one tile), results as gate by gate to rounding
         if ops:
             self._sv.apply_ops_fused(self._serialize_ops(ops))
         if rotations:
