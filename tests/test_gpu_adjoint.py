@@ -410,6 +410,8 @@ def test_several_observables_on_wide_states(capi, n, dtype):
     got = sv.adjoint_jacobian(ops, obs, [0, 1, 2, 3, 4, 5])
     want = O.adjoint_jacobian(psi.astype(dtype).astype(np.complex128), ops, obs, [0, 1, 2, 3, 4, 5])
     assert np.abs(got - want).max() < (1e-12 if dtype == np.complex128 else 1e-5)
+    alone = sv.adjoint_jacobian(ops, obs[1:2], [0, 1, 2, 3, 4, 5])  # one bra, lambda in place
+    assert np.abs(alone[0] - want[1]).max() < (1e-12 if dtype == np.complex128 else 1e-5)
 
 
 def test_more_observables_than_a_grid_dimension(capi):
