@@ -15,6 +15,13 @@ bool serves(const HostOp &h) {
     }
 }
 
+// A one-wire gate with a real matrix.
+bool is_real(const HostOp &h) {
+    if (h.form != F_MAT1 || h.bits.size() != 1) return false;
+    if (h.gate != kConstGate) return h.gate == B200SV_RY;
+    return std::all_of(h.cmat.begin(), h.cmat.end(), [](cd z) { return z.imag() == 0; });
+}
+
 std::vector<Step> make_steps(const std::vector<HostOp> &ops, uint32_t n) {
     std::vector<Step> out;
     std::vector<int> last(n, -1);  // latest step on each bit
@@ -78,7 +85,14 @@ std::vector<Step> make_steps(const std::vector<HostOp> &ops, uint32_t n) {
         out.push_back(std::move(s));
     }
     for (Step &s : out)
-        if (s.kind == S_RUN) s.targets = s.mask;
+        if (s.kind == S_RUN) {
+            s.targets = s.mask;
+            if (s.mems.size() == 2) {
+                const HostOp &a = ops[s.mems[0]], &b = ops[s.mems[1]];
+                if (is_real(a) && b.form == F_DIAG) s.split = 1;
+                else if (a.form == F_DIAG && is_real(b)) s.split = 2;
+            }
+        }
     return out;
 }
 
@@ -109,8 +123,9 @@ template <typename R, bool REV> void plan_dir(Builder &B, Plan &P, uint32_t n, i
     }
     D.step_begin = (uint32_t)B.steps.size();
     B.rec.ncoef = 0;
-    auto coef = [&](uint32_t si, SKind kind, const TOp &, const uint8_t *src, const int *, uint32_t at) {
+    auto coef = [&](uint32_t si, SKind kind, TOp &o, const uint8_t *src, const int *, uint32_t at) {
         const Step &s = P.steps[si];
+        if (kind == S_SPLIT) o.pad = (s.split == 2) != REV;
         CoefStep c{};
         c.kind = kind;
         c.mem_begin = (uint32_t)B.mem_list.size();
@@ -140,7 +155,8 @@ std::string structure_key(const std::vector<HostOp> &ops, uint32_t n) {
         const bool sign = h.form == F_DIAG && h.gate == kConstGate && h.bits.size() == 2 &&
                           ((h.nt == 0 && h.cmat[0] == cd(-1, 0)) ||
                            (h.nt == 1 && h.cmat[0] == cd(1, 0) && h.cmat[1] == cd(-1, 0)));
-        put((uint32_t)h.form | (uint32_t)h.nt << 8 | (h.diff ? 1u << 16 : 0u) | (sign ? 1u << 17 : 0u));
+        put((uint32_t)h.form | (uint32_t)h.nt << 8 | (h.diff ? 1u << 16 : 0u) | (sign ? 1u << 17 : 0u) |
+            (is_real(h) ? 1u << 18 : 0u));
         put(h.diff ? h.gate : 0u);
         put((uint32_t)h.bits.size());
         for (auto b : h.bits) put(b);

@@ -9,7 +9,7 @@
 // (circuits x tiles) independent pieces of work and nothing waits on another CTA.  One wide
 // circuit spreads over the whole GPU this way: a training step over 192 circuits of 10-18 qubits,
 // complex128, went from 121.5 ms (one CTA per circuit: the widest circuits' chains of tiles ran alone
-// at the end) to 6.7 ms, and the 1024-circuit step of 16 qubits, complex64, from 70.2 to 22.3 ms (fewer
+// at the end) to 6.35 ms, and the 1024-circuit step of 16 qubits, complex64, from 70.2 to 22.3 ms (fewer
 // barriers and shared-memory passes between steps, two 256-thread CTAs an SM, three in the complex64
 // forward sweep, instead of one of 512).
 // Circuits narrower than a tile are one tile of their own size in CTAs of fewer threads,
@@ -210,7 +210,7 @@ template <typename R> __global__ void k_tile_coefs(CoefArgs a) {
             const CoefStep st = a.steps[a.step_begin[c] + i];
             const uint32_t *list = a.mem_list + st.mem_begin;
             C<R> *o = out + st.coef;
-            if (st.kind == S_RUN || st.kind == S_DIAGRUN) {
+            if (st.kind == S_RUN || st.kind == S_SPLIT || st.kind == S_DIAGRUN) {
                 const double2 zero = make_double2(0, 0), one = make_double2(1, 0);
                 Mat2 run{{one, zero, zero, one}, {zero, zero, zero, zero}};
                 double2(&P)[4] = run.h;
@@ -219,6 +219,15 @@ template <typename R> __global__ void k_tile_coefs(CoefArgs a) {
                     if (rev && m.gslot >= 0) a.h[m.gslot] = gen_row(gen_code(m.gate), P);
                     Mat2 q{{}, {zero, zero, zero, zero}};
                     member_mat<double>(m, a.cs, a.consts, rev, q.h);
+                    if (st.kind == S_SPLIT) {
+                        if (m.form == F_DIAG) {
+                            o[2] = mk<R>((R)q.h[0].x, (R)q.h[0].y);
+                            o[3] = mk<R>((R)q.h[3].x, (R)q.h[3].y);
+                        } else {
+                            o[0] = mk<R>((R)q.h[0].x, (R)q.h[1].x);
+                            o[1] = mk<R>((R)q.h[2].x, (R)q.h[3].x);
+                        }
+                    }
                     if constexpr (sizeof(R) == 8) {
                         mul22(q, run);
                     } else {
@@ -229,7 +238,7 @@ template <typename R> __global__ void k_tile_coefs(CoefArgs a) {
                 }
                 if (st.kind == S_RUN) {
                     for (int e = 0; e < 4; ++e) o[e] = mk<R>((R)P[e].x, (R)P[e].y);
-                } else {  // a table whose lowest index bit is the run's bit
+                } else if (st.kind == S_DIAGRUN) {  // a table whose lowest index bit is the run's bit
                     for (int e = 0; e < 8; ++e) o[e] = mk<R>((R)P[(e & 1) * 3].x, (R)P[(e & 1) * 3].y);
                 }
                 continue;

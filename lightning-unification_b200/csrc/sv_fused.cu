@@ -285,13 +285,24 @@ std::vector<Step> make_steps(const std::vector<const GateDesc *> &gs, uint32_t n
         out.push_back(std::move(s));
     }
     for (Step &s : out)
-        if (!s.single && s.kind == S_RUN) s.targets = s.mask;
+        if (!s.single && s.kind == S_RUN) {
+            s.targets = s.mask;
+            if (s.mems.size() == 2) {
+                auto real = [&](int k) {
+                    cd m[4];
+                    one_bit_matrix(*gs[s.mems[k]], m);
+                    return m[0].imag() == 0 && m[1].imag() == 0 && m[2].imag() == 0 && m[3].imag() == 0;
+                };
+                if (gs[s.mems[1]]->kind == Kind::Diag && real(0)) s.split = 1;
+                else if (gs[s.mems[0]]->kind == Kind::Diag && real(1)) s.split = 2;
+            }
+        }
     return out;
 }
 
 // Coefficients of a step's record, in the positions plan_segments gave it.
 template <typename R>
-void put_coefs(std::vector<C<R>> &out, const std::vector<const GateDesc *> &gs, const Step &s, SKind kind, const TOp &o,
+void put_coefs(std::vector<C<R>> &out, const std::vector<const GateDesc *> &gs, const Step &s, SKind kind, TOp &o,
                const uint8_t *src, const int *tr, uint32_t at) {
     auto put = [&](uint32_t i, cd z) {
         if (out.size() <= at + i) out.resize(at + i + 1, mk<R>(0, 0));
@@ -304,6 +315,17 @@ void put_coefs(std::vector<C<R>> &out, const std::vector<const GateDesc *> &gs, 
         run_product<R>(gs, s.mems, P);
         if (kind == S_RUN) for (uint32_t e = 0; e < 4; ++e) put(e, P[e]);
         else for (uint32_t e = 0; e < 8; ++e) put(e, P[(e & 1) * 3]);
+        break;
+    }
+    case S_SPLIT: {  // the gates are in the order that they run in
+        cd r[4], d[4];
+        o.pad = s.split == 2;
+        one_bit_matrix(*gs[s.mems[s.split - 1]], r);
+        one_bit_matrix(*gs[s.mems[2 - s.split]], d);
+        put(0, cd(r[0].real(), r[1].real()));
+        put(1, cd(r[2].real(), r[3].real()));
+        put(2, d[0]);
+        put(3, d[3]);
         break;
     }
     case S_DENSE:
@@ -366,7 +388,6 @@ void put_coefs(std::vector<C<R>> &out, const std::vector<const GateDesc *> &gs, 
         break;
     default: break;
     }
-    (void)o;
 }
 
 // Device copies of host arrays in one upload (freed in stream order).
@@ -413,7 +434,7 @@ void run_fused(void *state, uint32_t nq, const std::vector<GateDesc> &descs,
     for (uint32_t i = 0; i < order.size(); ++i) order[i] = i;
     Records rec;
     std::vector<C<R>> coefs;
-    auto coef = [&](uint32_t si, SKind kind, const TOp &o, const uint8_t *src, const int *tr, uint32_t at) {
+    auto coef = [&](uint32_t si, SKind kind, TOp &o, const uint8_t *src, const int *tr, uint32_t at) {
         put_coefs<R>(coefs, gs, all[si], kind, o, src, tr, at);
     };
     const std::vector<Piece> pieces = plan_segments<R, false>(all, order, nq, 64, false, false, kMaxStateCoefs, rec, coef);
@@ -520,7 +541,7 @@ void run_fused_adjoint(void *&lam, void *&lam2, const std::vector<void *> &bras,
     for (uint32_t i = 0; i < order.size(); ++i) order[i] = i;
     Records rec;
     std::vector<C<R>> coefs;
-    auto coef = [&](uint32_t si, SKind kind, const TOp &o, const uint8_t *src, const int *tr, uint32_t at) {
+    auto coef = [&](uint32_t si, SKind kind, TOp &o, const uint8_t *src, const int *tr, uint32_t at) {
         put_coefs<R>(coefs, gs, all[si], kind, o, src, tr, at);
     };
     const std::vector<Piece> pieces = plan_segments<R, true>(all, order, nq, 64, false, false, kMaxStateCoefs, rec, coef);

@@ -21,6 +21,7 @@ enum SKind : uint8_t {
     S_WIDE = 6,     // dense on two or three bits
     S_PAIR2 = 7,    // excitation block on two bits
     S_PAIR4 = 8,    // excitation block on four bits
+    S_SPLIT = 9,    // a run of a real 2x2 and a diagonal (complex128): both kept apart
 };
 
 constexpr int kLookAhead = 4096;  // steps a segment leaves out before it is closed
@@ -32,6 +33,7 @@ struct Step {
     bool linear = false;             // CNOT, SWAP: between phases, in the tile's address map
     bool single = false;             // has no tile form: runs alone
     bool gamma = false;              // S_PAIR2, S_PAIR4: the other rows take a factor
+    uint8_t split = 0;               // S_RUN of two gates, 1: a real 2x2 and then a diagonal, 2: the reverse
     std::vector<uint32_t> mems;      // caller's indices of its gates, in order
     std::vector<uint32_t> ctl, tgt;  // state bits (tgt[0] the matrix index's most significant)
     uint64_t mask = 0;               // bits touched
@@ -53,12 +55,13 @@ struct Piece {
 };
 
 // A diagonal run with a gradient is a 2x2 step of the reverse sweep (its sums go over register pairs).
-template <bool REV> SKind effective_kind(const Step &s) {
+template <typename R, bool REV> SKind effective_kind(const Step &s) {
+    if (sizeof(R) == 8 && s.kind == S_RUN && s.split) return S_SPLIT;
     return REV && s.kind == S_DIAGRUN && s.grad ? S_RUN : s.kind;
 }
 template <typename R, bool REV> int coef_slots(const Step &s) {
-    switch (effective_kind<REV>(s)) {
-    case S_RUN: case S_DENSE: return 4;
+    switch (effective_kind<R, REV>(s)) {
+    case S_RUN: case S_SPLIT: case S_DENSE: return 4;
     case S_DIAGRUN: case S_DIAG: return 8;
     case S_PARITY: return 2;
     case S_PAIR2: case S_PAIR4: return 5;
@@ -248,7 +251,7 @@ std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector
             for (uint32_t i : cur) {
                 const uint32_t si = order[take[i]];
                 const Step &s = all[si];
-                const SKind kind = effective_kind<REV>(s);
+                const SKind kind = effective_kind<R, REV>(s);
                 TOp o{};
                 uint8_t src[3] = {255, 255, 255};
                 int tr[4] = {-1, -1, -1, -1};
@@ -289,6 +292,8 @@ std::vector<Piece> plan_segments(const std::vector<Step> &all, const std::vector
                     } else {
                         o.code = T_SWAP + pair_index(rm);
                     }
+                } else if (kind == S_SPLIT) {
+                    o.code = T_SPLIT + tr[0];
                 } else if (kind == S_RUN) {
                     o.code = (exact_single && o.grad && s.mems.size() == 1 ? T_DENSEC : T_DENSE) + tr[0];
                 } else if (kind == S_DENSE) {

@@ -27,10 +27,11 @@ enum TCode : uint16_t {
     T_SIGN2 = 32,    // -1: two register bits and thread bits
     T_SWAP = 40,     // exchange of a pair of register bits, any controls
     T_CX_R = 48,     // + target * 4 + control: swap along target, control one register bit (and thread bits)
-    T_DENSE2 = 64,   // dense matrix on a register pair, any controls (FP64 coefficients)
-    T_DENSE3 = 72,   // dense matrix on three register bits (trip_mask), any controls (FP64 coefficients)
-    T_PAIR2 = 80,    // 2x2 block on rows 01, 10 of a register pair, gamma on the others
-    T_PAIR4 = 88,    // 2x2 block on registers 3 and 12, gamma on the others
+    T_SPLIT = 64,    // real 2x2 on the register bit and a diagonal on it (complex128)
+    T_DENSE2 = 72,   // dense matrix on a register pair, any controls (FP64 coefficients)
+    T_DENSE3 = 80,   // dense matrix on three register bits (trip_mask), any controls (FP64 coefficients)
+    T_PAIR2 = 88,    // 2x2 block on rows 01, 10 of a register pair, gamma on the others
+    T_PAIR4 = 96,    // 2x2 block on registers 3 and 12, gamma on the others
 };
 
 struct alignas(16) TOp {
@@ -41,7 +42,7 @@ struct alignas(16) TOp {
     uint32_t pm;           // parity: tile bits
     uint64_t pmg;          // parity: state bits outside the tile
     uint8_t p0, p1, p2;
-    uint8_t pad;           // T_PAIR2, T_PAIR4: gamma is not 1
+    uint8_t pad;           // T_PAIR2, T_PAIR4: gamma is not 1; T_SPLIT: the diagonal comes first
     uint32_t dsign;        // T_DIAG with a gradient: generator entry of index i in bits 2i (1: +1, 2: -1)
 };
 // CNOT and SWAP steps move no data.  A segment keeps a GF(2)-linear map from the tile position of an
@@ -198,6 +199,30 @@ __device__ __forceinline__ void t_dense(Regs<R, A> &v, uint32_t creg, const C<R>
             v.set(g, p);
             v.set(g | B, q);
         }
+    }
+}
+// A real 2x2 r and a diagonal d on every pair of the register bit, one after the other: as many operations as
+// their product takes, and the gates' own rounding on each amplitude, where the product's is the same on
+// all of them.
+template <int A, int BIT>
+__device__ __forceinline__ void t_split(Regs<double, A> &v, const double2 (&r)[2], double2 d0, double2 d1, bool first) {
+    constexpr int B = 1 << BIT;
+#pragma unroll
+    for (int g = 0; g < A; ++g) {
+        if (g & B) continue;
+        double2 x = v.get(g), y = v.get(g | B);
+        if (first) {
+            x = cmul1<double>(d0, x);
+            y = cmul1<double>(d1, y);
+        }
+        double2 p = make_double2(fma(r[0].y, y.x, r[0].x * x.x), fma(r[0].y, y.y, r[0].x * x.y));
+        double2 q = make_double2(fma(r[1].y, y.x, r[1].x * x.x), fma(r[1].y, y.y, r[1].x * x.y));
+        if (!first) {
+            p = cmul1<double>(d0, p);
+            q = cmul1<double>(d1, q);
+        }
+        v.set(g, p);
+        v.set(g | B, q);
     }
 }
 // The four sums of a differentiated step on register bit BIT, in FP64.  EXACT: so are the products, of
@@ -438,6 +463,28 @@ __device__ __forceinline__ void t_step(Regs<R, A> &v, Regs<R, A> &w, const TOp &
         if (grad) add_sums(sacc, op.grad - 1u, s);
         return;
     }
+#define TILE_SPLIT(b)                                                                                          \
+    if constexpr (sizeof(R) == 8 && (1 << b) < A) {                                                            \
+        if (grad) t_cross<R, A, b, false, true>(v, w, 0, s);                                                   \
+        t_split<A, b>(v, r, d0, d1, first);                                                                    \
+        if (NS == 2) t_split<A, b>(w, r, d0, d1, first);                                                       \
+    }
+    // ahead of the others in the batch engine, whose ansatz layers are such runs; a single state's lists of
+    // all kinds ran 0.7 % slower with this test before the table (26 qubits, 200 gates)
+    if constexpr (sizeof(R) == 8 && !WIDE) {
+        if ((op.code & ~3) == T_SPLIT) {
+            const double2 r[2] = {cf[0], cf[1]}, d0 = cf[2], d1 = cf[3];
+            const bool grad = NS == 2 && op.grad, first = op.pad != 0;
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+            if (op.code & 2) {
+                if (op.code & 1) { TILE_SPLIT(3) } else { TILE_SPLIT(2) }
+            } else {
+                if (op.code & 1) { TILE_SPLIT(1) } else { TILE_SPLIT(0) }
+            }
+            if (grad) add_sums(sacc, op.grad - 1u, s);
+            return;
+        }
+    }
     switch (op.code) {
     case T_DIAG_T: {
         const uint32_t idx = (((base >> op.p0) & 1u) << 2) | (((base >> op.p1) & 1u) << 1) | ((base >> op.p2) & 1u);
@@ -491,6 +538,15 @@ __device__ __forceinline__ void t_step(Regs<R, A> &v, Regs<R, A> &w, const TOp &
         break;
     }
 #define TILE_BIT_CASES(b)                                                                                      \
+    case T_SPLIT + b:                                                                                          \
+        if constexpr (sizeof(R) == 8 && WIDE) {                                                                \
+            const double2 r[2] = {cf[0], cf[1]}, d0 = cf[2], d1 = cf[3];                                       \
+            const bool grad = NS == 2 && op.grad, first = op.pad != 0;                                         \
+            double s[4] = {0.0, 0.0, 0.0, 0.0};                                                                \
+            TILE_SPLIT(b)                                                                                      \
+            if (grad) add_sums(sacc, op.grad - 1u, s);                                                         \
+        }                                                                                                      \
+        break;                                                                                                 \
     case T_DIAG1 + b:                                                                                          \
         if constexpr ((1 << b) < A) {                                                                          \
             const uint32_t i = ((((base >> op.p0) & 1u) << 1) | ((base >> op.p1) & 1u)) * 2u;                  \
@@ -534,6 +590,7 @@ __device__ __forceinline__ void t_step(Regs<R, A> &v, Regs<R, A> &w, const TOp &
         break;
         TILE_EACH_BIT(TILE_BIT_CASES)
 #undef TILE_BIT_CASES
+#undef TILE_SPLIT
 #define TILE_PAIR_CASES(i)                                                                                     \
     case T_SIGN2 + i:                                                                                          \
         if constexpr (pair_mask(i) < A) {                                                                      \

@@ -175,3 +175,31 @@ def test_run_product_rounded_once(capi):
     want = [z.real, z.imag, abs(col[0]) ** 2 - abs(col[1]) ** 2]
     out = eng.forward(torch.empty(0, dtype=torch.float64, device="cuda")).cpu().numpy()
     assert np.abs(out - np.array(want, dtype=np.longdouble)).max() < 1e-15
+
+
+@pytest.mark.gpu
+def test_two_gate_runs_round_as_gate_by_gate(capi):
+    """A run of a real gate and a diagonal one is applied as the two of them: its coefficients are the gates' own, so
+    the squared norm after 16 layers on 13 qubits differs from gate by gate only by the amplitudes' rounding (which
+    averages out to 1e-17 over 2^13 of them) and the two reductions' (a few 1.1e-16).  As rounded products,
+    208 runs shift it by 1e-15."""
+    import torch
+    from lightning_b200.batch import BatchedCircuits
+    rng = np.random.default_rng(44)
+    n, worst = 13, 0.0
+    for _ in range(4):
+        ops = []
+        for l in range(16):
+            for q in range(n):
+                pair = [("RY", [q], False, [float(rng.uniform(0, 6.3))]),
+                        (("RZ", "PhaseShift")[q % 2], [q], False, [float(rng.uniform(0, 6.3))])]
+                ops += pair if l % 2 else pair[::-1]
+            ops += [("CNOT", [q, (q + 1 + l % 5) % n], False, []) for q in range(n)]
+        plain, fused = capi.StateVector(n), capi.StateVector(n)
+        plain.apply_ops(ops)
+        fused.apply_ops_fused(ops)
+        eng = BatchedCircuits([{"num_qubits": n, "ops": ops, "param_index": [-1] * len(ops),
+                                "observables": [[(1.0, "I", [0])]]}], 0, dtype=np.complex128)
+        batch = eng.forward(torch.empty(0, dtype=torch.float64, device="cuda")).item()
+        worst = max(worst, abs(fused.norm2() - plain.norm2()), abs(batch - plain.norm2()))
+    assert worst < 5e-16
